@@ -1599,12 +1599,17 @@ struct tf_ctx {
   const double* graph_key_P = nullptr;
   double* graph_key_J = nullptr;
   double* graph_key_K = nullptr;
+  const double* graph_key_Pb = nullptr;       // unrestricted builds: the beta arrays (else null)
+  double* graph_key_Jb = nullptr;
+  double* graph_key_Kb = nullptr;
   bool graph_key_mixed = false;
   int graph_key_want = 3;
   double graph_key_cutoff = 0.0;
   bool graph_key_mol_cut = false;             // the captured list passes read per-molecule cutoffs
   int graph_kernels = 0;
-  // class schedule (autotuned): graph branches and the branch of each class pair
+  // class schedule: graph branches and the branch of each class pair, set by the
+  // autotuner or, until it has run, at each capture (default_schedule)
+  bool sched_tuned = false;
   int sched_streams = 1;
   std::vector<int> sched_stream_of;
   std::vector<int> cls_variant;                          // launch-bound variant of each class pair's kernel
@@ -2511,17 +2516,112 @@ static int enqueue_finalize(tf_ctx* c, double* dJ, double* dK, double* dJb, doub
   return TF_OK;
 }
 
+// The branch streams and events of graph builds, up to n branches (the context stream
+// is the first).
+static int ensure_branches(tf_ctx* c, int n) {
+  while ((int)c->side.size() < n - 1) {
+    cudaStream_t x;
+    TF_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+    c->side.push_back(x);
+  }
+  while (c->join_ev.size() < c->side.size()) {
+    cudaEvent_t e;
+    TF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    c->join_ev.push_back(e);
+  }
+  if (!c->fork_ev) TF_CUDA(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
+  if (!c->list_fork_ev) TF_CUDA(cudaEventCreateWithFlags(&c->list_fork_ev, cudaEventDisableTiming));
+  if (!c->list_join_ev) TF_CUDA(cudaEventCreateWithFlags(&c->list_join_ev, cudaEventDisableTiming));
+  return TF_OK;
+}
+
+// Branches of a build whose schedule no autotuner has chosen.  A class pair's launch ends
+// in a tail of its longest quartets that leaves most SMs idle, and in a small build the
+// tails are nearly all of it, so the launches overlap.  Measured (graph builds, 1, 2, 4, 6
+// and 8 branches): (H2O)7 cc-pVDZ 6.09, 3.55, 2.41, 2.00 and 2.91 ms; (H2O)2 STO-3G from
+// host arrays 0.42, 0.27, 0.23, 0.18 and 0.17 ms; (H2O)12 cc-pVDZ, deterministic, 10.5, 7.4,
+// 6.1, 6.2 and 6.3 ms; (H2O)32 cc-pVDZ 81.4, 76.8, 76.9, 76.2 and 76.4 ms.
+constexpr int DEFAULT_BRANCHES = 6;
+
+// The class pair's kernel works in the context's one scratch area (d_wscratch), so such
+// launches follow one another on the context stream.
+static bool shares_scratch(const tf_ctx* c, int g) {
+  return c->group_cls[g].x >= pair_class(3, 0) || c->group_cls[g].y >= pair_class(3, 0);
+}
+
+// Class schedule of a build that no autotuner has chosen one for: the class pairs over
+// DEFAULT_BRANCHES branches, longest first, each to the least-loaded branch, by the FLOP
+// model at the given list lengths (goff: start, FP32 start and end per group) with eight
+// primitive quartets per entry, or, goff null, at the counts of the last build.
+static int default_schedule(tf_ctx* c, const long long* goff) {
+  if (c->sched_tuned) return TF_OK;
+  TF_TRY_RC(ensure_branches(c, DEFAULT_BRANCHES));
+  const int ng = (int)c->group_cls.size();
+  const unsigned long long* pc = c->pin->pc;
+  std::vector<double> cost(ng, 1.0);
+  for (int g = 0; g < ng; ++g) {
+    int l1h, l1l, l2h, l2l;
+    class_l(c->group_cls[g].x, l1h, l1l);
+    class_l(c->group_cls[g].y, l2h, l2l);
+    const int cid = qclass_id(l1h, l1l, l2h, l2l);
+    const double nq = goff ? (double)(goff[3 * g + 2] - goff[3 * g])
+                           : (double)pc[NQCLS + 1 + cid] + (double)pc[2 * NQCLS + 1 + cid];
+    cost[g] += class_flops(l1h, l1l, l2h, l2l, nq, goff ? 8.0 * nq : (double)pc[cid]);
+  }
+  std::vector<int> order(ng);
+  std::iota(order.begin(), order.end(), 0);
+  std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cost[x] > cost[y]; });
+  std::vector<double> load(DEFAULT_BRANCHES, 0.0);
+  c->sched_streams = DEFAULT_BRANCHES;
+  c->sched_stream_of.assign(ng, 0);
+  for (int g : order)
+    if (shares_scratch(c, g)) load[0] += cost[g];
+  for (int g : order) {
+    if (shares_scratch(c, g)) continue;
+    const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
+    c->sched_stream_of[g] = k;
+    load[k] += cost[g];
+  }
+  return TF_OK;
+}
+
+// Branches of the current schedule, and the start and end of a set of class launches on
+// them: the branches wait for the context stream's earlier work, and the context stream
+// then waits for the branches.
+static int sched_branches(const tf_ctx* c) { return std::max(1, std::min(c->sched_streams, 1 + (int)c->side.size())); }
+
+static int fork_branches(tf_ctx* c, int ns) {
+  if (ns <= 1) return TF_OK;
+  TF_CUDA(cudaEventRecord(c->fork_ev, c->stream));
+  for (int i = 0; i + 1 < ns; ++i) TF_CUDA(cudaStreamWaitEvent(c->side[i], c->fork_ev, 0));
+  return TF_OK;
+}
+
+static int join_branches(tf_ctx* c, int ns) {
+  for (int i = 0; i + 1 < ns; ++i) {
+    TF_CUDA(cudaEventRecord(c->join_ev[i], c->side[i]));
+    TF_CUDA(cudaStreamWaitEvent(c->stream, c->join_ev[i], 0));
+  }
+  return TF_OK;
+}
+
+static cudaStream_t branch_of(const tf_ctx* c, int g, int ns) {
+  if (ns <= 1 || g >= (int)c->sched_stream_of.size() || shares_scratch(c, g)) return c->stream;
+  const int k = c->sched_stream_of[g] % ns;
+  return k == 0 ? c->stream : c->side[k - 1];
+}
+
 // Graph path: every class launch reads its quartet range from the device
 // (persistent grids of fixed size), so the whole build is one captured graph
 // with no host round trip inside.  The list buffer holds list_cap quartets; a
 // build whose list is longer is detected on the host after the graph (the
 // ranges are clamped, so nothing is written out of bounds) and re-run on the
 // dynamic path with a larger buffer.
-static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* dK, bool mixed, int want,
-                              int& kernels) {
+static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* dK, const double* dPb, double* dJb,
+                              double* dKb, bool mixed, int want, int& kernels) {
   cudaStream_t s = c->stream;
   ListArgs la;
-  int rc = enqueue_counts(c, dP, nullptr, mixed, c->graph_cap, la, kernels);
+  int rc = enqueue_counts(c, dP, dPb, mixed, c->graph_cap, la, kernels);
   if (rc) return rc;
   ListArgs lw = la;
   lw.out_cap = c->graph_cap;
@@ -2532,21 +2632,18 @@ static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* d
   // class schedule: the class launches are spread over sched_streams branches of
   // the graph (the autotuner's choice), so that one class's tail overlaps another
   // class's start; J and K are summed with atomics, so the order is free
-  const int ns = std::max(1, std::min(c->sched_streams, 1 + (int)c->side.size()));
-  if (ns > 1) {
-    TF_CUDA(cudaEventRecord(c->fork_ev, s));
-    for (int i = 0; i + 1 < ns; ++i) TF_CUDA(cudaStreamWaitEvent(c->side[i], c->fork_ev, 0));
-  }
+  const int ns = sched_branches(c);
+  TF_TRY_RC(fork_branches(c, ns));
   for (int g = 0; g < ng; ++g) {
     if (c->group_task0[g + 1] == c->group_task0[g]) continue;   // no molecule has this class pair
     int l1h, l1l, l2h, l2l;
     class_l(c->group_cls[g].x, l1h, l1l);
     class_l(c->group_cls[g].y, l2h, l2l);
-    const int si = ns > 1 && g < (int)c->sched_stream_of.size() ? c->sched_stream_of[g] % ns : 0;
-    cudaStream_t sg = si == 0 ? s : c->side[si - 1];
+    cudaStream_t sg = branch_of(c, g, ns);
     JKArgs a{c->d_quartets.p, 0, c->d_pairs.p, c->d_prim_full.p, c->d_prim_skip.p, c->d_Pc.p, c->d_Jc.p,
              c->d_Kc.p, c->d_mols.p, c->d_prim_count.p, c->d_group_offsets.p + 3 * g, 0, c->graph_cap,
-             c->d_jkrec.p, c->d_pairR.p, nullptr, nullptr, nullptr, want};
+             c->d_jkrec.p, c->d_pairR.p, dPb ? c->d_PcB.p : nullptr, dPb ? c->d_JcB.p : nullptr,
+             dPb ? c->d_KcB.p : nullptr, want};
     a.wscratch = c->d_wscratch.p;
     a.wscratch_warps = c->wscratch_warps;
     a.qmask = c->d_qmask.p;
@@ -2567,16 +2664,12 @@ static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* d
       kernels++;
     }
   }
-  if (ns > 1)
-    for (int i = 0; i + 1 < ns; ++i) {
-      TF_CUDA(cudaEventRecord(c->join_ev[i], c->side[i]));
-      TF_CUDA(cudaStreamWaitEvent(s, c->join_ev[i], 0));
-    }
-  return enqueue_finalize(c, dJ, dK, nullptr, nullptr, kernels);
+  TF_TRY_RC(join_branches(c, ns));
+  return enqueue_finalize(c, dJ, dK, dJb, dKb, kernels);
 }
 
 // Statistics of the finished build from the pinned read-backs and the events.
-static int finish_stats(tf_ctx* c, int kernels, bool graph) {
+static int finish_stats(tf_ctx* c, int kernels, bool graph, bool timed = false) {
   const int ng = (int)c->group_cls.size();
   const long long* goff = c->pin->goff;
   const unsigned long long* pc = c->pin->pc;
@@ -2603,8 +2696,8 @@ static int finish_stats(tf_ctx* c, int kernels, bool graph) {
     npq += p;
     const double fl = class_flops(l1h, l1l, l2h, l2l, (double)nq, p);
     flops += fl;
-    float ms = 0.f;                       // per-class device time: direct builds only
-    if (!graph) {
+    float ms = 0.f;                       // per-class device time: class-by-class builds only
+    if (timed) {
       TF_CUDA(cudaEventElapsedTime(&ms, c->cls_ev[2 * g], c->cls_ev[2 * g + 1]));
       ms_eri += ms;
     }
@@ -2617,7 +2710,7 @@ static int finish_stats(tf_ctx* c, int kernels, bool graph) {
     c->cls_stats.push_back(cs);
   }
   c->stats.build_ms = ms_all;
-  c->stats.eri_ms = graph ? ms_all : ms_eri;
+  c->stats.eri_ms = timed ? ms_eri : ms_all;
   c->stats.quartets = n_all;
   c->stats.quartets_fp32 = n_fp32;
   c->stats.prim_quartets = npq;
@@ -2670,8 +2763,9 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
   }
   // graph path: once a dynamic build has sized the list buffer and set up every
   // launch, later builds with the same arrays replay one captured graph
-  if (c->use_graph && c->graph_cap > 0 && !dPb) {
+  if (c->use_graph && c->graph_cap > 0) {
     const bool same = c->graph_exec && c->graph_key_P == dP && c->graph_key_J == dJ && c->graph_key_K == dK &&
+                      c->graph_key_Pb == dPb && c->graph_key_Jb == dJb && c->graph_key_Kb == dKb &&
                       c->graph_key_mixed == mixed && c->graph_key_cutoff == c->opt.eri_schwarz_cutoff &&
                       c->graph_key_want == want && c->graph_key_mol_cut == c->use_mol_cut;
     if (!same) {
@@ -2687,10 +2781,11 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
           if (rc != TF_OK) return rc;
         }
       }
+      TF_TRY_RC(default_schedule(c, nullptr));
       int kernels = 0;
       cudaGraph_t graph = nullptr;
       TF_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      int rc = enqueue_graph_body(c, dP, dJ, dK, mixed, want, kernels);
+      int rc = enqueue_graph_body(c, dP, dJ, dK, dPb, dJb, dKb, mixed, want, kernels);
       cudaError_t ce = cudaStreamEndCapture(s, &graph);
       if (rc != TF_OK) { if (graph) cudaGraphDestroy(graph); return rc; }
       if (ce != cudaSuccess) { set_error(cudaGetErrorString(ce)); return TF_ECUDA; }
@@ -2698,6 +2793,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
       cudaGraphDestroy(graph);
       if (ce != cudaSuccess) { c->graph_exec = nullptr; set_error(cudaGetErrorString(ce)); return TF_ECUDA; }
       c->graph_key_P = dP; c->graph_key_J = dJ; c->graph_key_K = dK;
+      c->graph_key_Pb = dPb; c->graph_key_Jb = dJb; c->graph_key_Kb = dKb;
       c->graph_key_mixed = mixed;
       c->graph_key_cutoff = c->opt.eri_schwarz_cutoff;
       c->graph_key_want = want;
@@ -2766,6 +2862,11 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
     drop_graph(c);
     c->graph_cap = 0;
   }
+  // class-by-class builds proper (tf_set_graph 0) time each class pair's launches, so
+  // these follow one another; a build that only stands in for a graph build overlaps them
+  const bool timed = !c->use_graph;
+  if (!timed) TF_TRY_RC(default_schedule(c, goff.data()));
+  const int ns = timed ? 1 : sched_branches(c);
   for (size_t ci = 0; ci + 1 < chunk.size(); ++ci) {
     const int g0 = chunk[ci], g1 = chunk[ci + 1];
     const long long base = goff[3 * g0], nq = goff[3 * (g1 - 1) + 2] - base;
@@ -2781,11 +2882,13 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
                             c->d_quartets.p, s, kernels);
       if (rc) return rc;
     }
+    TF_TRY_RC(fork_branches(c, ns));
     for (int g = g0; g < g1; ++g) {
       int l1h, l1l, l2h, l2l;
       class_l(c->group_cls[g].x, l1h, l1l);
       class_l(c->group_cls[g].y, l2h, l2l);
-      TF_CUDA(cudaEventRecord(c->cls_ev[2 * g], s));
+      const cudaStream_t sg = branch_of(c, g, ns);
+      if (timed) TF_CUDA(cudaEventRecord(c->cls_ev[2 * g], s));
       JKArgs a{c->d_quartets.p + (goff[3 * g] - base), goff[3 * g + 1] - goff[3 * g], c->d_pairs.p,
                c->d_prim_full.p, c->d_prim_skip.p, c->d_Pc.p, c->d_Jc.p, c->d_Kc.p, c->d_mols.p,
                c->d_prim_count.p, nullptr, 0, LLONG_MAX, c->d_jkrec.p, c->d_pairR.p,
@@ -2804,24 +2907,25 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
       a32.n = goff[3 * g + 2] - goff[3 * g + 1];
       a32.bucket32 = 1;
       if (a.n > 0) {
-        rc = dispatch_jk(l1h, l1l, l2h, l2l, a, s, false, jk_variant(c, g));
+        rc = dispatch_jk(l1h, l1l, l2h, l2l, a, sg, false, jk_variant(c, g));
         if (rc != TF_OK) return rc;
         kernels++;
       }
       if (a32.n > 0) {
-        rc = dispatch_jk(l1h, l1l, l2h, l2l, a32, s, true, jk_variant(c, g));
+        rc = dispatch_jk(l1h, l1l, l2h, l2l, a32, sg, true, jk_variant(c, g));
         if (rc != TF_OK) return rc;
         kernels++;
       }
-      TF_CUDA(cudaEventRecord(c->cls_ev[2 * g + 1], s));
+      if (timed) TF_CUDA(cudaEventRecord(c->cls_ev[2 * g + 1], s));
     }
+    TF_TRY_RC(join_branches(c, ns));
   }
   (void)nq_total;
   rc = enqueue_finalize(c, dJ, dK, dJb, dKb, kernels);
   if (rc) return rc;
   TF_CUDA(cudaEventRecord(c->ev2, s));
   TF_CUDA(cudaStreamSynchronize(s));
-  return finish_stats(c, kernels, false);
+  return finish_stats(c, kernels, false, timed);
 }
 
 // Checks of one molecule's basis description, made before any device call: every
@@ -3111,17 +3215,8 @@ int tf_autotune(tf_ctx* c, const double* dP, double* dJ, double* dK, int flags, 
   int rc = set_device(c);
   if (rc) return rc;
   TF_CUDA(cudaDeviceSynchronize());    // dP may still be being written on any of the caller's streams
-  while ((int)c->side.size() < max_streams - 1) {
-    cudaStream_t x;
-    cudaEvent_t e;
-    TF_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
-    c->side.push_back(x);
-    TF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    c->join_ev.push_back(e);
-  }
-  if (!c->fork_ev) TF_CUDA(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
-  if (!c->list_fork_ev) TF_CUDA(cudaEventCreateWithFlags(&c->list_fork_ev, cudaEventDisableTiming));
-  if (!c->list_join_ev) TF_CUDA(cudaEventCreateWithFlags(&c->list_join_ev, cudaEventDisableTiming));
+  TF_TRY_RC(ensure_branches(c, max_streams));
+  c->sched_tuned = true;
   const bool use_graph = c->use_graph;
   tf_tune res{};
   const int ng = (int)c->group_cls.size();
