@@ -11,14 +11,17 @@ import os
 import shutil
 import subprocess
 import sys
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 LIB = os.path.join(HERE, "libtontofock.so")
 PEAK_LIB = os.path.join(HERE, "libtf_peak.so")
 
-SOURCES = ["tontofock.cu", "tf_mlp.cu"]
-DEPS = ["tontofock.cu", "tf_mlp.cu", "tf_device.cuh", "tf_warp.cuh", "tf_group.cuh", "rys_tables.inc", "boys_table.inc", "boys2_table.inc",
+SOURCES = ["tontofock.cu", "tf_jk_ss.cu", "tf_jk_ps.cu", "tf_jk_d.cu", "tf_jk_f.cu", "tf_rows_d.cu", "tf_rows_fs.cu",
+           "tf_rows_fd.cu", "tf_rows_ff.cu", "tf_mlp.cu"]
+DEPS = SOURCES + ["tf_device.cuh", "tf_thread.cuh", "tf_rows.cuh", "tf_warp.cuh", "rys_tables.inc", "boys_table.inc", "boys2_table.inc",
         os.path.join("..", "..", "include", "tontofock.h"), os.path.join("..", "..", "include", "tontofock_guess.h")]
 
 
@@ -52,10 +55,20 @@ def build(force: bool = False, verbose: bool = False) -> str:
     build_peak(force)
     if not force and up_to_date():
         return LIB
-    cmd = [nvcc()] + flags() + ["-o", LIB + ".tmp"] + [os.path.join(CSRC, s) for s in SOURCES]
-    if verbose:
-        print(" ".join(cmd))
-    subprocess.run(cmd, check=True, cwd=CSRC)
+    # one object per source, compiled side by side: the kernels are split over the
+    # sources by angular momentum so that they are
+    with tempfile.TemporaryDirectory() as tmp:
+        objs = [os.path.join(tmp, src + ".o") for src in SOURCES]
+
+        def compile_one(src: str, obj: str) -> None:
+            cmd = [nvcc()] + [f for f in flags() if f != "-shared"] + ["-c", "-o", obj, os.path.join(CSRC, src)]
+            if verbose:
+                print(" ".join(cmd), flush=True)
+            subprocess.run(cmd, check=True, cwd=CSRC)
+
+        with ThreadPoolExecutor(max_workers=os.cpu_count() or 1) as pool:
+            list(pool.map(compile_one, SOURCES, objs))
+        subprocess.run([nvcc()] + flags() + ["-o", LIB + ".tmp"] + objs, check=True, cwd=CSRC)
     os.replace(LIB + ".tmp", LIB)
     return LIB
 

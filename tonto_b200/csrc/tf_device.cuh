@@ -108,6 +108,9 @@ __device__ __forceinline__ void static_for(F&& f) {
 __host__ __device__ constexpr int ncart(int l) { return (l + 1) * (l + 2) / 2; }
 __host__ __device__ constexpr int ncart_upto(int l) { return l < 0 ? 0 : (l + 1) * (l + 2) * (l + 3) / 6; }
 
+// Switch key of a class (la lb|lc ld), l <= 3.
+__host__ __device__ constexpr int class_key(int la, int lb, int lc, int ld) { return ((la * 4 + lb) * 4 + lc) * 4 + ld; }
+
 constexpr int LCOMP = 8;                         // components tabulated up to l = 8
 constexpr int NCOMP_ALL = ncart_upto(LCOMP);     // 165
 

@@ -1,0 +1,17 @@
+// tf_jk_f.cu — thread kernels of the classes with an f shell (tf_thread.cuh).
+#include "tf_thread.cuh"
+
+namespace tf {
+
+bool launch_jk_f(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant) {
+  switch (key) {
+    case class_key(3, 0, 0, 0): launch_jk_f64<3, 0, 0, 0>(a, s, fp32, variant); return true;
+    case class_key(3, 0, 1, 0): launch_jk_f64<3, 0, 1, 0>(a, s, fp32, variant); return true;
+    case class_key(3, 1, 0, 0): launch_jk_f64<3, 1, 0, 0>(a, s, fp32, variant); return true;
+    case class_key(3, 2, 0, 0): launch_jk_f64<3, 2, 0, 0>(a, s, fp32, variant); return true;
+    case class_key(3, 3, 0, 0): launch_jk_f64<3, 3, 0, 0>(a, s, fp32, variant); return true;
+    default: return false;
+  }
+}
+
+}  // namespace tf

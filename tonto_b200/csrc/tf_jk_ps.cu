@@ -1,0 +1,15 @@
+// tf_jk_ps.cu — thread kernels of the |ps) kets (tf_thread.cuh).
+#include "tf_thread.cuh"
+
+namespace tf {
+
+bool launch_jk_ps(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant) {
+  switch (key) {
+    case class_key(1, 0, 1, 0): launch_jk<1, 0, 1, 0>(a, s, fp32, variant); return true;
+    case class_key(1, 1, 1, 0): launch_jk<1, 1, 1, 0>(a, s, fp32, variant); return true;
+    case class_key(2, 0, 1, 0): launch_jk<2, 0, 1, 0>(a, s, fp32, variant); return true;
+    default: return false;
+  }
+}
+
+}  // namespace tf

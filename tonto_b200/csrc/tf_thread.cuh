@@ -1,0 +1,449 @@
+// tf_thread.cuh — one thread per contracted quartet: the J/K kernels of the classes whose
+// (e0|f0) block fits a thread's registers, their launch arguments and launches.  The
+// classes are shared out over translation units (tf_jk_*.cu), which build in parallel.
+#pragma once
+#include "tf_device.cuh"
+
+#include <algorithm>
+
+namespace tf {
+
+constexpr int LMAX_SUPPORTED = 3;                 // s, p, d, f shells (f: the warp path)
+constexpr int NPAIRCLS = (LMAX_SUPPORTED + 1) * (LMAX_SUPPORTED + 2) / 2;
+constexpr int NQCLS = 625;                        // (la lb lc ld) counter slots, l <= 4
+// Counters of a build, zeroed with it and read back after it: primitive quartets per
+// class [0, NQCLS), the non-finite-density flag [NQCLS], contracted quartets per class
+// of the FP64 buckets [NQCLS + 1, 2 NQCLS + 1) and of the FP32 buckets after them.
+constexpr int BUILD_COUNTERS = 3 * NQCLS + 1;
+__host__ __device__ constexpr int pair_class(int lh, int ll) { return lh * (lh + 1) / 2 + ll; }
+__host__ __device__ constexpr int qclass_id(int la, int lb, int lc, int ld) { return ((la * 5 + lb) * 5 + lc) * 5 + ld; }
+// Bra-family members the thread kernel of a class holds at once (accumulator
+// capacity), for the classes where evaluating a bra family's primitive quartets once
+// measured faster on (H2O)32 cc-pVDZ: (ss|ss) 9.36 -> 8.36 ms, (ds|ss) 3.87 -> 3.63 ms.
+// (ps|ss), (ps|ps) and (ds|ps) measured slower with it (13.33 -> 13.45, 8.55 -> 8.90
+// and 4.29 -> 5.63 ms: the extra accumulators cost registers and the coefficient
+// loads and products every primitive quartet, and few of their bras are families),
+// so they, like every other class, take one member per list entry (capacity 1).
+__host__ __device__ constexpr int fam_cap_l(int la, int lb, int lc, int ld) {
+  return (la == 0 && lb == 0 && lc == 0 && ld == 0) ? 4 : (la == 2 && lb == 0 && lc == 0 && ld == 0) ? 2 : 1;
+}
+
+// ---------------------------------------------------------------------------
+// kernel: ERIs + digestion (one thread per contracted quartet)
+// ---------------------------------------------------------------------------
+struct JKArgs {
+  const int2* quartets;
+  long long n;
+  const PairRec* pairs;
+  const PrimPair* prim_full;
+  const PrimPair* prim_skip;
+  const double* P;              // Cartesian density (per-molecule blocks)
+  double* J;                    // Cartesian accumulators
+  double* K;
+  const MolInfo* mols;
+  unsigned long long* prim_count;   // per quartet class
+  // graph builds: the launch's quartets are list[range[0] - base, range[1] - base),
+  // range read on the device and clamped to base + cap (quartets = list start)
+  const long long* range;
+  long long base, cap;
+  const int4* jkrec;            // packed pair records (load_pair_jk)
+  const double2* pairR;
+  // unrestricted builds: the beta density and its J, K (else null); P, J, K above
+  // are then the alpha ones.  want: bit 0 J, bit 1 K.
+  const double* P2;
+  double* J2;
+  double* K2;
+  int want;
+  // bra families (family groups): per list entry the members' mask, per pair its
+  // family members; member quartets counted per class, FP64 buckets then FP32
+  const unsigned char* qmask;
+  const int4* fam_mem;
+  unsigned long long* qcount;
+  int fam;                      // bra-family capacity of the launch's kernel (1: none)
+  int bucket32;                 // 1: the launch covers the FP32 buckets
+  long long fx_lo;              // deterministic builds: offset of the lo words (fock_add), else 0
+};
+
+
+#ifndef TF_JK_MINB_N1
+#define TF_JK_MINB_N1 5
+#endif
+#ifndef TF_JK_MINB
+#define TF_JK_MINB 1
+#endif
+// Resident warps per SM, in units of four (bounds the registers per thread).
+// Variant 0 leaves the registers to the compiler (one-root classes: 20 warps);
+// variant 1 asks for more resident warps (24 for one root, 16 otherwise), at the
+// price of fewer registers.  The autotuner times the variants per class.
+template <int LA, int LB, int LC, int LD, int V>
+constexpr int jk_min_blocks() {
+  return Quartet<LA, LB, LC, LD>::NROOT == 1 ? ((V & 1) ? 6 : TF_JK_MINB_N1) : ((V & 1) ? 4 : TF_JK_MINB);
+}
+// Variant bits: 1 = more resident warps (see above); 2 = K atomics of lanes that hit
+// the same element summed first (segmented warp sums over lanes of one bra); 4 =
+// deterministic accumulation (fock_add), set by the context, not by the autotuner.
+constexpr int JK_VARIANTS = 4;
+// Threads per block: the resident warps of an SM form one block, so the SM holds
+// one copy of the shared Rys/Boys grid and leaves the rest of its shared storage to
+// the L1 cache, which serves the bra primitive records every iteration re-reads
+// (measured on (H2O)32, (ps|ss): L1 hit rate 42% -> 62%, 14.8 -> 13.7 ms against
+// five blocks of 128 threads).  A variant with no register bound uses up to 255
+// registers: 256 threads per SM.
+template <int LA, int LB, int LC, int LD, int V>
+constexpr int jk_threads() {
+  return jk_min_blocks<LA, LB, LC, LD, V>() == 1 ? 256 : 128 * jk_min_blocks<LA, LB, LC, LD, V>();
+}
+
+// Digestion of one quartet's Cartesian integrals I into J and K with the coincidence
+// factor f (f = 0: the lane adds nothing but still takes part in the warp sums):
+// bid is the bra pair (lanes of one bra are summed together), ob/oa the bra's and
+// oc/od the ket's first Cartesian functions.
+//   J(ab) += f sum_cd I P(cd);  J(cd) += f sum_ab I P(ab)  (per spin when unrestricted)
+//   K(ac) += f sum_bd I P(bd);  K(ad) += f sum_bc I P(bc)
+//   K(bc) += f sum_ad I P(ad);  K(bd) += f sum_ac I P(ac)
+// The lists are bra-major, so the lanes of a warp usually share the bra pair: then
+// J(ab) is summed over the warp and added once, and P(ab) is a broadcast.  Otherwise
+// the lanes of one bra are neighbours (a bra's kets of one cost bucket are
+// consecutive) and J(ab) is summed over each run of equal bras by a segmented warp
+// scan, then added by the run's last lane.  Variant bit 2: the K rows a and b are the
+// same for all lanes of one bra, and lanes whose kets share the c (or d) shell add to
+// the same K elements; such lanes are neighbours (pair-id order), so each run of
+// equal (bra, shell) keys is summed with a segmented warp scan and added once, by its
+// last lane.  K(bc), K(bd) are summed over a's components in registers first.
+template <int LA, int LB, int LC, int LD, int V>
+__device__ __forceinline__ void digest_jk(const JKArgs& a, const MolInfo& mi,
+                                          const double (&I)[ncart(LA)][ncart(LB)][ncart(LC) * ncart(LD)], double f,
+                                          int bid, int oa, int ob, int oc, int od) {
+  using Q = Quartet<LA, LB, LC, LD>;
+  constexpr bool FX = (V & 4) != 0;
+  const int lane = threadIdx.x & 31;
+  const bool live = f != 0.0;
+  const int n = mi.n_cart;
+  const bool uni = __all_sync(0xffffffffu, bid == __shfl_sync(0xffffffffu, bid, 0));
+  const unsigned lt_mask = lane == 31 ? 0xffffffffu : ((2u << lane) - 1u);
+  // (every lane executes the shuffle: none may be skipped by a short-circuit)
+  const int upx = __shfl_up_sync(0xffffffffu, bid, 1);
+  const bool headx = lane == 0 || bid != upx;
+  const unsigned heada = __ballot_sync(0xffffffffu, headx);
+  const int sega = 31 - __clz(heada & lt_mask);
+  const bool taila = lane == 31 || ((heada >> (lane + 1)) & 1u);
+  auto digest_j = [&](const double* __restrict__ P, double* __restrict__ Jm) {
+    double Pcd[Q::NC][Q::ND];
+#pragma unroll
+    for (int c = 0; c < Q::NC; ++c)
+#pragma unroll
+      for (int d = 0; d < Q::ND; ++d) Pcd[c][d] = __ldg(P + (size_t)(oc + c) * n + od + d);
+#pragma unroll
+    for (int ia = 0; ia < Q::NA; ++ia)
+#pragma unroll
+      for (int ib = 0; ib < Q::NB; ++ib) {
+        double s = 0.0;
+#pragma unroll
+        for (int c = 0; c < Q::NC; ++c)
+#pragma unroll
+          for (int d = 0; d < Q::ND; ++d) s += I[ia][ib][c * Q::ND + d] * Pcd[c][d];
+        s *= f;
+        if (uni) {
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+          if (lane == 0 && s != 0.0) fock_add<FX>(Jm + (size_t)(oa + ia) * n + ob + ib, s, a.fx_lo);
+        } else {                       // idle lanes join the last run with s = 0
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const double t = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane - o >= sega) s += t;
+          }
+          if (taila && s != 0.0) fock_add<FX>(Jm + (size_t)(oa + ia) * n + ob + ib, s, a.fx_lo);
+        }
+      }
+    if (live) {
+      double Pab[Q::NA][Q::NB];
+#pragma unroll
+      for (int ia = 0; ia < Q::NA; ++ia)
+#pragma unroll
+        for (int ib = 0; ib < Q::NB; ++ib) Pab[ia][ib] = __ldg(P + (size_t)(oa + ia) * n + ob + ib);
+#pragma unroll
+      for (int c = 0; c < Q::NC; ++c)
+#pragma unroll
+        for (int d = 0; d < Q::ND; ++d) {
+          double s = 0.0;
+#pragma unroll
+          for (int ia = 0; ia < Q::NA; ++ia)
+#pragma unroll
+            for (int ib = 0; ib < Q::NB; ++ib) s += I[ia][ib][c * Q::ND + d] * Pab[ia][ib];
+          fock_add<FX>(Jm + (size_t)(oc + c) * n + od + d, f * s, a.fx_lo);
+        }
+    }
+  };
+  if (a.want & 1) {                    // uniform over the warp (the J(ab) sums shuffle)
+    digest_j(a.P + mi.cmat, a.J + mi.cmat);
+    if (a.P2) digest_j(a.P2 + mi.cmat, a.J2 + mi.cmat);
+  }
+  constexpr bool SEG = (V & 2) != 0;
+  int segc = lane, segd = lane;
+  bool tailc = true, taild = true;
+  if constexpr (SEG) {
+    // (every lane executes both shuffles: none may be skipped by a short-circuit)
+    const int upc = __shfl_up_sync(0xffffffffu, oc, 1), upd = __shfl_up_sync(0xffffffffu, od, 1);
+    const unsigned headc = __ballot_sync(0xffffffffu, headx || oc != upc);
+    const unsigned headd = __ballot_sync(0xffffffffu, headx || od != upd);
+    segc = 31 - __clz(headc & lt_mask);
+    segd = 31 - __clz(headd & lt_mask);
+    tailc = lane == 31 || ((headc >> (lane + 1)) & 1u);
+    taild = lane == 31 || ((headd >> (lane + 1)) & 1u);
+  }
+  auto kadd = [&](double* addr, double v, int seg, bool tail) {
+    if constexpr (SEG) {
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const double t = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane - o >= seg) v += t;
+      }
+      if (tail && v != 0.0) fock_add<FX>(addr, v, a.fx_lo);
+    } else {
+      fock_add<FX>(addr, v, a.fx_lo);
+    }
+  };
+#define TF_KADD_C(addr, v) kadd((addr), (v), segc, tailc)
+#define TF_KADD_D(addr, v) kadd((addr), (v), segd, taild)
+  auto digest_k = [&](const double* __restrict__ P, double* __restrict__ Km) {
+    double Pbd[Q::NB][Q::ND], Pbc[Q::NB][Q::NC];
+    double Kbc[Q::NB][Q::NC], Kbd[Q::NB][Q::ND];
+#pragma unroll
+    for (int ib = 0; ib < Q::NB; ++ib) {
+#pragma unroll
+      for (int c = 0; c < Q::NC; ++c) Kbc[ib][c] = 0.0;
+#pragma unroll
+      for (int d = 0; d < Q::ND; ++d) Kbd[ib][d] = 0.0;
+    }
+#pragma unroll
+    for (int ib = 0; ib < Q::NB; ++ib) {
+#pragma unroll
+      for (int d = 0; d < Q::ND; ++d) Pbd[ib][d] = __ldg(P + (size_t)(ob + ib) * n + od + d);
+#pragma unroll
+      for (int c = 0; c < Q::NC; ++c) Pbc[ib][c] = __ldg(P + (size_t)(ob + ib) * n + oc + c);
+    }
+#pragma unroll
+    for (int ia = 0; ia < Q::NA; ++ia) {
+      double Pad[Q::ND], Pac[Q::NC];
+#pragma unroll
+      for (int d = 0; d < Q::ND; ++d) Pad[d] = __ldg(P + (size_t)(oa + ia) * n + od + d);
+#pragma unroll
+      for (int c = 0; c < Q::NC; ++c) Pac[c] = __ldg(P + (size_t)(oa + ia) * n + oc + c);
+#pragma unroll
+      for (int c = 0; c < Q::NC; ++c) {
+        double s = 0.0;
+#pragma unroll
+        for (int ib = 0; ib < Q::NB; ++ib)
+#pragma unroll
+          for (int d = 0; d < Q::ND; ++d) s += I[ia][ib][c * Q::ND + d] * Pbd[ib][d];
+        TF_KADD_C(Km + (size_t)(oa + ia) * n + oc + c, f * s);
+      }
+#pragma unroll
+      for (int d = 0; d < Q::ND; ++d) {
+        double s = 0.0;
+#pragma unroll
+        for (int ib = 0; ib < Q::NB; ++ib)
+#pragma unroll
+          for (int c = 0; c < Q::NC; ++c) s += I[ia][ib][c * Q::ND + d] * Pbc[ib][c];
+        TF_KADD_D(Km + (size_t)(oa + ia) * n + od + d, f * s);
+      }
+#pragma unroll
+      for (int ib = 0; ib < Q::NB; ++ib) {
+#pragma unroll
+        for (int c = 0; c < Q::NC; ++c)
+#pragma unroll
+          for (int d = 0; d < Q::ND; ++d) Kbc[ib][c] += I[ia][ib][c * Q::ND + d] * Pad[d];
+#pragma unroll
+        for (int d = 0; d < Q::ND; ++d)
+#pragma unroll
+          for (int c = 0; c < Q::NC; ++c) Kbd[ib][d] += I[ia][ib][c * Q::ND + d] * Pac[c];
+      }
+    }
+    // K(bc), K(bd): summed over the a components first, one atomic per element
+#pragma unroll
+    for (int ib = 0; ib < Q::NB; ++ib) {
+#pragma unroll
+      for (int c = 0; c < Q::NC; ++c) TF_KADD_C(Km + (size_t)(ob + ib) * n + oc + c, f * Kbc[ib][c]);
+#pragma unroll
+      for (int d = 0; d < Q::ND; ++d) TF_KADD_D(Km + (size_t)(ob + ib) * n + od + d, f * Kbd[ib][d]);
+    }
+  };
+  // with segmented sums every lane takes part (idle lanes add f = 0)
+  if ((SEG || live) && (a.want & 2)) {
+    digest_k(a.P + mi.cmat, a.K + mi.cmat);
+    if (a.P2) digest_k(a.P2 + mi.cmat, a.K2 + mi.cmat);
+  }
+#undef TF_KADD_C
+#undef TF_KADD_D
+}
+
+// Per-class counters of a launch, summed over the warp: primitive quartets, and
+// contracted (member) quartets of the FP64 or the FP32 buckets.
+__device__ __forceinline__ void count_quartets(const JKArgs& a, int cls, unsigned long long nprim,
+                                               unsigned long long nq) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    nprim += __shfl_xor_sync(0xffffffffu, nprim, o);
+    nq += __shfl_xor_sync(0xffffffffu, nq, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    if (nprim) atomicAdd(a.prim_count + cls, nprim);
+    if (nq) atomicAdd(a.qcount + (a.bucket32 ? NQCLS : 0) + cls, nq);
+  }
+}
+
+// One thread per contracted quartet.  MB = 1: a list entry is one quartet.  MB > 1
+// (family groups): a list entry is a bra family (its first member's pair id) with a
+// ket, and the mask of the members whose quartet passed the screen; the primitive
+// loop runs once for all members (accumulate_esfs_fam), then each member quartet of
+// the mask is transferred and digested with its own Cartesian offsets and
+// coincidence factors (molecule.fock.foo:1296-1300).
+template <int LA, int LB, int LC, int LD, typename T, int V, int MB>
+__global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArgs a) {
+  using Q = Quartet<LA, LB, LC, LD>;
+  using RS = RysSmem<Q::NROOT>;
+  extern __shared__ double rys_tab[];
+  RS::load(rys_tab);
+  __syncthreads();
+  unsigned long long nprim = 0, nquart = 0;
+  const int2* quartets = a.quartets;
+  long long nq = a.n;
+  long long qoff = 0;
+  resolve_range(a.range, a.base, a.cap, quartets, nq);
+  qoff = quartets - a.quartets;                      // offset of this launch's entries in the mask array
+  const long long stride = (long long)gridDim.x * blockDim.x;
+  const long long n_pad = (nq + 31) / 32 * 32;      // whole warps stay in the loop together
+  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n_pad; t += stride) {
+    // lanes past the end repeat the last quartet with weight 0, so that whole warps
+    // take part in the warp reductions below
+    const bool active = t < nq;
+    const long long te = active ? t : nq - 1;
+    const int2 qd = quartets[te];
+    const PairJK b = load_pair_jk(a.jkrec, a.pairR, qd.x);
+    const PairJK k = load_pair_jk(a.jkrec, a.pairR, qd.y);
+    const bool any_same = b.atom_hi == b.atom_lo || k.atom_hi == k.atom_lo || b.atom_hi == k.atom_hi ||
+                          b.atom_hi == k.atom_lo || b.atom_lo == k.atom_hi || b.atom_lo == k.atom_lo;
+    const PrimPair* bp = any_same ? a.prim_full + b.full_off : a.prim_skip + b.skip_off;
+    const PrimPair* kp = any_same ? a.prim_full + k.full_off : a.prim_skip + k.skip_off;
+    const int nbp = any_same ? b.n_full : b.n_skip;
+    const int nkp = any_same ? k.n_full : k.n_skip;
+    const double Rab[3] = {b.Rx, b.Ry, b.Rz};
+    const double Rcd[3] = {k.Rx, k.Ry, k.Rz};
+    const MolInfo mi = a.mols[b.mol];
+    double fk = 1.0;
+    if (k.same) fk *= 0.5;
+    if constexpr (MB == 1) {
+      if (active) { nprim += (unsigned long long)nbp * nkp; nquart += 1; }
+      double f = active ? fk : 0.0;
+      if (b.same) f *= 0.5;
+      if (qd.x == qd.y) f *= 0.5;
+      double I[Q::NA][Q::NB][Q::NC * Q::ND];
+      quartet_integrals<LA, LB, LC, LD, T>(bp, nbp, kp, nkp, Rab, Rcd, I, rys_tab);
+      digest_jk<LA, LB, LC, LD, V>(a, mi, I, f, qd.x, b.cart_hi, b.cart_lo, k.cart_hi, k.cart_lo);
+    } else {
+      const unsigned mask = active ? a.qmask[qoff + te] : 0u;
+      nprim += (unsigned long long)nbp * nkp * __popc(mask);
+      nquart += __popc(mask);
+      const int4 mv = a.fam_mem[qd.x];
+      const int mid[4] = {mv.x, mv.y, mv.z, mv.w};
+      PairJK bm[MB];
+      const PrimPair* bmp[MB];
+#pragma unroll
+      for (int m = 0; m < MB; ++m) {
+        bm[m] = load_pair_jk(a.jkrec, a.pairR, mid[m] >= 0 ? mid[m] : qd.x);
+        bmp[m] = mid[m] < 0 ? nullptr : (any_same ? a.prim_full + bm[m].full_off : a.prim_skip + bm[m].skip_off);
+      }
+      T esfs[MB][Q::NE][Q::NF];
+      accumulate_esfs_fam<LA, LB, LC, LD, T, MB>(bp, nbp, kp, nkp, bmp, esfs, rys_tab);
+#pragma unroll
+      for (int m = 0; m < MB; ++m) {
+        if (!__any_sync(0xffffffffu, (mask >> m) & 1u)) continue;      // uniform over the warp
+        double f = ((mask >> m) & 1u) ? fk : 0.0;
+        if (bm[m].same) f *= 0.5;
+        if (mid[m] == qd.y) f *= 0.5;
+        double I[Q::NA][Q::NB][Q::NC * Q::ND];
+        hrr_quartet<LA, LB, LC, LD, T>(esfs[m], Rab, Rcd, I);
+        digest_jk<LA, LB, LC, LD, V>(a, mi, I, f, mid[m] >= 0 ? mid[m] : qd.x, bm[m].cart_hi, bm[m].cart_lo,
+                                     k.cart_hi, k.cart_lo);
+      }
+    }
+  }
+  count_quartets(a, qclass_id(LA, LB, LC, LD), nprim, nquart);
+}
+
+// Launch set-up (shared-memory attribute, resident blocks per SM), done once per
+// kernel and before any graph capture: a zero-sized, range-less JKArgs only sets up.
+template <int LA, int LB, int LC, int LD, typename T, int V, int MB>
+static void launch_jk_t(const JKArgs& a, cudaStream_t s) {
+  constexpr int thr = jk_threads<LA, LB, LC, LD, V>();
+  constexpr size_t smem = RysSmem<Quartet<LA, LB, LC, LD>::NROOT>::SIZE * sizeof(double);
+  static int blocks_per_sm = -1;
+  if (blocks_per_sm < 0) {
+    cudaFuncSetAttribute(k_jk<LA, LB, LC, LD, T, V, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    {                                  // shared storage for one block, the rest to L1
+      int dev = 0, per_sm = 0;
+      cudaGetDevice(&dev);
+      cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+      const int pct = per_sm > 0 ? std::min(100, (int)((smem + 2048) * 100 / per_sm) + 1) : 100;
+      cudaFuncSetAttribute(k_jk<LA, LB, LC, LD, T, V, MB>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
+    }
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_jk<LA, LB, LC, LD, T, V, MB>, thr, smem);
+    if (blocks_per_sm < 1) blocks_per_sm = 1;
+  }
+  if (a.n <= 0 && !a.range) return;
+  int dev = 0, nsm = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  const long long full = (long long)nsm * blocks_per_sm;
+  const long long blocks = a.range ? full : std::min<long long>((a.n + thr - 1) / thr, full);
+  k_jk<LA, LB, LC, LD, T, V, MB><<<(unsigned)blocks, thr, smem, s>>>(a);
+}
+
+template <int LA, int LB, int LC, int LD, int V, int MB>
+static void launch_jk_v(const JKArgs& a, cudaStream_t s, bool fp32) {
+  if (fp32) launch_jk_t<LA, LB, LC, LD, float, V, MB>(a, s);
+  else launch_jk_t<LA, LB, LC, LD, double, V, MB>(a, s);
+}
+
+template <int LA, int LB, int LC, int LD, int MB>
+static void launch_jk_m(const JKArgs& a, cudaStream_t s, bool fp32, int variant) {
+  switch (variant & 7) {
+    case 1: launch_jk_v<LA, LB, LC, LD, 1, MB>(a, s, fp32); break;
+    case 2: launch_jk_v<LA, LB, LC, LD, 2, MB>(a, s, fp32); break;
+    case 3: launch_jk_v<LA, LB, LC, LD, 3, MB>(a, s, fp32); break;
+    case 4: case 6: launch_jk_v<LA, LB, LC, LD, 6, MB>(a, s, fp32); break;   // deterministic: always bit 2
+    case 5: case 7: launch_jk_v<LA, LB, LC, LD, 7, MB>(a, s, fp32); break;
+    default: launch_jk_v<LA, LB, LC, LD, 0, MB>(a, s, fp32); break;
+  }
+}
+
+// The bra-family kernel of the class (fam_cap_l) when the launch is a family group.
+template <int LA, int LB, int LC, int LD>
+static void launch_jk(const JKArgs& a, cudaStream_t s, bool fp32, int variant) {
+  constexpr int CAP = fam_cap_l(LA, LB, LC, LD);
+  if constexpr (CAP > 1) {
+    if (a.fam > 1) {
+      launch_jk_m<LA, LB, LC, LD, CAP>(a, s, fp32, variant);
+      return;
+    }
+  }
+  launch_jk_m<LA, LB, LC, LD, 1>(a, s, fp32, variant);
+}
+
+// Classes with an f shell: FP64 for the FP32 buckets too, and the two instantiations that
+// differ in their results' bits only (deterministic or not): their launches are too small
+// a share of a build for the register-bounded variants to matter.
+template <int LA, int LB, int LC, int LD>
+static void launch_jk_f64(const JKArgs& a, cudaStream_t s, bool, int variant) {
+  if (variant & 4) launch_jk_t<LA, LB, LC, LD, double, 6, 1>(a, s);
+  else launch_jk_t<LA, LB, LC, LD, double, 0, 1>(a, s);
+}
+
+// The classes of one translation unit each (tf_jk_*.cu); false: not a class of that unit.
+bool launch_jk_ss(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+bool launch_jk_ps(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+bool launch_jk_d(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+bool launch_jk_f(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+
+}  // namespace tf

@@ -1,10 +1,9 @@
 // tf_warp.cuh — warp-cooperative shell quartets with runtime angular momenta, used
-// for the Schwarz diagonal (ab|ab) of the pair classes above the thread kernels
-// (the (e0|f0) block, up to 31 x 31 for (dd|dd), does not fit one thread's
-// registers; the J/K builds of those classes use the lane-group kernels of
-// tf_group.cuh), and for everything with an f shell: its Schwarz bounds and its
-// J/K quartets (k_jk_warp), in a per-warp scratch area of global memory (up to
-// 248 KB for (ff|ff)).  One warp computes one contracted quartet:
+// for the Schwarz diagonal (ab|ab) of the pair classes above the thread kernels (the
+// (e0|f0) block, up to 31 x 31 for (dd|dd), does not fit one thread's registers; the
+// J/K builds of those classes use the lane-group kernels of tf_rows.cuh): in shared
+// memory up to d shells, with an f shell in a per-warp scratch area of global memory
+// (up to 248 KB for (ff|ff)).  One warp computes one contracted quartet:
 //   * every lane evaluates the Rys nodes/weights of the primitive quartet
 //     (warp-uniform table reads);
 //   * lanes (direction, root) build the 2D recurrence tables in shared memory;
@@ -47,7 +46,7 @@ constexpr int w_buf_need(int L) {
 constexpr int W_I2D = w_i2d_need(2);            // 375
 constexpr int W_BUF = w_buf_need(2);
 constexpr int W_SMEM = W_I2D + 2 * W_BUF;
-// up to f (quartets with an f shell, in global scratch)
+// up to f (pairs with an f shell, in global scratch)
 constexpr int WF_I2D = w_i2d_need(3);           // 1029
 constexpr int WF_BUF = w_buf_need(3);
 constexpr int WF_SCRATCH = WF_I2D + 2 * WF_BUF;
