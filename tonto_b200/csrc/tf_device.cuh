@@ -230,6 +230,21 @@ __device__ __forceinline__ void resolve_range(const long long* range, long long 
   }
 }
 
+// Cost buckets of the primitive-quartet count npq: npq itself below 8, then quarter
+// octaves (counts within a factor 1.19 share a bucket), so that the lanes of a warp
+// loop over nearly the same number of primitive quartets.
+constexpr int NCOST = 47;
+constexpr int NBUCKET = 2 * NCOST;         // FP64 buckets, then FP32 buckets
+
+// Work of one thread-kernel launch, computed on the device from the list's bucket counts
+// (k_group_offsets): the buckets, heaviest first, each cut into warps.  Bucket j holds
+// list entries [item0[j], item0[j] + count[j]); 2^lg[j] neighbouring lanes share one
+// entry's primitive quartets; warps [warp0[j], warp0[j + 1]) work on it.
+struct LaunchPlan {
+  long long item0[NCOST], count[NCOST], warp0[NCOST + 1];
+  int lg[NCOST];
+};
+
 // One molecule of a (possibly batched) context: its shells are a contiguous
 // global range; its matrices sit at fixed offsets in the concatenated buffers.
 struct __align__(16) MolInfo {
@@ -650,9 +665,12 @@ __device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& 
 // per-iteration bra loads are warp-wide broadcasts and each lane's ket record is
 // read once per ket primitive, one iteration ahead.  (Two primitive quartets per
 // iteration as independent chains measured no faster on (H2O)32.)
+// p0, npq: the share of the quartet's nbp x nkp primitive quartets to add up (flat
+// indices p0 .. p0 + npq - 1, p = ket * nbp + bra): all of them, or one lane's part where
+// several lanes share a quartet.
 template <int LA, int LB, int LC, int LD, typename T>
 __device__ __forceinline__ void accumulate_esfs(const PrimPair* __restrict__ bp, int nbp,
-                                                const PrimPair* __restrict__ kp, int nkp,
+                                                const PrimPair* __restrict__ kp, int nkp, int p0, int npq,
                                                 T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                 const double* __restrict__ rys_smem = nullptr) {
   using Q = Quartet<LA, LB, LC, LD>;
@@ -661,12 +679,11 @@ __device__ __forceinline__ void accumulate_esfs(const PrimPair* __restrict__ bp,
   for (int e = 0; e < Q::NE; ++e)
 #pragma unroll
     for (int f = 0; f < Q::NF; ++f) esfs[e][f] = T(0);
-  const int npq = nbp * nkp;
   if (npq <= 0) return;
   const double2* bq = reinterpret_cast<const double2*>(bp);
   const double2* kq = reinterpret_cast<const double2*>(kp);
-  int ib = 0, ik = 0;
-  PrimRegs kc = load_prim<KPA>(kq, 0);
+  int ik = p0 ? p0 / nbp : 0, ib = p0 - ik * nbp;
+  PrimRegs kc = load_prim<KPA>(kq, ik);
 #pragma unroll(kPrimUnroll)
   for (int p = 0; p < npq; ++p) {
     const PrimRegs b = load_prim<BPA>(bq, ib);
@@ -788,7 +805,7 @@ __device__ __forceinline__ void hrr_bra(const T (&G)[CT.first[LA + LB + 1] - CT.
 // with that member's coefficient product (bm[m][ib].cc; bm[m] null: no member m).
 template <int LA, int LB, int LC, int LD, typename T, int MB>
 __device__ __forceinline__ void accumulate_esfs_fam(const PrimPair* __restrict__ bp, int nbp,
-                                                    const PrimPair* __restrict__ kp, int nkp,
+                                                    const PrimPair* __restrict__ kp, int nkp, int p0, int npq,
                                                     const PrimPair* const (&bm)[MB],
                                                     T (&esfs)[MB][Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                     const double* __restrict__ rys_smem) {
@@ -800,12 +817,11 @@ __device__ __forceinline__ void accumulate_esfs_fam(const PrimPair* __restrict__
     for (int e = 0; e < Q::NE; ++e)
 #pragma unroll
       for (int f = 0; f < Q::NF; ++f) esfs[m][e][f] = T(0);
-  const int npq = nbp * nkp;
   if (npq <= 0) return;
   const double2* bq = reinterpret_cast<const double2*>(bp);
   const double2* kq = reinterpret_cast<const double2*>(kp);
-  int ib = 0, ik = 0;
-  PrimRegs kc = load_prim<KPA>(kq, 0);
+  int ik = p0 ? p0 / nbp : 0, ib = p0 - ik * nbp;
+  PrimRegs kc = load_prim<KPA>(kq, ik);
   for (int p = 0; p < npq; ++p) {
     PrimRegs b = load_prim<BPA>(bq, ib);
     double cb[MB];
@@ -866,7 +882,7 @@ __device__ __forceinline__ void quartet_integrals(const PrimPair* bp, int nbp, c
                                                   const double* __restrict__ rys_smem = nullptr) {
   using Q = Quartet<LA, LB, LC, LD>;
   T esfs[Q::NE][Q::NF];
-  accumulate_esfs<LA, LB, LC, LD, T>(bp, nbp, kp, nkp, esfs, rys_smem);
+  accumulate_esfs<LA, LB, LC, LD, T>(bp, nbp, kp, nkp, 0, nbp * nkp, esfs, rys_smem);
   double ed[Q::NE][Q::NF];
 #pragma unroll
   for (int e = 0; e < Q::NE; ++e)

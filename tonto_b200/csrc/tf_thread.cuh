@@ -42,10 +42,12 @@ struct JKArgs {
   double* K;
   const MolInfo* mols;
   unsigned long long* prim_count;   // per quartet class
-  // graph builds: the launch's quartets are list[range[0] - base, range[1] - base),
-  // range read on the device and clamped to base + cap (quartets = list start)
+  // the list's memory (quartets) starts at list entry base; a thread kernel reads its
+  // entries from its plan, a lane-group kernel takes list[range[0] - base, range[1] - base)
+  // (graph builds: read on the device and clamped to base + cap) or n entries from first
+  const LaunchPlan* plan;
   const long long* range;
-  long long base, cap;
+  long long base, cap, first;
   const int4* jkrec;            // packed pair records (load_pair_jk)
   const double2* pairR;
   // unrestricted builds: the beta density and its J, K (else null); P, J, K above
@@ -293,7 +295,10 @@ __device__ __forceinline__ void count_quartets(const JKArgs& a, int cls, unsigne
   }
 }
 
-// One thread per contracted quartet.  MB = 1: a list entry is one quartet.  MB > 1
+// One thread per contracted quartet, or, in the buckets whose quartets have so many
+// primitive quartets that they would outlast the rest of the launch, 2, 4, .. 32
+// neighbouring lanes (LaunchPlan): each adds up a share, the shares are summed by
+// shuffles and one lane digests.  MB = 1: a list entry is one quartet.  MB > 1
 // (family groups): a list entry is a bra family (its first member's pair id) with a
 // ket, and the mask of the members whose quartet passed the screen; the primitive
 // loop runs once for all members (accumulate_esfs_fam), then each member quartet of
@@ -304,22 +309,30 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
   using Q = Quartet<LA, LB, LC, LD>;
   using RS = RysSmem<Q::NROOT>;
   extern __shared__ double rys_tab[];
+  __shared__ LaunchPlan plan;
+  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  const long long n_warps = a.plan->warp0[NCOST], stride = (long long)gridDim.x * (blockDim.x >> 5);
+  // a long list: the warps of an SM take neighbouring entries (one bra's records serve them
+  // all from L1); a short one is spread over the SMs
+  const bool spread = n_warps < 4 * stride;
+  if ((spread ? (long long)blockIdx.x : (long long)blockIdx.x * (blockDim.x >> 5)) >= n_warps) return;
+  for (int q = threadIdx.x; q < (int)(sizeof(LaunchPlan) / sizeof(int)); q += blockDim.x)
+    reinterpret_cast<int*>(&plan)[q] = __ldg(reinterpret_cast<const int*>(a.plan) + q);
   RS::load(rys_tab);
   __syncthreads();
   unsigned long long nprim = 0, nquart = 0;
-  const int2* quartets = a.quartets;
-  long long nq = a.n;
-  long long qoff = 0;
-  resolve_range(a.range, a.base, a.cap, quartets, nq);
-  qoff = quartets - a.quartets;                      // offset of this launch's entries in the mask array
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  const long long n_pad = (nq + 31) / 32 * 32;      // whole warps stay in the loop together
-  for (long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x; t < n_pad; t += stride) {
-    // lanes past the end repeat the last quartet with weight 0, so that whole warps
+  int seg = 0;
+  for (long long w = spread ? (long long)wib * gridDim.x + blockIdx.x : (long long)blockIdx.x * (blockDim.x >> 5) + wib;
+       w < n_warps; w += stride) {
+    while (w >= plan.warp0[seg + 1]) ++seg;
+    const int lg = plan.lg[seg], sub = lane & ((1 << lg) - 1);
+    const long long at = (w - plan.warp0[seg]) * (32 >> lg) + (lane >> lg);
+    // lanes past the end repeat the bucket's last entry with weight 0, so that whole warps
     // take part in the warp reductions below
-    const bool active = t < nq;
-    const long long te = active ? t : nq - 1;
-    const int2 qd = quartets[te];
+    const bool in_list = at < plan.count[seg];
+    const bool active = in_list && sub == 0;          // the lane that digests and counts the entry
+    const long long te = plan.item0[seg] + (in_list ? at : plan.count[seg] - 1) - a.base;
+    const int2 qd = a.quartets[te];
     const PairJK b = load_pair_jk(a.jkrec, a.pairR, qd.x);
     const PairJK k = load_pair_jk(a.jkrec, a.pairR, qd.y);
     const bool any_same = b.atom_hi == b.atom_lo || k.atom_hi == k.atom_lo || b.atom_hi == k.atom_hi ||
@@ -330,6 +343,10 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
     const int nkp = any_same ? k.n_full : k.n_skip;
     const double Rab[3] = {b.Rx, b.Ry, b.Rz};
     const double Rcd[3] = {k.Rx, k.Ry, k.Rz};
+    // this lane's share of the primitive quartets
+    const int npq = nbp * nkp;
+    const int p0 = lg ? (int)((long long)npq * sub >> lg) : 0;
+    const int np = lg ? (int)((long long)npq * (sub + 1) >> lg) - p0 : npq;
     const MolInfo mi = a.mols[b.mol];
     double fk = 1.0;
     if (k.same) fk *= 0.5;
@@ -339,10 +356,17 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
       if (b.same) f *= 0.5;
       if (qd.x == qd.y) f *= 0.5;
       double I[Q::NA][Q::NB][Q::NC * Q::ND];
-      quartet_integrals<LA, LB, LC, LD, T>(bp, nbp, kp, nkp, Rab, Rcd, I, rys_tab);
+      T esfs[Q::NE][Q::NF];
+      accumulate_esfs<LA, LB, LC, LD, T>(bp, nbp, kp, nkp, p0, np, esfs, rys_tab);
+      for (int o = 1; o < 1 << lg; o <<= 1)
+#pragma unroll
+        for (int e = 0; e < Q::NE; ++e)
+#pragma unroll
+          for (int q = 0; q < Q::NF; ++q) esfs[e][q] += __shfl_xor_sync(0xffffffffu, esfs[e][q], o);
+      hrr_quartet<LA, LB, LC, LD, T>(esfs, Rab, Rcd, I);
       digest_jk<LA, LB, LC, LD, V>(a, mi, I, f, qd.x, b.cart_hi, b.cart_lo, k.cart_hi, k.cart_lo);
     } else {
-      const unsigned mask = active ? a.qmask[qoff + te] : 0u;
+      const unsigned mask = active ? a.qmask[te] : 0u;
       nprim += (unsigned long long)nbp * nkp * __popc(mask);
       nquart += __popc(mask);
       const int4 mv = a.fam_mem[qd.x];
@@ -355,7 +379,14 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
         bmp[m] = mid[m] < 0 ? nullptr : (any_same ? a.prim_full + bm[m].full_off : a.prim_skip + bm[m].skip_off);
       }
       T esfs[MB][Q::NE][Q::NF];
-      accumulate_esfs_fam<LA, LB, LC, LD, T, MB>(bp, nbp, kp, nkp, bmp, esfs, rys_tab);
+      accumulate_esfs_fam<LA, LB, LC, LD, T, MB>(bp, nbp, kp, nkp, p0, np, bmp, esfs, rys_tab);
+      for (int o = 1; o < 1 << lg; o <<= 1)
+#pragma unroll
+        for (int m = 0; m < MB; ++m)
+#pragma unroll
+          for (int e = 0; e < Q::NE; ++e)
+#pragma unroll
+            for (int q = 0; q < Q::NF; ++q) esfs[m][e][q] += __shfl_xor_sync(0xffffffffu, esfs[m][e][q], o);
 #pragma unroll
       for (int m = 0; m < MB; ++m) {
         if (!__any_sync(0xffffffffu, (mask >> m) & 1u)) continue;      // uniform over the warp
@@ -391,12 +422,13 @@ static void launch_jk_t(const JKArgs& a, cudaStream_t s) {
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_jk<LA, LB, LC, LD, T, V, MB>, thr, smem);
     if (blocks_per_sm < 1) blocks_per_sm = 1;
   }
-  if (a.n <= 0 && !a.range) return;
+  if (!a.plan) return;
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   const long long full = (long long)nsm * blocks_per_sm;
-  const long long blocks = a.range ? full : std::min<long long>((a.n + thr - 1) / thr, full);
+  // (n known: at most a warp an entry)
+  const long long blocks = a.range ? full : std::min<long long>((a.n * 32 + thr - 1) / thr, full);
   k_jk<LA, LB, LC, LD, T, V, MB><<<(unsigned)blocks, thr, smem, s>>>(a);
 }
 

@@ -261,11 +261,6 @@ __global__ void k_pmax(BatchArgs b, const double* __restrict__ P, const double* 
 // ---------------------------------------------------------------------------
 // kernels: quartet lists
 // ---------------------------------------------------------------------------
-// Cost buckets of the primitive-quartet count npq: npq itself below 8, then quarter
-// octaves (counts within a factor 1.19 share a bucket), so that the lanes of a warp
-// loop over nearly the same number of primitive quartets.
-constexpr int NCOST = 47;
-constexpr int NBUCKET = 2 * NCOST;         // FP64 buckets, then FP32 buckets
 static_assert(NBUCKET < 0xff, "bucket ids are recorded as bytes, 0xff = screened out");
 
 // One (class pair, molecule) unit of the list builder.  Units of the same class
@@ -1112,6 +1107,7 @@ struct tf_ctx {
   tf::DBuf<double2> d_pairR;
   tf::DBuf<long long> d_task_cand_off;
   tf::DBuf<long long> d_counts, d_offsets, d_group_offsets;
+  tf::DBuf<tf::LaunchPlan> d_plans;                      // per group: its FP64 and its FP32 launch
   tf::DBuf<double> d_mol_cut;                            // per-molecule cutoffs (tf_set_molecule_cutoffs)
   bool use_mol_cut = false;
   tf::DBuf<unsigned long long> d_pglob, d_prim_count;
@@ -1170,24 +1166,77 @@ static BatchArgs batch_args(tf_ctx* c) {
                    c->d_shell_nbf.p,  c->spherical};
 }
 
-// gather (start, FP32 start, end) of every group's quartet range, and the list
-// length at out[3 n_groups].  A list longer than cap (the buffer of a captured
-// build) gets empty ranges: that build's class launches do nothing, and the host,
+// Lanes per quartet of a launch (LaunchPlan::lg).  A launch cannot end before its longest
+// quartet, so no lane should get more primitive quartets than its fair share of the
+// launch, taken over PLAN_LANES resident lanes (148 SMs, 12 warps) with a factor
+// 2 of slack, nor fewer than PLAN_MIN: beyond that the split costs more (one lane of
+// the sharers digests) than its shorter chain saves.  Measured, (ss|ss) and the whole
+// build, one thread a quartet throughout -> split: (H2O)2 cc-pVTZ 1.32 -> 0.06 and 2.12 -> 0.87
+// ms, (H2O)3 6-31G(d) 0.35 -> 0.02 and 0.54 -> 0.31, (H2O)7 cc-pVDZ 1.77 -> 0.34 and 2.04 ->
+// 1.68; (H2O)32 cc-pVDZ, where few buckets are split, 72.7 -> 73.0 ms.
+constexpr double PLAN_LANES = 148.0 * 12 * 32;
+constexpr int PLAN_MIN = 12;
+
+// (start, FP32 start, end) of every group's quartet range, the list length at
+// out[3 n_groups], and the launch plans of the group's FP64 and FP32 buckets.  One block
+// of two warps per group.  A list longer than cap (the buffer of a captured build) gets
+// empty ranges and plans: that build's class launches do nothing, and the host,
 // seeing the length, redoes the build with a larger buffer.
-__global__ void k_group_offsets(int n_groups, const int* __restrict__ group_task0, const long long* __restrict__ offs,
-                                long long cap, long long* __restrict__ out) {
-  const int g = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(64) k_group_offsets(int n_groups, const int* __restrict__ group_task0,
+                                                      const long long* __restrict__ offs, long long cap,
+                                                      long long* __restrict__ out, LaunchPlan* __restrict__ plans) {
+  const int g = blockIdx.x, half = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (g >= n_groups) return;
   const long long total = offs[(long long)group_task0[n_groups] * NBUCKET];
-  if (g == 0) out[3 * n_groups] = total;
-  if (total > cap) {
-    out[3 * g] = out[3 * g + 1] = out[3 * g + 2] = 0;
-    return;
+  const long long t0 = group_task0[g], t1 = group_task0[g + 1], nt = t1 - t0;
+  const bool fits = total <= cap;
+  if (threadIdx.x == 0) {
+    if (g == 0) out[3 * n_groups] = total;
+    out[3 * g] = fits ? offs[t0 * NBUCKET] : 0;
+    out[3 * g + 1] = fits ? offs[t0 * NBUCKET + (long long)NCOST * nt] : 0;
+    out[3 * g + 2] = fits ? offs[t1 * NBUCKET] : 0;
   }
-  const long long t0 = group_task0[g], t1 = group_task0[g + 1];
-  out[3 * g] = offs[t0 * NBUCKET];
-  out[3 * g + 1] = offs[t0 * NBUCKET + (long long)NCOST * (t1 - t0)];
-  out[3 * g + 2] = offs[t1 * NBUCKET];
+  // lane's buckets, heaviest first: j = lane and lane + 32
+  LaunchPlan& plan = plans[2 * g + half];
+  long long i0[2], n[2], cost[2];
+  double work = 0.0;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int j = lane + 32 * q, k = NCOST - 1 - j;
+    i0[q] = n[q] = cost[q] = 0;
+    if (j < NCOST) {
+      i0[q] = offs[t0 * NBUCKET + (long long)(half * NCOST + k) * nt];
+      n[q] = fits ? offs[t0 * NBUCKET + (long long)(half * NCOST + k + 1) * nt] - i0[q] : 0;
+      // the bucket's largest count (cost_bucket); the last one has no upper end
+      cost[q] = k < 7 ? k + 1 : ((5LL + (k - 7) % 4) << ((k - 7) / 4 + 1));
+      work += (double)n[q] * (double)cost[q];
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) work += __shfl_xor_sync(0xffffffffu, work, o);
+  const double share = fmax((double)PLAN_MIN, 2.0 * work / PLAN_LANES);
+  long long start = 0;
+#pragma unroll
+  for (int q = 0; q < 2; ++q) {
+    const int j = lane + 32 * q;
+    int lg = 0;
+    while (lg < 5 && (double)cost[q] > share * (double)(1 << lg)) ++lg;
+    const long long warps = (n[q] + (32 >> lg) - 1) / (32 >> lg);
+    long long incl = warps;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const long long up = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += up;
+    }
+    if (j < NCOST) {
+      plan.item0[j] = i0[q];
+      plan.count[j] = n[q];
+      plan.lg[j] = lg;
+      plan.warp0[j] = start + incl - warps;
+      if (j == NCOST - 1) plan.warp0[NCOST] = start + incl;
+    }
+    start += __shfl_sync(0xffffffffu, incl, 31);
+  }
 }
 
 // Kernel variant of each class pair chosen by the last tf_autotune on a device; new
@@ -1558,6 +1607,7 @@ static int build_tasks(tf_ctx* c) {
   TF_CUDA(c->d_unit_group.reserve(std::max<size_t>(c->unit_group.size(), 1)));
   TF_CUDA(c->d_group_task0.reserve(ng + 1));
   TF_CUDA(c->d_group_offsets.reserve(3 * ng + 1));
+  TF_CUDA(c->d_plans.reserve(std::max<size_t>(2 * ng, 1)));
   TF_CUDA(c->d_tasks.reserve(std::max<size_t>(tasks.size(), 1)));
   if ((long long)tasks.size() * NBUCKET + 1 > 0x7fffffffLL) {    // the count scan indexes with int
     set_error("too many bra tasks for the quartet-list counts");
@@ -1759,7 +1809,7 @@ static int dispatch_jk(int la, int lb, int lc, int ld, const JKArgs& a, cudaStre
   if (launch_jk_ss(key, a, s, fp32, variant) || launch_jk_ps(key, a, s, fp32, variant) ||
       launch_jk_d(key, a, s, fp32, variant) || launch_jk_f(key, a, s, fp32, variant))
     return TF_OK;
-  const RowArgs r{a.quartets, a.n, a.prim_full, a.prim_skip, a.P, a.J, a.K, a.mols, a.prim_count, a.range, a.base,
+  const RowArgs r{a.quartets + (a.range ? 0 : a.first - a.base), a.n, a.prim_full, a.prim_skip, a.P, a.J, a.K, a.mols, a.prim_count, a.range, a.base,
                   a.cap, a.jkrec, a.pairR, a.P2, a.J2, a.K2, a.want,
                   a.qcount ? a.qcount + (a.bucket32 ? NQCLS : 0) : nullptr, a.fx_lo};
   for (auto* launch : {launch_rows_d, launch_rows_fs, launch_rows_fd, launch_rows_ff}) {
@@ -1884,7 +1934,8 @@ static int enqueue_counts(tf_ctx* c, const double* dP, const double* dPb, bool m
   TF_CUDA(cub::DeviceScan::ExclusiveSum(c->d_scan_tmp.p, tmp_bytes, c->d_counts.p, c->d_offsets.p, (int)(nslots + 1),
                                         s));
   const int ng = (int)c->group_cls.size();
-  k_group_offsets<<<(ng + 63) / 64, 64, 0, s>>>(ng, c->d_group_task0.p, c->d_offsets.p, cap, c->d_group_offsets.p);
+  k_group_offsets<<<std::max(ng, 1), 64, 0, s>>>(ng, c->d_group_task0.p, c->d_offsets.p, cap, c->d_group_offsets.p,
+                                                 c->d_plans.p);
   kernels += 3;
   const long long nacc = acc_elems(c);
   TF_CUDA(cudaMemsetAsync(c->d_Jc.p, 0, nacc * sizeof(double), s));
@@ -2032,8 +2083,8 @@ static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* d
     class_l(c->group_cls[g].y, l2h, l2l);
     cudaStream_t sg = branch_of(c, g, ns);
     JKArgs a{c->d_quartets.p, 0, c->d_pairs.p, c->d_prim_full.p, c->d_prim_skip.p, c->d_Pc.p, c->d_Jc.p,
-             c->d_Kc.p, c->d_mols.p, c->d_prim_count.p, c->d_group_offsets.p + 3 * g, 0, c->graph_cap,
-             c->d_jkrec.p, c->d_pairR.p, dPb ? c->d_PcB.p : nullptr, dPb ? c->d_JcB.p : nullptr,
+             c->d_Kc.p, c->d_mols.p, c->d_prim_count.p, c->d_plans.p + 2 * g, c->d_group_offsets.p + 3 * g, 0,
+             c->graph_cap, 0, c->d_jkrec.p, c->d_pairR.p, dPb ? c->d_PcB.p : nullptr, dPb ? c->d_JcB.p : nullptr,
              dPb ? c->d_KcB.p : nullptr, want};
     a.qmask = c->d_qmask.p;
     a.fam_mem = c->d_fam_mem.p;
@@ -2042,6 +2093,7 @@ static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* d
     a.bucket32 = 0;
     a.fx_lo = fx_offset(c);
     JKArgs a32 = a;
+    a32.plan = c->d_plans.p + 2 * g + 1;
     a32.range = c->d_group_offsets.p + 3 * g + 1;
     a32.bucket32 = 1;
     rc = dispatch_jk(l1h, l1l, l2h, l2l, a, sg, false, jk_variant(c, g));
@@ -2278,19 +2330,20 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
       class_l(c->group_cls[g].y, l2h, l2l);
       const cudaStream_t sg = branch_of(c, g, ns);
       if (timed) TF_CUDA(cudaEventRecord(c->cls_ev[2 * g], s));
-      JKArgs a{c->d_quartets.p + (goff[3 * g] - base), goff[3 * g + 1] - goff[3 * g], c->d_pairs.p,
+      JKArgs a{c->d_quartets.p, goff[3 * g + 1] - goff[3 * g], c->d_pairs.p,
                c->d_prim_full.p, c->d_prim_skip.p, c->d_Pc.p, c->d_Jc.p, c->d_Kc.p, c->d_mols.p,
-               c->d_prim_count.p, nullptr, 0, LLONG_MAX, c->d_jkrec.p, c->d_pairR.p,
+               c->d_prim_count.p, c->d_plans.p + 2 * g, nullptr, base, LLONG_MAX, goff[3 * g], c->d_jkrec.p,
+               c->d_pairR.p,
                dPb ? c->d_PcB.p : nullptr, dPb ? c->d_JcB.p : nullptr, dPb ? c->d_KcB.p : nullptr, want};
-      a.qmask = c->d_qmask.p + (goff[3 * g] - base);
+      a.qmask = c->d_qmask.p;
       a.fam_mem = c->d_fam_mem.p;
       a.qcount = c->d_prim_count.p + NQCLS + 1;
       a.fam = c->group_fam[g];
       a.bucket32 = 0;
       a.fx_lo = fx_offset(c);
       JKArgs a32 = a;
-      a32.quartets = c->d_quartets.p + (goff[3 * g + 1] - base);
-      a32.qmask = c->d_qmask.p + (goff[3 * g + 1] - base);
+      a32.plan = c->d_plans.p + 2 * g + 1;
+      a32.first = goff[3 * g + 1];
       a32.n = goff[3 * g + 2] - goff[3 * g + 1];
       a32.bucket32 = 1;
       if (a.n > 0) {
