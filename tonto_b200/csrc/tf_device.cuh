@@ -305,7 +305,7 @@ __device__ __forceinline__ void rys_eval(double x, double (&u)[N], double (&w)[N
 // The same tables staged in shared memory, transposed to [coef][function][interval]
 // so that lanes evaluating different intervals hit different banks.
 template <int N>
-struct RysSmem {
+struct RysPoly {
   static constexpr int NI = rys_xmax(N);              // intervals
   static constexpr int SIZE = TF_RYS_NCOEF * 2 * N * NI;
   // layout [k][j][i] with the pairs (u_i, w_i) adjacent: one 16-byte load per
@@ -351,6 +351,9 @@ struct RysSmem {
     }
   }
 };
+
+template <int N>
+struct RysSmem : RysPoly<N> {};
 
 // One root: the rule is exact for f linear in t^2, so w = F0(x) and u = F1(x)/F0(x).
 // F0 and F1 come from an 8-term Taylor step about the nearest point k/8 of a grid
@@ -857,32 +860,6 @@ __device__ __forceinline__ void hrr_quartet(const T (&esfs)[Quartet<LA, LB, LC, 
                                             const double* Rab, const double* Rcd,
                                             double (&abcd)[ncart(LA)][ncart(LB)][ncart(LC) * ncart(LD)]) {
   using Q = Quartet<LA, LB, LC, LD>;
-  double ed[Q::NE][Q::NF];
-#pragma unroll
-  for (int e = 0; e < Q::NE; ++e)
-#pragma unroll
-    for (int f = 0; f < Q::NF; ++f) ed[e][f] = (double)esfs[e][f];
-  double ket[Q::NE][Q::NC][Q::ND];
-  hrr_ket<LC, LD, Q::NE, double>(ed, Rcd, ket);
-  double flat[Q::NE][Q::NC * Q::ND];
-#pragma unroll
-  for (int e = 0; e < Q::NE; ++e)
-#pragma unroll
-    for (int c = 0; c < Q::NC; ++c)
-#pragma unroll
-      for (int d = 0; d < Q::ND; ++d) flat[e][c * Q::ND + d] = ket[e][c][d];
-  hrr_bra<LA, LB, Q::NC * Q::ND, double>(flat, Rab, abcd);
-}
-
-// Contracted Cartesian integrals (ab|cd) of one quartet, as double.
-template <int LA, int LB, int LC, int LD, typename T>
-__device__ __forceinline__ void quartet_integrals(const PrimPair* bp, int nbp, const PrimPair* kp, int nkp,
-                                                  const double* Rab, const double* Rcd,
-                                                  double (&abcd)[ncart(LA)][ncart(LB)][ncart(LC) * ncart(LD)],
-                                                  const double* __restrict__ rys_smem = nullptr) {
-  using Q = Quartet<LA, LB, LC, LD>;
-  T esfs[Q::NE][Q::NF];
-  accumulate_esfs<LA, LB, LC, LD, T>(bp, nbp, kp, nkp, 0, nbp * nkp, esfs, rys_smem);
   double ed[Q::NE][Q::NF];
 #pragma unroll
   for (int e = 0; e < Q::NE; ++e)

@@ -117,18 +117,33 @@ __global__ void k_pair_prep(int n_pairs, PairRec* __restrict__ pairs, const doub
   pairs[p] = pr;
 }
 
+// Schwarz bounds, one warp per pair: the lanes share the pair's n^2 primitive quartets
+// (up to 4,096 for two eight-primitive shells: on one thread (H2O)9 cc-pVDZ's (ss|ss) took
+// 1.17 ms; tf_set_geometry of that cluster, with its host lists, 3.9 -> 1.7 ms), sum the (e0|f0) block by shuffles and then all hold the integrals.
+constexpr int SCHWARZ_WARPS = 4;
 template <int LA, int LB>
-__global__ void k_schwarz(const int* __restrict__ ids, int n, PairRec* __restrict__ pairs,
-                          const PrimPair* __restrict__ prim_full, int spherical) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void __launch_bounds__(32 * SCHWARZ_WARPS) k_schwarz(const int* __restrict__ ids, int n,
+                                                                PairRec* __restrict__ pairs,
+                                                                const PrimPair* __restrict__ prim_full, int spherical) {
+  using Q = Quartet<LA, LB, LA, LB>;
+  const int t = blockIdx.x * SCHWARZ_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (t >= n) return;
   const int p = ids[t];
   const PairRec pr = pairs[p];
   const double R[3] = {pr.Rx, pr.Ry, pr.Rz};
   constexpr int NA = ncart(LA), NB = ncart(LB);
-  double I[NA][NB][NA * NB];
-  quartet_integrals<LA, LB, LA, LB, double>(prim_full + pr.full_off, pr.n_full, prim_full + pr.full_off,
-                                            pr.n_full, R, R, I);
+  double es[Q::NE][Q::NF], I[NA][NB][NA * NB];
+  const long long npq = (long long)pr.n_full * pr.n_full;
+  const int p0 = (int)(npq * lane / 32), np = (int)(npq * (lane + 1) / 32) - p0;
+  accumulate_esfs<LA, LB, LA, LB, double>(prim_full + pr.full_off, pr.n_full, prim_full + pr.full_off, pr.n_full, p0,
+                                          np, es);
+#pragma unroll
+  for (int e = 0; e < Q::NE; ++e)
+#pragma unroll
+    for (int f = 0; f < Q::NF; ++f)
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) es[e][f] += __shfl_xor_sync(0xffffffffu, es[e][f], o);
+  hrr_quartet<LA, LB, LA, LB, double>(es, R, R, I);
   double m = 0.0;
   const bool sa = spherical && LA >= 2, sb = spherical && LB >= 2;
   const int MA = sa ? 2 * LA + 1 : NA, MB = sb ? 2 * LB + 1 : NB;
@@ -157,7 +172,7 @@ __global__ void k_schwarz(const int* __restrict__ ids, int n, PairRec* __restric
       }
       m = fmax(m, fabs(s));
     }
-  pairs[p].imax = sqrt(m);
+  if (lane == 0) pairs[p].imax = sqrt(m);
 }
 
 // ---------------------------------------------------------------------------
@@ -648,121 +663,144 @@ __device__ __forceinline__ void rys_eval_n(double x, double* u, double* w) {
   for (int i = 0; i < N; ++i) { u[i] = uu[i]; w[i] = ww[i]; }
 }
 
-// One thread per shell pair record (pairs of one molecule only); the Cartesian
-// blocks go into the molecule's n_cart x n_cart slices of S, T, V.
-__global__ void k_one_electron(long long n_pairs, const PairRec* __restrict__ pairs, const MolInfo* __restrict__ mols,
-                               const double* __restrict__ xyz, const double* __restrict__ Z,
-                               const int* __restrict__ shell_atom, const int* __restrict__ shell_l,
-                               const int* __restrict__ shell_nprim, const int* __restrict__ shell_poff,
-                               const int* __restrict__ shell_cart, const double* __restrict__ exps,
-                               const double* __restrict__ coefs, double* __restrict__ S,
-                               double* __restrict__ T, double* __restrict__ V) {
-  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (t >= n_pairs) return;
-  const PairRec pr = pairs[t];
-  const MolInfo mi = mols[pr.mol];
-  const int sa = pr.sh_hi, sb = pr.sh_lo;
-  const int n_cart = mi.n_cart;
-  S += mi.cmat;
-  T += mi.cmat;
-  V += mi.cmat;
-  const int la = shell_l[sa], lb = shell_l[sb];
-  const int na = ncart(la), nb = ncart(lb);
-  const double* A = xyz + 3 * shell_atom[sa];
-  const double* B = xyz + 3 * shell_atom[sb];
-  const double AB[3] = {A[0] - B[0], A[1] - B[1], A[2] - B[2]};
-  const double r2 = AB[0] * AB[0] + AB[1] * AB[1] + AB[2] * AB[2];
-  double s_c[100], t_c[100], v_c[100];     // na x nb, l <= 3
-  for (int i = 0; i < na * nb; ++i) { s_c[i] = 0.0; t_c[i] = 0.0; v_c[i] = 0.0; }
-  constexpr int LD = 6;                    // 1D table edge (l <= 3: i <= 4, j <= 5)
-  const int nroot = (la + lb) / 2 + 1;
-  for (int ia = 0; ia < shell_nprim[sa]; ++ia)
-    for (int ib = 0; ib < shell_nprim[sb]; ++ib) {
-      const double a = exps[shell_poff[sa] + ia], ca = coefs[shell_poff[sa] + ia];
-      const double b = exps[shell_poff[sb] + ib], cb = coefs[shell_poff[sb] + ib];
-      const double z = a + b, oo2z = 0.5 / z;
-      const double Kab = exp(-a * b * r2 / z) * ca * cb;
-      double P[3], PA[3], PB[3];
-      for (int k = 0; k < 3; ++k) { P[k] = (a * A[k] + b * B[k]) / z; PA[k] = P[k] - A[k]; PB[k] = P[k] - B[k]; }
-      double s1[3][LD][LD];
+// S, T and V of the shell pairs ids[0, n) of one class (LA LB), pairs of every molecule of
+// the context; the Cartesian blocks go into the molecule's n_cart x n_cart slices.  One warp
+// per pair: lanes over the pair's primitive pairs for S and T, over (primitive pair,
+// atom) for V, each with its own na x nb sums in registers, added up by shuffles at the end.
+// (One thread a pair, with run-time angular momenta and its tables in local memory, left
+// a 64-primitive pair of a 27-atom cluster as a serial chain of 1,728 Rys evaluations:
+// (H2O)9 cc-pVDZ 4.97 ms, where the whole call, copies back included, now takes 0.46.)  Primitive pairs as k_pair_prep left them: cc = c_a c_b / zeta
+// times the Gaussian product's factor.
+constexpr int ONE_EL_WARPS = 4;
+template <int N>
+struct OneElRoots : std::conditional_t<N == 1, RysSmem<1>, RysPoly<N>> {};
+
+template <int LA, int LB>
+__global__ void __launch_bounds__(32 * ONE_EL_WARPS) k_one_electron(
+    const int* __restrict__ ids, int n, const PairRec* __restrict__ pairs, const MolInfo* __restrict__ mols,
+    const PrimPair* __restrict__ prim_full, const double* __restrict__ xyz, const double* __restrict__ Z,
+    const int* __restrict__ shell_nprim, const int* __restrict__ shell_poff, const double* __restrict__ exps,
+    double* __restrict__ S, double* __restrict__ T, double* __restrict__ V) {
+  constexpr int NA = ncart(LA), NB = ncart(LB), L = LA + LB, NR = L / 2 + 1;
+  using RT = OneElRoots<NR>;
+  extern __shared__ __align__(16) double one_el_tab[];
+  RT::load(one_el_tab);
+  __syncthreads();
+  const int lane = threadIdx.x & 31;
+  for (int t = blockIdx.x * ONE_EL_WARPS + (threadIdx.x >> 5); t < n; t += gridDim.x * ONE_EL_WARPS) {
+    const PairRec pr = pairs[ids[t]];
+    const MolInfo mi = mols[pr.mol];
+    const PrimPair* pp = prim_full + pr.full_off;
+    const double AB[3] = {pr.Rx, pr.Ry, pr.Rz};
+    const int nl = shell_nprim[pr.sh_lo];
+    double s_c[NA][NB], t_c[NA][NB], v_c[NA][NB];
+#pragma unroll
+    for (int i = 0; i < NA; ++i)
+#pragma unroll
+      for (int j = 0; j < NB; ++j) s_c[i][j] = t_c[i][j] = v_c[i][j] = 0.0;
+    for (int p = lane; p < pr.n_full; p += 32) {
+      const PrimPair q = pp[p];
+      const double b = exps[shell_poff[pr.sh_lo] + p % nl], oo2z = q.half_zinv;
+      const double PA[3] = {q.PAx, q.PAy, q.PAz};
+      double s1[3][LA + 1][LB + 3];
+#pragma unroll
       for (int d = 0; d < 3; ++d) {
-        s1[d][0][0] = 1.0;
-        for (int i = 0; i <= la + 1; ++i)
-          for (int j = 0; j <= lb + 2; ++j) {
-            if (i == 0 && j == 0) continue;
+        const double pa = PA[d], pb = PA[d] + AB[d];
+#pragma unroll
+        for (int i = 0; i <= LA; ++i)
+#pragma unroll
+          for (int j = 0; j <= LB + 2; ++j) {
+            if (i == 0 && j == 0) { s1[d][0][0] = 1.0; continue; }
             double v;
             if (i > 0) {
-              v = PA[d] * s1[d][i - 1][j];
+              v = pa * s1[d][i - 1][j];
               if (i > 1) v += (i - 1) * oo2z * s1[d][i - 2][j];
               if (j > 0) v += j * oo2z * s1[d][i - 1][j - 1];
             } else {
-              v = PB[d] * s1[d][0][j - 1];
+              v = pb * s1[d][0][j - 1];
               if (j > 1) v += (j - 1) * oo2z * s1[d][0][j - 2];
             }
             s1[d][i][j] = v;
           }
       }
-      const double pre = Kab * pow(M_PI / z, 1.5);
-      for (int i = 0; i < na; ++i) {
-        const int g = ncart_upto(la - 1) + i;
-        const int ix = c_comp[0][g], iy = c_comp[1][g], iz = c_comp[2][g];
-        for (int j = 0; j < nb; ++j) {
-          const int h = ncart_upto(lb - 1) + j;
-          const int jx = c_comp[0][h], jy = c_comp[1][h], jz = c_comp[2][h];
+      const double pre = q.cc * M_PI * sqrt(2.0 * M_PI * oo2z);
+      auto kin = [&](int d, int i1, int j1) {
+        double v = -2.0 * b * b * s1[d][i1][j1 + 2] + b * (2 * j1 + 1) * s1[d][i1][j1];
+        if (j1 >= 2) v += -0.5 * j1 * (j1 - 1) * s1[d][i1][j1 - 2];
+        return v;
+      };
+      static_for<NA>([&](auto ii) {
+        static_for<NB>([&](auto jj) {
+          constexpr int i = decltype(ii)::value, j = decltype(jj)::value;
+          constexpr int ix = cx(LA, i), iy = cy(LA, i), iz = cz(LA, i), jx = cx(LB, j), jy = cy(LB, j), jz = cz(LB, j);
           const double Sx = s1[0][ix][jx], Sy = s1[1][iy][jy], Sz = s1[2][iz][jz];
-          auto kin = [&](int d, int i1, int j1) {
-            double v = -2.0 * b * b * s1[d][i1][j1 + 2] + b * (2 * j1 + 1) * s1[d][i1][j1];
-            if (j1 >= 2) v += -0.5 * j1 * (j1 - 1) * s1[d][i1][j1 - 2];
-            return v;
-          };
-          s_c[i * nb + j] += pre * Sx * Sy * Sz;
-          t_c[i * nb + j] += pre * (kin(0, ix, jx) * Sy * Sz + Sx * kin(1, iy, jy) * Sz + Sx * Sy * kin(2, iz, jz));
+          s_c[i][j] += pre * Sx * Sy * Sz;
+          t_c[i][j] += pre * (kin(0, ix, jx) * Sy * Sz + Sx * kin(1, iy, jy) * Sz + Sx * Sy * kin(2, iz, jz));
+        });
+      });
+    }
+    const int n_work = pr.n_full * mi.n_atom;
+    for (int q0 = lane; q0 < n_work; q0 += 32) {
+      const int p = q0 / mi.n_atom, at = mi.atom0 + q0 - p * mi.n_atom;
+      const PrimPair q = pp[p];
+      const double PC[3] = {q.Px - xyz[3 * at], q.Py - xyz[3 * at + 1], q.Pz - xyz[3 * at + 2]};
+      const double PA[3] = {q.PAx, q.PAy, q.PAz};
+      const double x = q.zeta * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
+      double u[NR], w[NR];
+      RT::eval(one_el_tab, x, u, w);
+      const double pv = -Z[at] * (2.0 * M_PI) * q.cc;
+#pragma unroll
+      for (int r = 0; r < NR; ++r) {
+        double tab[3][LA + 1][LB + 1];
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          const double c0 = PA[d] - u[r] * PC[d], bb = (1.0 - u[r]) * q.half_zinv;
+          double h[L + 1][LB + 1];
+          h[0][0] = d == 2 ? pv * w[r] : 1.0;
+          if (L >= 1) h[1][0] = c0 * h[0][0];
+#pragma unroll
+          for (int e = 1; e < L; ++e) h[e + 1][0] = c0 * h[e][0] + e * bb * h[e - 1][0];
+#pragma unroll
+          for (int j = 1; j <= LB; ++j)
+#pragma unroll
+            for (int e = 0; e <= L - j; ++e) h[e][j] = h[e + 1][j - 1] + AB[d] * h[e][j - 1];
+#pragma unroll
+          for (int i = 0; i <= LA; ++i)
+#pragma unroll
+            for (int j = 0; j <= LB; ++j) tab[d][i][j] = h[i][j];
         }
-      }
-      for (int at = mi.atom0; at < mi.atom0 + mi.n_atom; ++at) {
-        const double* C = xyz + 3 * at;
-        const double PC[3] = {P[0] - C[0], P[1] - C[1], P[2] - C[2]};
-        const double x = z * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
-        double u[4], w[4];
-        if (nroot == 1) rys_eval_n<1>(x, u, w);
-        else if (nroot == 2) rys_eval_n<2>(x, u, w);
-        else if (nroot == 3) rys_eval_n<3>(x, u, w);
-        else rys_eval_n<4>(x, u, w);
-        const double pv = -Z[at] * 2.0 * M_PI / z * Kab;
-        for (int r = 0; r < nroot; ++r) {
-          double tab[3][4][4];
-          for (int d = 0; d < 3; ++d) {
-            const double c0 = PA[d] - u[r] * PC[d], bb = (1.0 - u[r]) * oo2z;
-            double g[7], h[7][4];
-            g[0] = 1.0;
-            const int L = la + lb;
-            if (L >= 1) g[1] = c0;
-            for (int e = 1; e < L; ++e) g[e + 1] = c0 * g[e] + e * bb * g[e - 1];
-            for (int e = 0; e <= L; ++e) h[e][0] = g[e];
-            for (int j = 1; j <= lb; ++j)
-              for (int e = 0; e <= L - j; ++e) h[e][j] = h[e + 1][j - 1] + AB[d] * h[e][j - 1];
-            for (int i = 0; i <= la; ++i)
-              for (int j = 0; j <= lb; ++j) tab[d][i][j] = h[i][j];
-          }
-          const double wv = pv * w[r];
-          for (int i = 0; i < na; ++i) {
-            const int g2 = ncart_upto(la - 1) + i;
-            for (int j = 0; j < nb; ++j) {
-              const int h2 = ncart_upto(lb - 1) + j;
-              v_c[i * nb + j] += wv * tab[0][c_comp[0][g2]][c_comp[0][h2]] * tab[1][c_comp[1][g2]][c_comp[1][h2]] * tab[2][c_comp[2][g2]][c_comp[2][h2]];
-            }
-          }
-        }
+        static_for<NA>([&](auto ii) {
+          static_for<NB>([&](auto jj) {
+            constexpr int i = decltype(ii)::value, j = decltype(jj)::value;
+            v_c[i][j] += tab[0][cx(LA, i)][cx(LB, j)] * tab[1][cy(LA, i)][cy(LB, j)] * tab[2][cz(LA, i)][cz(LB, j)];
+          });
+        });
       }
     }
-  const int oa = shell_cart[sa], ob = shell_cart[sb];
-  for (int i = 0; i < na; ++i)
-    for (int j = 0; j < nb; ++j) {
-      const size_t p = (size_t)(oa + i) * n_cart + ob + j, q = (size_t)(ob + j) * n_cart + oa + i;
-      S[p] = S[q] = s_c[i * nb + j];
-      T[p] = T[q] = t_c[i * nb + j];
-      V[p] = V[q] = v_c[i * nb + j];
-    }
+    double* const Sm = S + mi.cmat;
+    double* const Tm = T + mi.cmat;
+    double* const Vm = V + mi.cmat;
+    static_for<NA>([&](auto ii) {
+      static_for<NB>([&](auto jj) {
+        constexpr int i = decltype(ii)::value, j = decltype(jj)::value;
+        double s = s_c[i][j], k = t_c[i][j], v = v_c[i][j];
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+          s += __shfl_xor_sync(0xffffffffu, s, o);
+          k += __shfl_xor_sync(0xffffffffu, k, o);
+          v += __shfl_xor_sync(0xffffffffu, v, o);
+        }
+        // (a shell with itself: the lower triangle writes both positions)
+        if (lane == (i * NB + j) % 32 && (LA != LB || j <= i || pr.sh_hi != pr.sh_lo)) {
+          const size_t x = (size_t)(pr.cart_hi + i) * mi.n_cart + pr.cart_lo + j;
+          const size_t y = (size_t)(pr.cart_lo + j) * mi.n_cart + pr.cart_hi + i;
+          Sm[x] = Sm[y] = s;
+          Tm[x] = Tm[y] = k;
+          Vm[x] = Vm[y] = v;
+        }
+      });
+    });
+  }
 }
 
 // Cartesian symmetric matrices -> Tonto basis (column-major), no folding, for
@@ -1067,6 +1105,7 @@ struct tf_ctx {
   std::vector<int> pair_cls;
   std::vector<int> cls_n, cls_off;                       // [mol * NPAIRCLS + class]
   tf::ClassLists lists;                                  // host copy of the sorted class lists
+  std::vector<int> cls_start;                            // first entry of each pair class in d_schwarz_ids
   std::vector<double> shard_cost;                        // estimated FLOPs of every shard (tf_set_shard)
   std::vector<tf::CPUnit> units;
   std::vector<int> unit_group, group_task0;
@@ -1084,7 +1123,7 @@ struct tf_ctx {
   // device
   tf::DBuf<tf::MolInfo> d_mols;
   tf::DBuf<long long> d_cmat_off, d_bmat_off, d_pmax_off;
-  tf::DBuf<double> d_xyz, d_exps, d_coefs, d_P, d_Pc, d_Jc, d_Kc, d_J, d_K, d_H, d_pmax, d_sorted_imax, d_sorted_bmax;
+  tf::DBuf<double> d_xyz, d_exps, d_coefs, d_P, d_Pc, d_Jc, d_Kc, d_J, d_K, d_H, d_pmax, d_sorted_imax, d_sorted_bmax, d_Z;
   tf::DBuf<double> d_PcB, d_JcB, d_KcB, d_Pb, d_Jb, d_Kb;  // unrestricted builds (allocated on first use)
   tf::DBuf<double> d_wscratch;                             // f shells: per-warp scratch of their Schwarz bounds
   tf::DBuf<int> d_csorted, d_cxstart, d_cn;                // collapsed (family) class lists
@@ -1156,6 +1195,53 @@ static void drop_graph(tf_ctx* c) {
 
 static int set_device(tf_ctx* c) {
   TF_CUDA(cudaSetDevice(c->device));
+  return TF_OK;
+}
+
+// The branch streams and events of graph builds, up to n branches (the context stream
+// is the first).
+static int ensure_branches(tf_ctx* c, int n) {
+  while ((int)c->side.size() < n - 1) {
+    cudaStream_t x;
+    TF_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
+    c->side.push_back(x);
+  }
+  while (c->join_ev.size() < c->side.size()) {
+    cudaEvent_t e;
+    TF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    c->join_ev.push_back(e);
+  }
+  if (!c->fork_ev) TF_CUDA(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
+  if (!c->list_fork_ev) TF_CUDA(cudaEventCreateWithFlags(&c->list_fork_ev, cudaEventDisableTiming));
+  if (!c->list_join_ev) TF_CUDA(cudaEventCreateWithFlags(&c->list_join_ev, cudaEventDisableTiming));
+  return TF_OK;
+}
+
+// Branches of a build whose schedule no autotuner has chosen.  A class pair's launch ends
+// in a tail of its longest quartets that leaves most SMs idle, and in a small build the
+// tails are nearly all of it, so the launches overlap.  Measured (graph builds, 1, 2, 4, 6
+// and 8 branches): (H2O)7 cc-pVDZ 6.09, 3.55, 2.41, 2.00 and 2.91 ms; (H2O)2 STO-3G from
+// host arrays 0.42, 0.27, 0.23, 0.18 and 0.17 ms; (H2O)12 cc-pVDZ, deterministic, 10.5, 7.4,
+// 6.1, 6.2 and 6.3 ms; (H2O)32 cc-pVDZ 81.4, 76.8, 76.9, 76.2 and 76.4 ms.
+constexpr int DEFAULT_BRANCHES = 6;
+
+// Branches of the current schedule, and the start and end of a set of class launches on
+// them: the branches wait for the context stream's earlier work, and the context stream
+// then waits for the branches.
+static int sched_branches(const tf_ctx* c) { return std::max(1, std::min(c->sched_streams, 1 + (int)c->side.size())); }
+
+static int fork_branches(tf_ctx* c, int ns) {
+  if (ns <= 1) return TF_OK;
+  TF_CUDA(cudaEventRecord(c->fork_ev, c->stream));
+  for (int i = 0; i + 1 < ns; ++i) TF_CUDA(cudaStreamWaitEvent(c->side[i], c->fork_ev, 0));
+  return TF_OK;
+}
+
+static int join_branches(tf_ctx* c, int ns) {
+  for (int i = 0; i + 1 < ns; ++i) {
+    TF_CUDA(cudaEventRecord(c->join_ev[i], c->side[i]));
+    TF_CUDA(cudaStreamWaitEvent(c->stream, c->join_ev[i], 0));
+  }
   return TF_OK;
 }
 
@@ -1665,7 +1751,8 @@ static int setup_pairs(tf_ctx* c) {
   std::vector<std::vector<int>> by_cls(NPAIRCLS);
   for (long long p = 0; p < c->n_pairs; ++p) by_cls[c->pair_cls[p]].push_back((int)p);
   std::vector<int> ids;
-  std::vector<int> cls_start(NPAIRCLS + 1, 0);
+  std::vector<int>& cls_start = c->cls_start;
+  cls_start.assign(NPAIRCLS + 1, 0);
   for (int k = 0; k < NPAIRCLS; ++k) {
     cls_start[k] = (int)ids.size();
     ids.insert(ids.end(), by_cls[k].begin(), by_cls[k].end());
@@ -1674,13 +1761,18 @@ static int setup_pairs(tf_ctx* c) {
   TF_CUDA(c->d_schwarz_ids.reserve(std::max<size_t>(ids.size(), 1)));
   TF_CUDA(cudaMemcpyAsync(c->d_schwarz_ids.p, ids.data(), ids.size() * sizeof(int), cudaMemcpyHostToDevice,
                           c->stream));
-#define TF_SCHWARZ(LH, LL)                                                                                 \
-  {                                                                                                        \
-    const int k = pair_class(LH, LL);                                                                      \
-    const int nk = cls_start[k + 1] - cls_start[k];                                                        \
-    if (nk > 0)                                                                                            \
-      k_schwarz<LH, LL><<<(nk + 63) / 64, 64, 0, c->stream>>>(c->d_schwarz_ids.p + cls_start[k], nk,       \
-                                                              c->d_pairs.p, c->d_prim_full.p, c->spherical); \
+  // the classes' launches overlap on the build's branch streams (each ends in a tail of its
+  // longest contractions); the f classes share one scratch area and stay on the context's
+  TF_TRY_RC(ensure_branches(c, DEFAULT_BRANCHES));
+  TF_TRY_RC(fork_branches(c, DEFAULT_BRANCHES));
+  auto branch = [&](int k) { return k == 0 ? c->stream : c->side[(k - 1) % (DEFAULT_BRANCHES - 1)]; };
+#define TF_SCHWARZ(LH, LL)                                                                                  \
+  {                                                                                                         \
+    const int k = pair_class(LH, LL);                                                                       \
+    const int nk = cls_start[k + 1] - cls_start[k];                                                         \
+    if (nk > 0)                                                                                             \
+      k_schwarz<LH, LL><<<(nk + SCHWARZ_WARPS - 1) / SCHWARZ_WARPS, 32 * SCHWARZ_WARPS, 0, branch(k)>>>(    \
+          c->d_schwarz_ids.p + cls_start[k], nk, c->d_pairs.p, c->d_prim_full.p, c->spherical);             \
   }
   TF_SCHWARZ(0, 0) TF_SCHWARZ(1, 0) TF_SCHWARZ(1, 1) TF_SCHWARZ(2, 0)
 #undef TF_SCHWARZ
@@ -1690,7 +1782,7 @@ static int setup_pairs(tf_ctx* c) {
       const int nk = cls_start[k + 1] - cls_start[k];
       if (nk > 0)
         k_schwarz_warp<<<std::min(4096, (nk + WARPS_PER_BLOCK - 1) / WARPS_PER_BLOCK), 32 * WARPS_PER_BLOCK,
-                         WARPS_PER_BLOCK * W_SMEM * sizeof(double), c->stream>>>(
+                         WARPS_PER_BLOCK * W_SMEM * sizeof(double), branch(k)>>>(
             c->d_schwarz_ids.p + cls_start[k], nk, c->d_pairs.p, c->d_prim_full.p, c->spherical, lh, ll, nullptr);
     }
   // pair classes with an f shell: the warp path in global scratch (two blocks of
@@ -1710,6 +1802,7 @@ static int setup_pairs(tf_ctx* c) {
                                                               c->d_prim_full.p, c->spherical, 3, ll, c->d_wscratch.p);
     }
   }
+  TF_TRY_RC(join_branches(c, DEFAULT_BRANCHES));
   TF_CUDA(cudaGetLastError());
   TF_CUDA(cudaMemcpyAsync(c->pairs_h.data(), c->d_pairs.p, c->n_pairs * sizeof(PairRec), cudaMemcpyDeviceToHost,
                           c->stream));
@@ -1793,6 +1886,21 @@ static int setup_pairs(tf_ctx* c) {
   if (rc) return rc;
   c->geometry_ready = true;
   return TF_OK;
+}
+
+// S, T and V of the context's pairs of class k = (LA LB) into out[0..2] on stream s.
+template <int LA, int LB>
+static void launch_one_electron(tf_ctx* c, int k, double* const* out, cudaStream_t s) {
+  constexpr size_t smem = OneElRoots<(LA + LB) / 2 + 1>::SIZE * sizeof(double);
+  const int i0 = c->cls_start[k], n = c->cls_start[k + 1] - i0;
+  if (n <= 0) return;
+  cudaFuncSetAttribute(k_one_electron<LA, LB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  int nsm = 148;
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, c->device);
+  const int blocks = std::min((n + ONE_EL_WARPS - 1) / ONE_EL_WARPS, 4 * nsm);   // each loads the root table once
+  k_one_electron<LA, LB><<<blocks, 32 * ONE_EL_WARPS, smem, s>>>(
+      c->d_schwarz_ids.p + i0, n, c->d_pairs.p, c->d_mols.p, c->d_prim_full.p, c->d_xyz.p, c->d_Z.p,
+      c->d_shell_nprim.p, c->d_shell_poff.p, c->d_exps.p, out[0], out[1], out[2]);
 }
 
 // pair class id -> (lh, ll)
@@ -1967,33 +2075,6 @@ static int enqueue_finalize(tf_ctx* c, double* dJ, double* dK, double* dJb, doub
   return TF_OK;
 }
 
-// The branch streams and events of graph builds, up to n branches (the context stream
-// is the first).
-static int ensure_branches(tf_ctx* c, int n) {
-  while ((int)c->side.size() < n - 1) {
-    cudaStream_t x;
-    TF_CUDA(cudaStreamCreateWithFlags(&x, cudaStreamNonBlocking));
-    c->side.push_back(x);
-  }
-  while (c->join_ev.size() < c->side.size()) {
-    cudaEvent_t e;
-    TF_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-    c->join_ev.push_back(e);
-  }
-  if (!c->fork_ev) TF_CUDA(cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming));
-  if (!c->list_fork_ev) TF_CUDA(cudaEventCreateWithFlags(&c->list_fork_ev, cudaEventDisableTiming));
-  if (!c->list_join_ev) TF_CUDA(cudaEventCreateWithFlags(&c->list_join_ev, cudaEventDisableTiming));
-  return TF_OK;
-}
-
-// Branches of a build whose schedule no autotuner has chosen.  A class pair's launch ends
-// in a tail of its longest quartets that leaves most SMs idle, and in a small build the
-// tails are nearly all of it, so the launches overlap.  Measured (graph builds, 1, 2, 4, 6
-// and 8 branches): (H2O)7 cc-pVDZ 6.09, 3.55, 2.41, 2.00 and 2.91 ms; (H2O)2 STO-3G from
-// host arrays 0.42, 0.27, 0.23, 0.18 and 0.17 ms; (H2O)12 cc-pVDZ, deterministic, 10.5, 7.4,
-// 6.1, 6.2 and 6.3 ms; (H2O)32 cc-pVDZ 81.4, 76.8, 76.9, 76.2 and 76.4 ms.
-constexpr int DEFAULT_BRANCHES = 6;
-
 // Class schedule of a build that no autotuner has chosen one for: the class pairs over
 // DEFAULT_BRANCHES branches, longest first, each to the least-loaded branch, by the FLOP
 // model at the given list lengths (goff: start, FP32 start and end per group) with eight
@@ -2023,26 +2104,6 @@ static int default_schedule(tf_ctx* c, const long long* goff) {
     const int k = (int)(std::min_element(load.begin(), load.end()) - load.begin());
     c->sched_stream_of[g] = k;
     load[k] += cost[g];
-  }
-  return TF_OK;
-}
-
-// Branches of the current schedule, and the start and end of a set of class launches on
-// them: the branches wait for the context stream's earlier work, and the context stream
-// then waits for the branches.
-static int sched_branches(const tf_ctx* c) { return std::max(1, std::min(c->sched_streams, 1 + (int)c->side.size())); }
-
-static int fork_branches(tf_ctx* c, int ns) {
-  if (ns <= 1) return TF_OK;
-  TF_CUDA(cudaEventRecord(c->fork_ev, c->stream));
-  for (int i = 0; i + 1 < ns; ++i) TF_CUDA(cudaStreamWaitEvent(c->side[i], c->fork_ev, 0));
-  return TF_OK;
-}
-
-static int join_branches(tf_ctx* c, int ns) {
-  for (int i = 0; i + 1 < ns; ++i) {
-    TF_CUDA(cudaEventRecord(c->join_ev[i], c->side[i]));
-    TF_CUDA(cudaStreamWaitEvent(c->stream, c->join_ev[i], 0));
   }
   return TF_OK;
 }
@@ -2967,27 +3028,30 @@ int tf_one_electron(tf_ctx* c, const double* Z, double* S, double* T, double* V)
   int rc = set_device(c);
   if (rc) return rc;
   cudaStream_t s = c->stream;
-  DBuf<double> dZ;
-  TF_CUDA(dZ.reserve(c->n_atom));
-  TF_CUDA(cudaMemcpyAsync(dZ.p, Z, c->n_atom * sizeof(double), cudaMemcpyHostToDevice, s));
+  TF_CUDA(c->d_Z.reserve(c->n_atom));
+  TF_CUDA(cudaMemcpyAsync(c->d_Z.p, Z, c->n_atom * sizeof(double), cudaMemcpyHostToDevice, s));
   // Cartesian blocks into the (reused) Cartesian accumulators, then to the basis
-  double* Sc = c->d_Jc.p;
-  double* Tc = c->d_Kc.p;
-  double* Vc = c->d_Pc.p;
-  k_one_electron<<<(unsigned)((c->n_pairs + 127) / 128), 128, 0, s>>>(
-      c->n_pairs, c->d_pairs.p, c->d_mols.p, c->d_xyz.p, dZ.p, c->d_shell_atom.p, c->d_shell_l.p,
-      c->d_shell_nprim.p, c->d_shell_poff.p, c->d_shell_cart.p, c->d_exps.p, c->d_coefs.p, Sc, Tc, Vc);
+  double* const in[3] = {c->d_Jc.p, c->d_Kc.p, c->d_Pc.p};
+  TF_TRY_RC(ensure_branches(c, DEFAULT_BRANCHES));
+  TF_TRY_RC(fork_branches(c, DEFAULT_BRANCHES));
+#define TF_ONE_EL(LH, LL)                                                                                  \
+  launch_one_electron<LH, LL>(c, pair_class(LH, LL), in,                                                   \
+                              pair_class(LH, LL) == 0 ? s : c->side[(pair_class(LH, LL) - 1) % (DEFAULT_BRANCHES - 1)])
+  TF_ONE_EL(0, 0); TF_ONE_EL(1, 0); TF_ONE_EL(1, 1); TF_ONE_EL(2, 0); TF_ONE_EL(2, 1);
+  TF_ONE_EL(2, 2); TF_ONE_EL(3, 0); TF_ONE_EL(3, 1); TF_ONE_EL(3, 2); TF_ONE_EL(3, 3);
+#undef TF_ONE_EL
   TF_CUDA(cudaGetLastError());
+  TF_TRY_RC(join_branches(c, DEFAULT_BRANCHES));
   const long long n2 = c->bmat_off[c->n_mol];
   const BatchArgs bt = batch_args(c);
-  double* outs[3] = {S, T, V};
-  double* ins[3] = {Sc, Tc, Vc};
+  double* const outs[3] = {S, T, V};
+  double* const basis[3] = {c->d_J.p, c->d_K.p, c->d_P.p};
   for (int k = 0; k < 3; ++k) {
-    k_cart_to_basis<<<(unsigned)((n2 + 255) / 256), 256, 0, s>>>(bt, ins[k], c->d_J.p);
-    TF_CUDA(cudaMemcpyAsync(outs[k], c->d_J.p, n2 * sizeof(double), cudaMemcpyDeviceToHost, s));
-    TF_CUDA(cudaStreamSynchronize(s));
+    k_cart_to_basis<<<(unsigned)((n2 + 255) / 256), 256, 0, s>>>(bt, in[k], basis[k]);
+    TF_CUDA(cudaMemcpyAsync(outs[k], basis[k], n2 * sizeof(double), cudaMemcpyDeviceToHost, s));
   }
   TF_CUDA(cudaGetLastError());
+  TF_CUDA(cudaStreamSynchronize(s));
   return TF_OK;
 }
 
