@@ -176,11 +176,21 @@ __host__ __device__ constexpr int gidx(int x, int y, int z) { return CT.first[x 
 // 2 pi^(5/2) cc_ab zeta^(-3/2) cc_cd eta^(-3/2) sqrt(rho), rho = zeta eta / (zeta + eta),
 // becomes 2 pi^(5/2) cc_ab cc_cd / sqrt(zeta + eta): one reciprocal square root of
 // zeta + eta gives both it and 1/(zeta + eta) (its square).
-struct __align__(16) PrimPair {
+// P - A (A: the centre of the higher-l shell) is f (A - B), f = -b / zeta: one factor per
+// primitive pair, the difference of centres once per shell pair.  Two 32-byte words, each
+// one load instruction (ldg256).
+struct __align__(64) PrimPair {
   double Px, Py, Pz, zeta;
-  double cc, half_zinv;              // prefactor, 1/(2 zeta)
-  double PAx, PAy, PAz, pad;         // P - (centre of the higher-l shell)
+  double cc, half_zinv, f, pad;      // prefactor, 1/(2 zeta), see above
 };
+static_assert(sizeof(PrimPair) == 64, "primitive-pair record layout");
+
+// One 32-byte read-only load (p 32-byte aligned).
+__device__ __forceinline__ double4 ldg256(const void* p) {
+  double4 v;
+  asm("ld.global.nc.v4.f64 {%0, %1, %2, %3}, [%4];" : "=d"(v.x), "=d"(v.y), "=d"(v.z), "=d"(v.w) : "l"(p));
+  return v;
+}
 
 // One shell pair, oriented so that shell "hi" has the higher l (ties: the
 // shell with the larger index, as Tonto's pair (a >= b) orientation).
@@ -460,6 +470,49 @@ struct RysSmem<2> {
 };
 #endif
 
+// Boys functions F_0 .. F_M, M <= 3, of the classes evaluated by the vertical recurrence
+// (prim_quartet_vrr): the 8-term Taylor step of the grids above about the nearest point
+// k/8, one independent chain per order; beyond the grid (42, or 50 for M >= 2)
+// F_0 = sqrt(pi/x)/2 and F_{m+1} = (2m+1)/(2x) F_m, where exp(-x)/(2x) is below rounding.
+template <int M>
+struct BoysSmem {
+  static constexpr bool WIDE = M >= 2;
+  static constexpr int NM = WIDE ? TF_BOYS2_NM : TF_BOYS_NM, NPTS = WIDE ? TF_BOYS2_NPTS : TF_BOYS_NPTS;
+  static constexpr int XMAX = WIDE ? TF_BOYS2_XMAX : TF_BOYS_XMAX;
+  static constexpr int SIZE = NPTS * NM;
+  static __device__ __forceinline__ void load(double* t) {
+    const double* g = WIDE ? tf_boys2_grid : tf_boys_grid;
+    for (int q = threadIdx.x; q < SIZE; q += blockDim.x) t[q] = g[q];
+  }
+  static __device__ __forceinline__ void eval(const double* __restrict__ t, double x, double (&F)[M + 1]) {
+    static_assert(M <= 3 && TF_BOYS_NTERM == 8, "grids of F_0 .. F_8 and F_0 .. F_10");
+    if (x < (double)XMAX) {
+      const int k = (int)(x * (double)TF_BOYS_H_INV + 0.5);
+      const double d = (double)k * (1.0 / TF_BOYS_H_INV) - x;
+      const double2* g = reinterpret_cast<const double2*>(t + k * NM);
+      double f[2 * ((M + 9) / 2)];
+#pragma unroll
+      for (int q = 0; q < (M + 9) / 2; ++q) {
+        const double2 v = g[q];
+        f[2 * q] = v.x;
+        f[2 * q + 1] = v.y;
+      }
+      const double dj[8] = {0.0, d, d * 0.5, d * (1.0 / 3.0), d * 0.25, d * 0.2, d * (1.0 / 6.0), d * (1.0 / 7.0)};
+#pragma unroll
+      for (int m = 0; m <= M; ++m) F[m] = f[m + 7];
+#pragma unroll
+      for (int j = 7; j >= 1; --j)
+#pragma unroll
+        for (int m = 0; m <= M; ++m) F[m] = fma(dj[j], F[m], f[m + j - 1]);
+    } else {
+      const double r = rsqrt_nr(x), ix = r * r;
+      F[0] = tf_rys_hweight[rys_hoffset(1)] * r;
+#pragma unroll
+      for (int m = 0; m < M; ++m) F[m + 1] = (m + 0.5) * ix * F[m];
+    }
+  }
+};
+
 // ---------------------------------------------------------------------------
 // One contracted shell quartet (LA LB | LC LD), LA >= LB, LC >= LD, in
 // arithmetic type T for the 2D recurrences and (e0|f0) sums (double, or float
@@ -475,43 +528,33 @@ struct Quartet {
   static constexpr int NINT = NA * NB * NC * ND;
 };
 
-// read-only loads of a primitive-pair record: half 0 = (Px, Py, Pz, zeta),
-// half 1 = (PAx, PAy, PAz, 1/(2 zeta))
-__device__ __forceinline__ double4 ld4(const PrimPair* p, int half) {
-  const double2* q = reinterpret_cast<const double2*>(p);
-  if (half == 0) {
-    const double2 a = __ldg(q), b = __ldg(q + 1);
-    return make_double4(a.x, a.y, b.x, b.y);
-  }
-  const double2 c = __ldg(q + 2), d = __ldg(q + 3), e = __ldg(q + 4);
-  return make_double4(d.x, d.y, e.x, c.y);
-}
-
 // (e0|f0) accumulation over all primitive quartets of a contracted quartet.
 #ifndef TF_PRIM_UNROLL
 #define TF_PRIM_UNROLL 1
 #endif
 
 constexpr int kPrimUnroll = TF_PRIM_UNROLL;
-constexpr int PPS = sizeof(PrimPair) / sizeof(double2);         // 5 16-byte loads per record
 
-// The loaded part of a primitive-pair record: (Px, Py), (Pz, zeta), (cc, 1/(2 zeta)),
-// and (PAx, PAy), (PAz, -) only where the recurrences need P - A.
+// The loaded part of a primitive-pair record: P and zeta, then the prefactor and, where the
+// class's recurrences use them, 1/(2 zeta) and f of P - A.
 struct PrimRegs {
-  double2 P, Z, C, A0, A1;
+  double4 P;
+  double cc, half_zinv, f;
 };
 
-template <bool NEED_PA>
-__device__ __forceinline__ PrimRegs load_prim(const double2* __restrict__ q, int i) {
+// FULL: the whole second word (pairs with a p or higher shell), else the prefactor alone.
+template <bool FULL>
+__device__ __forceinline__ PrimRegs load_prim(const PrimPair* __restrict__ q, int i) {
   PrimRegs r;
-  r.P = __ldg(q + i * PPS);
-  r.Z = __ldg(q + i * PPS + 1);
-  r.C = __ldg(q + i * PPS + 2);
-  if constexpr (NEED_PA) {
-    r.A0 = __ldg(q + i * PPS + 3);
-    r.A1 = __ldg(q + i * PPS + 4);
+  r.P = ldg256(q + i);
+  if constexpr (FULL) {
+    const double4 c = ldg256(&q[i].cc);
+    r.cc = c.x;
+    r.half_zinv = c.y;
+    r.f = c.z;
   } else {
-    r.A0 = r.A1 = make_double2(0.0, 0.0);
+    r.cc = __ldg(&q[i].cc);
+    r.half_zinv = r.f = 0.0;
   }
   return r;
 }
@@ -529,32 +572,172 @@ __device__ __forceinline__ float rsqrt_f32(float x) {
   return y;
 }
 
+// Classes evaluated by the vertical recurrence over Boys functions (Obara and Saika, J. Chem.
+// Phys. 84, 3963 (1986)) instead of Rys quadrature: up to three quanta in all and an ss or ps
+// ket.  There the recurrence takes a third to a half of the quadrature's FP64 operations
+// ((ps|ps) 33 against about 120 after the Boys functions: no root finding, no sum over
+// roots) with as few live values; from four quanta on, its tables no longer fit the
+// registers beside the (e0|f0) block.  T = float (mixed precision) keeps the quadrature: an
+// incremental build is nearly all FP32 quartets, and its rounding is part of its result.
+// Measured: (H2O)32 cc-pVDZ (ps|ps) 10.17 -> 9.31 ms, (pp|ss) 5.28 -> 4.73, (ds|ss) 4.27 ->
+// 3.86, (ps|ss) 12.63 -> 12.45, the build 73.2 -> 71.0; 24 clusters batched 191 -> 184 ms.
+template <int LA, int LB, int LC, int LD, typename T>
+__host__ __device__ constexpr bool use_vrr() {
+  return std::is_same<T, double>::value && LC + LD <= 1 && LA + LB + LC + LD <= 3;
+}
+
+// The table a thread kernel's primitive loop reads in shared memory.
+template <int LA, int LB, int LC, int LD, typename T>
+using RootTable = std::conditional_t<use_vrr<LA, LB, LC, LD, T>(),
+                                     BoysSmem<(use_vrr<LA, LB, LC, LD, T>() ? LA + LB + LC + LD : 0)>,
+                                     RysSmem<(LA + LB + LC + LD) / 2 + 1>>;
+
+// Direction along which Cartesian component g is raised from a lower one: the smallest
+// non-zero power, so that most components need no third term.
+__host__ __device__ constexpr int vrr_dir(int g) {
+  const int v[3] = {gx(g), gy(g), gz(g)};
+  int d = -1;
+  for (int i = 0; i < 3; ++i)
+    if (v[i] > 0 && (d < 0 || v[i] < v[d])) d = i;
+  return d;
+}
+__host__ __device__ constexpr int comp_power(int g, int i) { return i == 0 ? gx(g) : (i == 1 ? gy(g) : gz(g)); }
+__host__ __device__ constexpr int comp_lower(int g, int i) {
+  return gidx(gx(g) - (i == 0), gy(g) - (i == 1), gz(g) - (i == 2));
+}
+
+// [e0|f0] of one primitive quartet, added to esfs, from S[m] = [00|00]^(m):
+//   [e+1_i, 0]^m = PA_i [e]^m + WP_i [e]^(m+1) + e_i/(2 zeta) ([e-1_i]^m - r_z [e-1_i]^(m+1)),
+//   [e, 1_j] = QC_j [e]^0 + WQ_j [e]^1 + e_j/(2(zeta+eta)) [e-1_j]^1,
+// WP = r_z QP, WQ = -r_e QP, r_z = rho/zeta, r_e = rho/eta.
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void vrr_add(const double (&S)[LA + LB + LC + LD + 1], const double (&PA)[3], const double (&WP)[3],
+                                        const double (&QC)[3], const double (&WQ)[3], double half_zinv, double r_z, double half_inv,
+                                        double (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF]) {
+  using Q = Quartet<LA, LB, LC, LD>;
+  constexpr int L = Q::LAB + Q::LCD, LAB = Q::LAB, LCD = Q::LCD, NG = ncart_upto(LAB);
+  double v[NG][L + 1], dz[NG][L + 1];             // [e]^m, and 1/(2 zeta) ([e]^m - r_z [e]^(m+1))
+#pragma unroll
+  for (int m = 0; m <= L; ++m) v[0][m] = S[m];
+  static_for<NG>([&](auto gg) {
+    constexpr int g = decltype(gg)::value, l = gx(g) + gy(g) + gz(g);
+    if constexpr (l > 0) {
+      constexpr int i = vrr_dir(g), p = comp_lower(g, i), e = comp_power(p, i);
+      // the highest level without a ket step is only added up
+      constexpr int MM = (LAB - l) + LCD;
+      constexpr bool sum_only = MM == 0;
+      static_for<MM + 1>([&](auto mm) {
+        constexpr int m = decltype(mm)::value;
+        double t = sum_only ? esfs[g - Q::FE >= 0 ? g - Q::FE : 0][0] : 0.0;
+        t = sum_only ? fma(PA[i], v[p][m], t) : PA[i] * v[p][m];
+        t = fma(WP[i], v[p][m + 1], t);
+        if constexpr (e > 0) {
+          constexpr int pp = comp_lower(p, i);
+          t = fma(double(e), dz[pp][m], t);
+        }
+        if constexpr (sum_only) esfs[g - Q::FE][0] = t;
+        else v[g][m] = t;
+      });
+    }
+    if constexpr (l + 2 <= LAB) {            // raised twice along one direction later
+      static_for<LAB - l - 2 + LCD + 1>([&](auto mm) {
+        constexpr int m = decltype(mm)::value;
+        dz[g][m] = half_zinv * fma(-r_z, v[g][m + 1], v[g][m]);
+      });
+    }
+  });
+  static_for<Q::NE>([&](auto ee) {
+    constexpr int e = decltype(ee)::value, g = Q::FE + e, l = gx(g) + gy(g) + gz(g);
+    if constexpr (LCD == 0) {
+      if constexpr (l < LAB || LAB == 0) esfs[e][0] += v[g][0];
+    } else {
+      static_for<3>([&](auto jj) {
+        constexpr int j = decltype(jj)::value, ej = comp_power(g, j);
+        double t = fma(QC[j], v[g][0], esfs[e][j]);
+        t = fma(WQ[j], v[g][1], t);
+        if constexpr (ej > 0) t = fma(double(ej) * half_inv, v[comp_lower(g, j)][1], t);
+        esfs[e][j] = t;
+      });
+    }
+  });
+}
+
+// F_0 .. F_M at x from the table in shared memory, or (null) from the Rys rule, which is
+// exact for them.
+template <int M>
+__device__ __forceinline__ void boys_eval(const double* __restrict__ tab, double x, double (&F)[M + 1]) {
+  if (tab) {
+    BoysSmem<M>::eval(tab, x, F);
+  } else {
+    constexpr int N = M / 2 + 1;
+    double u[N], w[N];
+    rys_eval<N>(x, u, w);
+#pragma unroll
+    for (int m = 0; m <= M; ++m) F[m] = 0.0;
+#pragma unroll
+    for (int r = 0; r < N; ++r) {
+      double p = w[r];
+#pragma unroll
+      for (int m = 0; m <= M; ++m) { F[m] += p; p *= u[r]; }
+    }
+  }
+}
+
+// One primitive quartet by the vertical recurrence.
+template <int LA, int LB, int LC, int LD>
+__device__ __forceinline__ void prim_quartet_vrr(const PrimRegs& B, const PrimRegs& K, const double* Rab,
+                                                 const double* Rcd,
+                                                 double (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
+                                                 const double* __restrict__ tab) {
+  constexpr int L = LA + LB + LC + LD;
+  const double zeta = B.P.w, eta = K.P.w;
+  const double sq = rsqrt_nr(zeta + eta);      // 1/sqrt(zeta + eta)
+  const double inv = sq * sq, r_z = eta * inv, r_e = zeta * inv;
+  const double QP[3] = {K.P.x - B.P.x, K.P.y - B.P.y, K.P.z - B.P.z};
+  const double xx = zeta * r_z * (QP[0] * QP[0] + QP[1] * QP[1] + QP[2] * QP[2]);
+  double F[L + 1];
+  boys_eval<L>(tab, xx, F);
+  const double scale = B.cc * K.cc * TWOPI5ON2 * sq;
+  double S[L + 1], PA[3], WP[3], QC[3], WQ[3];
+#pragma unroll
+  for (int m = 0; m <= L; ++m) S[m] = F[m] * scale;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    PA[i] = B.f * Rab[i];
+    WP[i] = r_z * QP[i];
+    QC[i] = K.f * Rcd[i];
+    WQ[i] = -r_e * QP[i];
+  }
+  vrr_add<LA, LB, LC, LD>(S, PA, WP, QC, WQ, B.half_zinv, r_z, 0.5 * inv, esfs);
+}
+
 // One primitive quartet in the mixed-precision path: the Boys-function argument
 // and everything after the Rys nodes and weights in FP32 (exponent sums, rho, the
 // prefactor, the recurrence coefficients, the 2D recurrences and the (e0|f0)
 // products); P - Q in FP64 (a difference of positions), then the nodes and weights
 // themselves in FP64 from the FP64 tables, as for the FP64 path.
 template <int LA, int LB, int LC, int LD>
-__device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRegs& K, double wmask,
+__device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRegs& K, const double* Rab,
+                                                 const double* Rcd,
                                                  float (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                  const double* __restrict__ rys_smem) {
   using Q = Quartet<LA, LB, LC, LD>;
   constexpr int D1 = Q::LAB + 1, D2 = Q::LCD + 1, NR = Q::NROOT;
-  const float zeta = (float)B.Z.y, eta = (float)K.Z.y;
-  const float half_zinv = (float)B.C.y, half_einv = (float)K.C.y;
+  const float zeta = (float)B.P.w, eta = (float)K.P.w;
+  const float half_zinv = (float)B.half_zinv, half_einv = (float)K.half_zinv;
   const float sq = rsqrt_f32(zeta + eta);
   const float inv = sq * sq;
   const float rho = zeta * eta * inv;
-  const float QP[3] = {(float)(K.P.x - B.P.x), (float)(K.P.y - B.P.y), (float)(K.Z.x - B.Z.x)};
+  const float QP[3] = {(float)(K.P.x - B.P.x), (float)(K.P.y - B.P.y), (float)(K.P.z - B.P.z)};
   const float xx = rho * (QP[0] * QP[0] + QP[1] * QP[1] + QP[2] * QP[2]);
   double u[NR], w[NR];
   if (rys_smem) RysSmem<NR>::eval(rys_smem, (double)xx, u, w);
   else rys_eval<NR>((double)xx, u, w);
-  const float scale = (float)(B.C.x * K.C.x * (TWOPI5ON2 * wmask)) * sq;
+  const float scale = (float)(B.cc * K.cc * TWOPI5ON2) * sq;
   const float r_z = eta * inv;     // rho / zeta
   const float r_e = zeta * inv;    // rho / eta
-  const float PA[3] = {(float)B.A0.x, (float)B.A0.y, (float)B.A1.x};
-  const float QC[3] = {(float)K.A0.x, (float)K.A0.y, (float)K.A1.x};
+  const float PA[3] = {(float)(B.f * Rab[0]), (float)(B.f * Rab[1]), (float)(B.f * Rab[2])};
+  const float QC[3] = {(float)(K.f * Rcd[0]), (float)(K.f * Rcd[1]), (float)(K.f * Rcd[2])};
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
     const float t2 = (float)u[r];
@@ -595,29 +778,32 @@ __device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRe
 }
 
 // One primitive quartet: Rys nodes and weights, the 2D recurrences and the
-// (e0|f0) products, added to esfs with weight `wmask`.
+// (e0|f0) products, added to esfs.  Rab, Rcd: A - B and C - D of the two pairs.
 template <int LA, int LB, int LC, int LD, typename T>
-__device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& K, double wmask,
-                                             T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
+__device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& K, const double* Rab,
+                                             const double* Rcd, T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                              const double* __restrict__ rys_smem) {
-  if constexpr (std::is_same<T, float>::value) {
-    prim_quartet_f32<LA, LB, LC, LD>(B, K, wmask, esfs, rys_smem);
+  if constexpr (use_vrr<LA, LB, LC, LD, T>()) {
+    prim_quartet_vrr<LA, LB, LC, LD>(B, K, Rab, Rcd, esfs, rys_smem);
     return;
-  }
+  } else if constexpr (std::is_same<T, float>::value) {
+    prim_quartet_f32<LA, LB, LC, LD>(B, K, Rab, Rcd, esfs, rys_smem);
+    return;
+  } else {
   using Q = Quartet<LA, LB, LC, LD>;
   constexpr int D1 = Q::LAB + 1, D2 = Q::LCD + 1, NR = Q::NROOT;
-  const double bcc = B.C.x * TWOPI5ON2, kcc = K.C.x;
-  const double zeta = B.Z.y, half_zinv = B.C.y;
-  const double eta = K.Z.y, half_einv = K.C.y;
+  const double bcc = B.cc * TWOPI5ON2, kcc = K.cc;
+  const double zeta = B.P.w, half_zinv = B.half_zinv;
+  const double eta = K.P.w, half_einv = K.half_zinv;
   const double sq = rsqrt_nr(zeta + eta);     // 1/sqrt(zeta + eta)
   const double inv = sq * sq;
   const double rho = zeta * eta * inv;
-  const double QPx = K.P.x - B.P.x, QPy = K.P.y - B.P.y, QPz = K.Z.x - B.Z.x;
+  const double QPx = K.P.x - B.P.x, QPy = K.P.y - B.P.y, QPz = K.P.z - B.P.z;
   const double xx = rho * (QPx * QPx + QPy * QPy + QPz * QPz);
   double u[NR], w[NR];
   if (rys_smem) RysSmem<NR>::eval(rys_smem, xx, u, w);
   else rys_eval<NR>(xx, u, w);
-  const double scale = bcc * kcc * sq * wmask;
+  const double scale = bcc * kcc * sq;
   const double r_z = eta * inv;     // rho / zeta
   const double r_e = zeta * inv;    // rho / eta
 #pragma unroll
@@ -629,8 +815,8 @@ __device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& 
     const T B00 = T(0.5 * t2 * inv);
     const T wt = T(w[r] * scale);
     T I[3][D1][D2];
-    const double PA[3] = {B.A0.x, B.A0.y, B.A1.x};
-    const double QC[3] = {K.A0.x, K.A0.y, K.A1.x};
+    const double PA[3] = {B.f * Rab[0], B.f * Rab[1], B.f * Rab[2]};
+    const double QC[3] = {K.f * Rcd[0], K.f * Rcd[1], K.f * Rcd[2]};
     const double QP[3] = {QPx, QPy, QPz};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
@@ -661,6 +847,7 @@ __device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& 
     });
   }
 }
+}
 
 // One flat loop over the nbp x nkp primitive quartets: lanes with the same count but
 // different (nbp, nkp) splits stay converged.  Kets are the outer index and bras the
@@ -674,6 +861,7 @@ __device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& 
 template <int LA, int LB, int LC, int LD, typename T>
 __device__ __forceinline__ void accumulate_esfs(const PrimPair* __restrict__ bp, int nbp,
                                                 const PrimPair* __restrict__ kp, int nkp, int p0, int npq,
+                                                const double* Rab, const double* Rcd,
                                                 T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                 const double* __restrict__ rys_smem = nullptr) {
   using Q = Quartet<LA, LB, LC, LD>;
@@ -683,20 +871,18 @@ __device__ __forceinline__ void accumulate_esfs(const PrimPair* __restrict__ bp,
 #pragma unroll
     for (int f = 0; f < Q::NF; ++f) esfs[e][f] = T(0);
   if (npq <= 0) return;
-  const double2* bq = reinterpret_cast<const double2*>(bp);
-  const double2* kq = reinterpret_cast<const double2*>(kp);
   int ik = p0 ? p0 / nbp : 0, ib = p0 - ik * nbp;
-  PrimRegs kc = load_prim<KPA>(kq, ik);
+  PrimRegs kc = load_prim<KPA>(kp, ik);
 #pragma unroll(kPrimUnroll)
   for (int p = 0; p < npq; ++p) {
-    const PrimRegs b = load_prim<BPA>(bq, ib);
+    const PrimRegs b = load_prim<BPA>(bp, ib);
     const PrimRegs k = kc;
     if (++ib == nbp) {
       ib = 0;
       ++ik;
-      if (ik < nkp) kc = load_prim<KPA>(kq, ik);
+      if (ik < nkp) kc = load_prim<KPA>(kp, ik);
     }
-    prim_quartet<LA, LB, LC, LD, T>(b, k, 1.0, esfs, rys_smem);
+    prim_quartet<LA, LB, LC, LD, T>(b, k, Rab, Rcd, esfs, rys_smem);
   }
 }
 
@@ -809,6 +995,7 @@ __device__ __forceinline__ void hrr_bra(const T (&G)[CT.first[LA + LB + 1] - CT.
 template <int LA, int LB, int LC, int LD, typename T, int MB>
 __device__ __forceinline__ void accumulate_esfs_fam(const PrimPair* __restrict__ bp, int nbp,
                                                     const PrimPair* __restrict__ kp, int nkp, int p0, int npq,
+                                                    const double* Rab, const double* Rcd,
                                                     const PrimPair* const (&bm)[MB],
                                                     T (&esfs)[MB][Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                     const double* __restrict__ rys_smem) {
@@ -821,28 +1008,26 @@ __device__ __forceinline__ void accumulate_esfs_fam(const PrimPair* __restrict__
 #pragma unroll
       for (int f = 0; f < Q::NF; ++f) esfs[m][e][f] = T(0);
   if (npq <= 0) return;
-  const double2* bq = reinterpret_cast<const double2*>(bp);
-  const double2* kq = reinterpret_cast<const double2*>(kp);
   int ik = p0 ? p0 / nbp : 0, ib = p0 - ik * nbp;
-  PrimRegs kc = load_prim<KPA>(kq, ik);
+  PrimRegs kc = load_prim<KPA>(kp, ik);
   for (int p = 0; p < npq; ++p) {
-    PrimRegs b = load_prim<BPA>(bq, ib);
+    PrimRegs b = load_prim<BPA>(bp, ib);
     double cb[MB];
 #pragma unroll
     for (int m = 0; m < MB; ++m) cb[m] = bm[m] ? __ldg(&bm[m][ib].cc) : 0.0;
-    b.C.x = 1.0;
+    b.cc = 1.0;
     const PrimRegs k = kc;
     if (++ib == nbp) {
       ib = 0;
       ++ik;
-      if (ik < nkp) kc = load_prim<KPA>(kq, ik);
+      if (ik < nkp) kc = load_prim<KPA>(kp, ik);
     }
     T one[Q::NE][Q::NF];
 #pragma unroll
     for (int e = 0; e < Q::NE; ++e)
 #pragma unroll
       for (int f = 0; f < Q::NF; ++f) one[e][f] = T(0);
-    prim_quartet<LA, LB, LC, LD, T>(b, k, 1.0, one, rys_smem);
+    prim_quartet<LA, LB, LC, LD, T>(b, k, Rab, Rcd, one, rys_smem);
 #pragma unroll
     for (int m = 0; m < MB; ++m) {
       const T w = T(cb[m]);

@@ -253,9 +253,9 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
               k1 = make_double4(0, 0, 0, 0);
       double inv = 0.0, r_z = 0.0, r_e = 0.0, scale = 0.0, xx = 0.0;
       if (v) {
-        b0 = ld4(bp + ib, 0); b1 = ld4(bp + ib, 1);
-        k0 = ld4(kp + ik, 0); k1 = ld4(kp + ik, 1);
-        const double bcc = __ldg(&bp[ib].cc) * TWOPI5ON2, kcc = __ldg(&kp[ik].cc);
+        b0 = ldg256(bp + ib); b1 = ldg256(&bp[ib].cc);
+        k0 = ldg256(kp + ik); k1 = ldg256(&kp[ik].cc);
+        const double bcc = b1.x * TWOPI5ON2, kcc = k1.x;
         const double sq = rsqrt_nr(b0.w + k0.w);
         inv = sq * sq;
         const double rho = b0.w * k0.w * inv;
@@ -276,10 +276,10 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
           for (int i = 0; i < NR; ++i)
             if (i == r) { t2 = u[i]; wr = w[i]; }
           const double QPd = d == 0 ? k0.x - b0.x : (d == 1 ? k0.y - b0.y : k0.z - b0.z);
-          const double PA = d == 0 ? b1.x : (d == 1 ? b1.y : b1.z);
-          const double QC = d == 0 ? k1.x : (d == 1 ? k1.y : k1.z);
+          const double PA = b1.z * (d == 0 ? b.Rx : (d == 1 ? b.Ry : b.Rz));
+          const double QC = k1.z * (d == 0 ? k.Rx : (d == 1 ? k.Ry : k.Rz));
           const double t2_rz = t2 * r_z, t2_re = t2 * r_e;
-          const double B10 = (1.0 - t2_rz) * b1.w, B01 = (1.0 - t2_re) * k1.w, B00 = 0.5 * t2 * inv;
+          const double B10 = (1.0 - t2_rz) * b1.y, B01 = (1.0 - t2_re) * k1.y, B00 = 0.5 * t2 * inv;
           const double c00 = PA + t2_rz * QPd, d00 = QC - t2_re * QPd;
           double* out = T2 + task * (D2 * D1P);
           // one ket column at a time: I[e][f + 1] from columns f and f - 1

@@ -307,7 +307,7 @@ __device__ __forceinline__ void count_quartets(const JKArgs& a, int cls, unsigne
 template <int LA, int LB, int LC, int LD, typename T, int V, int MB>
 __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArgs a) {
   using Q = Quartet<LA, LB, LC, LD>;
-  using RS = RysSmem<Q::NROOT>;
+  using RS = RootTable<LA, LB, LC, LD, T>;
   extern __shared__ double rys_tab[];
   __shared__ LaunchPlan plan;
   const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
@@ -357,7 +357,7 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
       if (qd.x == qd.y) f *= 0.5;
       double I[Q::NA][Q::NB][Q::NC * Q::ND];
       T esfs[Q::NE][Q::NF];
-      accumulate_esfs<LA, LB, LC, LD, T>(bp, nbp, kp, nkp, p0, np, esfs, rys_tab);
+      accumulate_esfs<LA, LB, LC, LD, T>(bp, nbp, kp, nkp, p0, np, Rab, Rcd, esfs, rys_tab);
       for (int o = 1; o < 1 << lg; o <<= 1)
 #pragma unroll
         for (int e = 0; e < Q::NE; ++e)
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
         bmp[m] = mid[m] < 0 ? nullptr : (any_same ? a.prim_full + bm[m].full_off : a.prim_skip + bm[m].skip_off);
       }
       T esfs[MB][Q::NE][Q::NF];
-      accumulate_esfs_fam<LA, LB, LC, LD, T, MB>(bp, nbp, kp, nkp, p0, np, bmp, esfs, rys_tab);
+      accumulate_esfs_fam<LA, LB, LC, LD, T, MB>(bp, nbp, kp, nkp, p0, np, Rab, Rcd, bmp, esfs, rys_tab);
       for (int o = 1; o < 1 << lg; o <<= 1)
 #pragma unroll
         for (int m = 0; m < MB; ++m)
@@ -408,7 +408,7 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
 template <int LA, int LB, int LC, int LD, typename T, int V, int MB>
 static void launch_jk_t(const JKArgs& a, cudaStream_t s) {
   constexpr int thr = jk_threads<LA, LB, LC, LD, V>();
-  constexpr size_t smem = RysSmem<Quartet<LA, LB, LC, LD>::NROOT>::SIZE * sizeof(double);
+  constexpr size_t smem = RootTable<LA, LB, LC, LD, T>::SIZE * sizeof(double);
   static int blocks_per_sm = -1;
   if (blocks_per_sm < 0) {
     cudaFuncSetAttribute(k_jk<LA, LB, LC, LD, T, V, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);

@@ -85,13 +85,13 @@ __device__ int warp_quartet(const WarpQuartet& q, const PrimPair* __restrict__ b
   for (int k = lane; k < nef; k += 32) es[k] = 0.0;
   const int tsz = q.d1 * q.d2;
   for (int ib = 0; ib < nbp; ++ib) {
-    const double4 b0 = ld4(bp + ib, 0);
-    const double4 b1 = ld4(bp + ib, 1);
-    const double bcc = __ldg(&bp[ib].cc) * TWOPI5ON2;
+    const double4 b0 = ldg256(bp + ib);
+    const double4 b1 = ldg256(&bp[ib].cc);
+    const double bcc = b1.x * TWOPI5ON2;
     for (int ik = 0; ik < nkp; ++ik) {
-      const double4 k0 = ld4(kp + ik, 0);
-      const double4 k1 = ld4(kp + ik, 1);
-      const double kcc = __ldg(&kp[ik].cc);
+      const double4 k0 = ldg256(kp + ik);
+      const double4 k1 = ldg256(&kp[ik].cc);
+      const double kcc = k1.x;
       const double zeta = b0.w, eta = k0.w;
       const double sq = rsqrt_nr(zeta + eta);
       const double inv = sq * sq;
@@ -119,9 +119,8 @@ __device__ int warp_quartet(const WarpQuartet& q, const PrimPair* __restrict__ b
         for (int i = 0; i < WNR_MAX; ++i)
           if (i == r) { t2 = u[i]; wr = w[i]; }
         const double t2_rz = t2 * r_z, t2_re = t2 * r_e;
-        const double B10 = (1.0 - t2_rz) * b1.w, B01 = (1.0 - t2_re) * k1.w, B00 = 0.5 * t2 * inv;
-        const double PA = d == 0 ? b1.x : (d == 1 ? b1.y : b1.z);
-        const double QC = d == 0 ? k1.x : (d == 1 ? k1.y : k1.z);
+        const double B10 = (1.0 - t2_rz) * b1.y, B01 = (1.0 - t2_re) * k1.y, B00 = 0.5 * t2 * inv;
+        const double PA = b1.z * Rab[d], QC = k1.z * Rcd[d];
         const double c00 = PA + t2_rz * QP[d], d00 = QC - t2_re * QP[d];
         double* I = I2 + (d * q.nr + r) * tsz;
         I[0] = (d == 2) ? wr * scale : 1.0;

@@ -104,11 +104,10 @@ __global__ void k_pair_prep(int n_pairs, PairRec* __restrict__ pairs, const doub
       q.Py = (eh * A[1] + el * B[1]) * inv;
       q.Pz = (eh * A[2] + el * B[2]) * inv;
       q.zeta = zeta;
-      q.PAx = q.Px - A[0]; q.PAy = q.Py - A[1]; q.PAz = q.Pz - A[2];
+      q.f = -el * inv;
       q.half_zinv = 0.5 * inv;
       q.cc = ch * cl * inv * prefac;      // c_a c_b / zeta x prefactor: see PrimPair
       q.pad = 0.0;
-      static_assert(sizeof(PrimPair) == 80, "primitive-pair record layout");
       prim_full[pr.full_off + i] = q;
       if (!same && !(prefac < pair_cutoff)) prim_skip[pr.skip_off + k++] = q;
     }
@@ -136,7 +135,7 @@ __global__ void __launch_bounds__(32 * SCHWARZ_WARPS) k_schwarz(const int* __res
   const long long npq = (long long)pr.n_full * pr.n_full;
   const int p0 = (int)(npq * lane / 32), np = (int)(npq * (lane + 1) / 32) - p0;
   accumulate_esfs<LA, LB, LA, LB, double>(prim_full + pr.full_off, pr.n_full, prim_full + pr.full_off, pr.n_full, p0,
-                                          np, es);
+                                          np, R, R, es);
 #pragma unroll
   for (int e = 0; e < Q::NE; ++e)
 #pragma unroll
@@ -701,7 +700,7 @@ __global__ void __launch_bounds__(32 * ONE_EL_WARPS) k_one_electron(
     for (int p = lane; p < pr.n_full; p += 32) {
       const PrimPair q = pp[p];
       const double b = exps[shell_poff[pr.sh_lo] + p % nl], oo2z = q.half_zinv;
-      const double PA[3] = {q.PAx, q.PAy, q.PAz};
+      const double PA[3] = {q.f * AB[0], q.f * AB[1], q.f * AB[2]};
       double s1[3][LA + 1][LB + 3];
 #pragma unroll
       for (int d = 0; d < 3; ++d) {
@@ -744,7 +743,7 @@ __global__ void __launch_bounds__(32 * ONE_EL_WARPS) k_one_electron(
       const int p = q0 / mi.n_atom, at = mi.atom0 + q0 - p * mi.n_atom;
       const PrimPair q = pp[p];
       const double PC[3] = {q.Px - xyz[3 * at], q.Py - xyz[3 * at + 1], q.Pz - xyz[3 * at + 2]};
-      const double PA[3] = {q.PAx, q.PAy, q.PAz};
+      const double PA[3] = {q.f * AB[0], q.f * AB[1], q.f * AB[2]};
       const double x = q.zeta * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
       double u[NR], w[NR];
       RT::eval(one_el_tab, x, u, w);
@@ -1306,7 +1305,10 @@ __global__ void __launch_bounds__(64) k_group_offsets(int n_groups, const int* _
   for (int q = 0; q < 2; ++q) {
     const int j = lane + 32 * q;
     int lg = 0;
-    while (lg < 5 && (double)cost[q] > share * (double)(1 << lg)) ++lg;
+    // (FP32 sums keep their order: in an incremental build, nearly all FP32 quartets, it
+    // shows in the result)
+    if (half == 0)
+      while (lg < 5 && (double)cost[q] > share * (double)(1 << lg)) ++lg;
     const long long warps = (n[q] + (32 >> lg) - 1) / (32 >> lg);
     long long incl = warps;
 #pragma unroll
