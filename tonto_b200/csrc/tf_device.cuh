@@ -176,14 +176,15 @@ __host__ __device__ constexpr int gidx(int x, int y, int z) { return CT.first[x 
 // 2 pi^(5/2) cc_ab zeta^(-3/2) cc_cd eta^(-3/2) sqrt(rho), rho = zeta eta / (zeta + eta),
 // becomes 2 pi^(5/2) cc_ab cc_cd / sqrt(zeta + eta): one reciprocal square root of
 // zeta + eta gives both it and 1/(zeta + eta) (its square).
-// P - A (A: the centre of the higher-l shell) is f (A - B), f = -b / zeta: one factor per
-// primitive pair, the difference of centres once per shell pair.  Two 32-byte words, each
-// one load instruction (ldg256).
-struct __align__(64) PrimPair {
-  double Px, Py, Pz, zeta;
-  double cc, half_zinv, f, pad;      // prefactor, 1/(2 zeta), see above
+// Positions are not stored: P - A (A: the centre of the higher-l shell) is f (A - B),
+// f = -b / zeta, so a record is one 32-byte word, one sector and one load instruction
+// (ldg256).  The thread kernels are bound by the sectors their lanes' loads touch (one L1 data
+// cycle each; every lane has its own ket): with 64-byte records (P and zeta, the rest) a ket
+// primitive cost two, with 80-byte ones read 16 bytes at a time three to five.
+struct __align__(32) PrimPair {
+  double zeta, cc, f, half_zinv;     // cc: prefactor, half_zinv: 1/(2 zeta)
 };
-static_assert(sizeof(PrimPair) == 64, "primitive-pair record layout");
+static_assert(sizeof(PrimPair) == 32, "primitive-pair record layout");
 
 // One 32-byte read-only load (p 32-byte aligned).
 __device__ __forceinline__ double4 ldg256(const void* p) {
@@ -205,27 +206,31 @@ struct __align__(16) PairRec {
   double imax;               // Schwarz bound sqrt(max |(ab|ab)|)
 };
 
-// What the ERI kernels read of a shell pair, packed: rec[2 id] = {cart_hi, cart_lo,
-// full_off, skip_off}, rec[2 id + 1] = {atom_hi, atom_lo, n_full | n_skip << 16,
-// mol | (shell hi == shell lo) << 31} (32 bytes, one sector), and pairR[id] = (A - B, 0)
-// read only by classes whose transfers need it.
+// What the ERI kernels read of a shell pair, packed into one 32-byte word: {cart_hi,
+// cart_lo, full_off, skip_off, atom_hi, atom_lo, n_full | n_skip << 16, mol | (shell hi ==
+// shell lo) << 31}; the centres come from the atom positions (32 bytes an atom), which the
+// neighbouring kets of a warp share.
 struct PairJK {
   int cart_hi, cart_lo, full_off, skip_off;
   int atom_hi, atom_lo, n_full, n_skip, mol;
   bool same;                 // both shells the same (coincidence factor 1/2)
-  double Rx, Ry, Rz;
+  double Ax, Ay, Az;         // hi centre
+  double Rx, Ry, Rz;         // hi centre - lo centre
 };
 
-__device__ __forceinline__ PairJK load_pair_jk(const int4* __restrict__ rec, const double2* __restrict__ pairR,
-                                               int id) {
-  const int4 x = __ldg(rec + 2 * id), y = __ldg(rec + 2 * id + 1);
+__device__ __forceinline__ PairJK load_pair_jk(const int4* __restrict__ rec, const double4* __restrict__ xyz4, int id) {
+  int4 x, y;
+  asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+      : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w), "=r"(y.x), "=r"(y.y), "=r"(y.z), "=r"(y.w)
+      : "l"(rec + 2 * id));
   PairJK p;
   p.cart_hi = x.x; p.cart_lo = x.y; p.full_off = x.z; p.skip_off = x.w;
   p.atom_hi = y.x; p.atom_lo = y.y;
   p.n_full = y.z & 0xffff; p.n_skip = (int)((unsigned)y.z >> 16);
   p.mol = y.w & 0x7fffffff; p.same = y.w < 0;
-  const double2 r0 = __ldg(pairR + 2 * id), r1 = __ldg(pairR + 2 * id + 1);
-  p.Rx = r0.x; p.Ry = r0.y; p.Rz = r1.x;
+  const double4 A = ldg256(xyz4 + p.atom_hi), B = ldg256(xyz4 + p.atom_lo);
+  p.Ax = A.x; p.Ay = A.y; p.Az = A.z;
+  p.Rx = A.x - B.x; p.Ry = A.y - B.y; p.Rz = A.z - B.z;
   return p;
 }
 
@@ -535,26 +540,29 @@ struct Quartet {
 
 constexpr int kPrimUnroll = TF_PRIM_UNROLL;
 
-// The loaded part of a primitive-pair record: P and zeta, then the prefactor and, where the
-// class's recurrences use them, 1/(2 zeta) and f of P - A.
-struct PrimRegs {
-  double4 P;
-  double cc, half_zinv, f;
-};
+// A loaded primitive-pair record: (zeta, cc, f, 1/(2 zeta)).
+typedef double4 PrimRegs;
+__device__ __forceinline__ PrimRegs load_prim(const PrimPair* __restrict__ q, int i) { return ldg256(q + i); }
 
-// FULL: the whole second word (pairs with a p or higher shell), else the prefactor alone.
-template <bool FULL>
-__device__ __forceinline__ PrimRegs load_prim(const PrimPair* __restrict__ q, int i) {
-  PrimRegs r;
-  r.P = ldg256(q + i);
-  if constexpr (FULL) {
-    const double4 c = ldg256(&q[i].cc);
-    r.cc = c.x;
-    r.half_zinv = c.y;
-    r.f = c.z;
-  } else {
-    r.cc = __ldg(&q[i].cc);
-    r.half_zinv = r.f = 0.0;
+// Geometry of a quartet: A - B, C - D, and C - A.
+struct QuartetGeom {
+  double Rab[3], Rcd[3], CA[3];
+};
+__device__ __forceinline__ QuartetGeom quartet_geom(const PairJK& b, const PairJK& k) {
+  return QuartetGeom{{b.Rx, b.Ry, b.Rz}, {k.Rx, k.Ry, k.Rz}, {k.Ax - b.Ax, k.Ay - b.Ay, k.Az - b.Az}};
+}
+
+// P - A, Q - C and Q - P of a primitive quartet.
+struct PrimGeom {
+  double PA[3], QC[3], QP[3];
+};
+__device__ __forceinline__ PrimGeom prim_geom(const PrimRegs& B, const PrimRegs& K, const QuartetGeom& g) {
+  PrimGeom r;
+#pragma unroll
+  for (int i = 0; i < 3; ++i) {
+    r.PA[i] = B.z * g.Rab[i];
+    r.QC[i] = K.z * g.Rcd[i];
+    r.QP[i] = fma(-B.z, g.Rab[i], fma(K.z, g.Rcd[i], g.CA[i]));
   }
   return r;
 }
@@ -685,30 +693,27 @@ __device__ __forceinline__ void boys_eval(const double* __restrict__ tab, double
 
 // One primitive quartet by the vertical recurrence.
 template <int LA, int LB, int LC, int LD>
-__device__ __forceinline__ void prim_quartet_vrr(const PrimRegs& B, const PrimRegs& K, const double* Rab,
-                                                 const double* Rcd,
+__device__ __forceinline__ void prim_quartet_vrr(const PrimRegs& B, const PrimRegs& K, const QuartetGeom& g,
                                                  double (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                  const double* __restrict__ tab) {
   constexpr int L = LA + LB + LC + LD;
-  const double zeta = B.P.w, eta = K.P.w;
+  const PrimGeom p = prim_geom(B, K, g);
+  const double zeta = B.x, eta = K.x;
   const double sq = rsqrt_nr(zeta + eta);      // 1/sqrt(zeta + eta)
   const double inv = sq * sq, r_z = eta * inv, r_e = zeta * inv;
-  const double QP[3] = {K.P.x - B.P.x, K.P.y - B.P.y, K.P.z - B.P.z};
-  const double xx = zeta * r_z * (QP[0] * QP[0] + QP[1] * QP[1] + QP[2] * QP[2]);
+  const double xx = zeta * r_z * (p.QP[0] * p.QP[0] + p.QP[1] * p.QP[1] + p.QP[2] * p.QP[2]);
   double F[L + 1];
   boys_eval<L>(tab, xx, F);
-  const double scale = B.cc * K.cc * TWOPI5ON2 * sq;
-  double S[L + 1], PA[3], WP[3], QC[3], WQ[3];
+  const double scale = B.y * K.y * TWOPI5ON2 * sq;
+  double S[L + 1], WP[3], WQ[3];
 #pragma unroll
   for (int m = 0; m <= L; ++m) S[m] = F[m] * scale;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    PA[i] = B.f * Rab[i];
-    WP[i] = r_z * QP[i];
-    QC[i] = K.f * Rcd[i];
-    WQ[i] = -r_e * QP[i];
+    WP[i] = r_z * p.QP[i];
+    WQ[i] = -r_e * p.QP[i];
   }
-  vrr_add<LA, LB, LC, LD>(S, PA, WP, QC, WQ, B.half_zinv, r_z, 0.5 * inv, esfs);
+  vrr_add<LA, LB, LC, LD>(S, p.PA, WP, p.QC, WQ, B.w, r_z, 0.5 * inv, esfs);
 }
 
 // One primitive quartet in the mixed-precision path: the Boys-function argument
@@ -717,27 +722,27 @@ __device__ __forceinline__ void prim_quartet_vrr(const PrimRegs& B, const PrimRe
 // products); P - Q in FP64 (a difference of positions), then the nodes and weights
 // themselves in FP64 from the FP64 tables, as for the FP64 path.
 template <int LA, int LB, int LC, int LD>
-__device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRegs& K, const double* Rab,
-                                                 const double* Rcd,
+__device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRegs& K, const QuartetGeom& g,
                                                  float (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                  const double* __restrict__ rys_smem) {
   using Q = Quartet<LA, LB, LC, LD>;
   constexpr int D1 = Q::LAB + 1, D2 = Q::LCD + 1, NR = Q::NROOT;
-  const float zeta = (float)B.P.w, eta = (float)K.P.w;
-  const float half_zinv = (float)B.half_zinv, half_einv = (float)K.half_zinv;
+  const PrimGeom p = prim_geom(B, K, g);
+  const float zeta = (float)B.x, eta = (float)K.x;
+  const float half_zinv = (float)B.w, half_einv = (float)K.w;
   const float sq = rsqrt_f32(zeta + eta);
   const float inv = sq * sq;
   const float rho = zeta * eta * inv;
-  const float QP[3] = {(float)(K.P.x - B.P.x), (float)(K.P.y - B.P.y), (float)(K.P.z - B.P.z)};
+  const float QP[3] = {(float)p.QP[0], (float)p.QP[1], (float)p.QP[2]};
   const float xx = rho * (QP[0] * QP[0] + QP[1] * QP[1] + QP[2] * QP[2]);
   double u[NR], w[NR];
   if (rys_smem) RysSmem<NR>::eval(rys_smem, (double)xx, u, w);
   else rys_eval<NR>((double)xx, u, w);
-  const float scale = (float)(B.cc * K.cc * TWOPI5ON2) * sq;
+  const float scale = (float)(B.y * K.y * TWOPI5ON2) * sq;
   const float r_z = eta * inv;     // rho / zeta
   const float r_e = zeta * inv;    // rho / eta
-  const float PA[3] = {(float)(B.f * Rab[0]), (float)(B.f * Rab[1]), (float)(B.f * Rab[2])};
-  const float QC[3] = {(float)(K.f * Rcd[0]), (float)(K.f * Rcd[1]), (float)(K.f * Rcd[2])};
+  const float PA[3] = {(float)p.PA[0], (float)p.PA[1], (float)p.PA[2]};
+  const float QC[3] = {(float)p.QC[0], (float)p.QC[1], (float)p.QC[2]};
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
     const float t2 = (float)u[r];
@@ -778,28 +783,27 @@ __device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRe
 }
 
 // One primitive quartet: Rys nodes and weights, the 2D recurrences and the
-// (e0|f0) products, added to esfs.  Rab, Rcd: A - B and C - D of the two pairs.
+// (e0|f0) products, added to esfs.
 template <int LA, int LB, int LC, int LD, typename T>
-__device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& K, const double* Rab,
-                                             const double* Rcd, T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
+__device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& K, const QuartetGeom& g, T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                              const double* __restrict__ rys_smem) {
   if constexpr (use_vrr<LA, LB, LC, LD, T>()) {
-    prim_quartet_vrr<LA, LB, LC, LD>(B, K, Rab, Rcd, esfs, rys_smem);
+    prim_quartet_vrr<LA, LB, LC, LD>(B, K, g, esfs, rys_smem);
     return;
   } else if constexpr (std::is_same<T, float>::value) {
-    prim_quartet_f32<LA, LB, LC, LD>(B, K, Rab, Rcd, esfs, rys_smem);
+    prim_quartet_f32<LA, LB, LC, LD>(B, K, g, esfs, rys_smem);
     return;
   } else {
   using Q = Quartet<LA, LB, LC, LD>;
   constexpr int D1 = Q::LAB + 1, D2 = Q::LCD + 1, NR = Q::NROOT;
-  const double bcc = B.cc * TWOPI5ON2, kcc = K.cc;
-  const double zeta = B.P.w, half_zinv = B.half_zinv;
-  const double eta = K.P.w, half_einv = K.half_zinv;
+  const PrimGeom p = prim_geom(B, K, g);
+  const double bcc = B.y * TWOPI5ON2, kcc = K.y;
+  const double zeta = B.x, half_zinv = B.w;
+  const double eta = K.x, half_einv = K.w;
   const double sq = rsqrt_nr(zeta + eta);     // 1/sqrt(zeta + eta)
   const double inv = sq * sq;
   const double rho = zeta * eta * inv;
-  const double QPx = K.P.x - B.P.x, QPy = K.P.y - B.P.y, QPz = K.P.z - B.P.z;
-  const double xx = rho * (QPx * QPx + QPy * QPy + QPz * QPz);
+  const double xx = rho * (p.QP[0] * p.QP[0] + p.QP[1] * p.QP[1] + p.QP[2] * p.QP[2]);
   double u[NR], w[NR];
   if (rys_smem) RysSmem<NR>::eval(rys_smem, xx, u, w);
   else rys_eval<NR>(xx, u, w);
@@ -815,13 +819,10 @@ __device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& 
     const T B00 = T(0.5 * t2 * inv);
     const T wt = T(w[r] * scale);
     T I[3][D1][D2];
-    const double PA[3] = {B.f * Rab[0], B.f * Rab[1], B.f * Rab[2]};
-    const double QC[3] = {K.f * Rcd[0], K.f * Rcd[1], K.f * Rcd[2]};
-    const double QP[3] = {QPx, QPy, QPz};
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const T c00 = T(PA[d] + t2_rz * QP[d]);
-      const T d00 = T(QC[d] - t2_re * QP[d]);
+      const T c00 = T(p.PA[d] + t2_rz * p.QP[d]);
+      const T d00 = T(p.QC[d] - t2_re * p.QP[d]);
       I[d][0][0] = (d == 2) ? wt : T(1);
       if (D1 > 1) I[d][1][0] = c00 * I[d][0][0];
 #pragma unroll
@@ -861,28 +862,26 @@ __device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& 
 template <int LA, int LB, int LC, int LD, typename T>
 __device__ __forceinline__ void accumulate_esfs(const PrimPair* __restrict__ bp, int nbp,
                                                 const PrimPair* __restrict__ kp, int nkp, int p0, int npq,
-                                                const double* Rab, const double* Rcd,
-                                                T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
+                                                const QuartetGeom& g, T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                 const double* __restrict__ rys_smem = nullptr) {
   using Q = Quartet<LA, LB, LC, LD>;
-  constexpr bool BPA = Q::LAB > 0, KPA = Q::LCD > 0;
 #pragma unroll
   for (int e = 0; e < Q::NE; ++e)
 #pragma unroll
     for (int f = 0; f < Q::NF; ++f) esfs[e][f] = T(0);
   if (npq <= 0) return;
   int ik = p0 ? p0 / nbp : 0, ib = p0 - ik * nbp;
-  PrimRegs kc = load_prim<KPA>(kp, ik);
+  PrimRegs kc = load_prim(kp, ik);
 #pragma unroll(kPrimUnroll)
   for (int p = 0; p < npq; ++p) {
-    const PrimRegs b = load_prim<BPA>(bp, ib);
+    const PrimRegs b = load_prim(bp, ib);
     const PrimRegs k = kc;
     if (++ib == nbp) {
       ib = 0;
       ++ik;
-      if (ik < nkp) kc = load_prim<KPA>(kp, ik);
+      if (ik < nkp) kc = load_prim(kp, ik);
     }
-    prim_quartet<LA, LB, LC, LD, T>(b, k, Rab, Rcd, esfs, rys_smem);
+    prim_quartet<LA, LB, LC, LD, T>(b, k, g, esfs, rys_smem);
   }
 }
 
@@ -995,12 +994,11 @@ __device__ __forceinline__ void hrr_bra(const T (&G)[CT.first[LA + LB + 1] - CT.
 template <int LA, int LB, int LC, int LD, typename T, int MB>
 __device__ __forceinline__ void accumulate_esfs_fam(const PrimPair* __restrict__ bp, int nbp,
                                                     const PrimPair* __restrict__ kp, int nkp, int p0, int npq,
-                                                    const double* Rab, const double* Rcd,
+                                                    const QuartetGeom& g,
                                                     const PrimPair* const (&bm)[MB],
                                                     T (&esfs)[MB][Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                     const double* __restrict__ rys_smem) {
   using Q = Quartet<LA, LB, LC, LD>;
-  constexpr bool BPA = Q::LAB > 0, KPA = Q::LCD > 0;
 #pragma unroll
   for (int m = 0; m < MB; ++m)
 #pragma unroll
@@ -1009,25 +1007,25 @@ __device__ __forceinline__ void accumulate_esfs_fam(const PrimPair* __restrict__
       for (int f = 0; f < Q::NF; ++f) esfs[m][e][f] = T(0);
   if (npq <= 0) return;
   int ik = p0 ? p0 / nbp : 0, ib = p0 - ik * nbp;
-  PrimRegs kc = load_prim<KPA>(kp, ik);
+  PrimRegs kc = load_prim(kp, ik);
   for (int p = 0; p < npq; ++p) {
-    PrimRegs b = load_prim<BPA>(bp, ib);
+    PrimRegs b = load_prim(bp, ib);
     double cb[MB];
 #pragma unroll
     for (int m = 0; m < MB; ++m) cb[m] = bm[m] ? __ldg(&bm[m][ib].cc) : 0.0;
-    b.cc = 1.0;
+    b.y = 1.0;
     const PrimRegs k = kc;
     if (++ib == nbp) {
       ib = 0;
       ++ik;
-      if (ik < nkp) kc = load_prim<KPA>(kp, ik);
+      if (ik < nkp) kc = load_prim(kp, ik);
     }
     T one[Q::NE][Q::NF];
 #pragma unroll
     for (int e = 0; e < Q::NE; ++e)
 #pragma unroll
       for (int f = 0; f < Q::NF; ++f) one[e][f] = T(0);
-    prim_quartet<LA, LB, LC, LD, T>(b, k, Rab, Rcd, one, rys_smem);
+    prim_quartet<LA, LB, LC, LD, T>(b, k, g, one, rys_smem);
 #pragma unroll
     for (int m = 0; m < MB; ++m) {
       const T w = T(cb[m]);

@@ -42,7 +42,7 @@ struct RowArgs {
   const long long* range;       // graph builds: see resolve_range
   long long base, cap;
   const int4* jkrec;            // packed pair records (load_pair_jk)
-  const double2* pairR;
+  const double4* xyz4;          // atom positions (load_pair_jk)
   const double* P2;             // unrestricted: beta density and its J, K (else null)
   double* J2;
   double* K2;
@@ -213,8 +213,8 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
     const long long t = base + (in_group ? gq : 0);
     const bool act = in_group && t < nq;
     const int2 qd = act ? quartets[t] : make_int2(0, 0);
-    const PairJK b = load_pair_jk(a.jkrec, a.pairR, qd.x);
-    const PairJK k = load_pair_jk(a.jkrec, a.pairR, qd.y);
+    const PairJK b = load_pair_jk(a.jkrec, a.xyz4, qd.x);
+    const PairJK k = load_pair_jk(a.jkrec, a.xyz4, qd.y);
     const bool any_same = b.atom_hi == b.atom_lo || k.atom_hi == k.atom_lo || b.atom_hi == k.atom_hi ||
                           b.atom_hi == k.atom_lo || b.atom_lo == k.atom_hi || b.atom_lo == k.atom_lo;
     const PrimPair* bp = any_same ? a.prim_full + b.full_off : a.prim_skip + b.skip_off;
@@ -242,6 +242,7 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
       }
     }
     const int maxnpq = GW > 1 ? npq : (int)__reduce_max_sync(0xffffffffu, npq);
+    const QuartetGeom geom = quartet_geom(b, k);
     double es[NE];
 #pragma unroll
     for (int e = 0; e < NE; ++e) es[e] = 0.0;
@@ -249,21 +250,20 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
     for (int p = 0; p < maxnpq; ++p) {
       const bool v = p < npq;
       double u[NR], w[NR];
-      double4 b0 = make_double4(0, 0, 0, 1), b1 = make_double4(0, 0, 0, 0), k0 = make_double4(0, 0, 0, 1),
-              k1 = make_double4(0, 0, 0, 0);
+      double4 b0 = make_double4(1, 0, 0, 0), k0 = make_double4(1, 0, 0, 0);
       double inv = 0.0, r_z = 0.0, r_e = 0.0, scale = 0.0, xx = 0.0;
       if (v) {
-        b0 = ldg256(bp + ib); b1 = ldg256(&bp[ib].cc);
-        k0 = ldg256(kp + ik); k1 = ldg256(&kp[ik].cc);
-        const double bcc = b1.x * TWOPI5ON2, kcc = k1.x;
-        const double sq = rsqrt_nr(b0.w + k0.w);
+        b0 = load_prim(bp, ib);
+        k0 = load_prim(kp, ik);
+        const double bcc = b0.y * TWOPI5ON2, kcc = k0.y;
+        const double sq = rsqrt_nr(b0.x + k0.x);
         inv = sq * sq;
-        const double rho = b0.w * k0.w * inv;
-        const double QPx = k0.x - b0.x, QPy = k0.y - b0.y, QPz = k0.z - b0.z;
-        xx = rho * (QPx * QPx + QPy * QPy + QPz * QPz);
+        const double rho = b0.x * k0.x * inv;
+        const PrimGeom pg = prim_geom(b0, k0, geom);
+        xx = rho * (pg.QP[0] * pg.QP[0] + pg.QP[1] * pg.QP[1] + pg.QP[2] * pg.QP[2]);
         scale = bcc * kcc * sq;                  // (cc holds the pair's sqrt(zeta))
-        r_z = k0.w * inv;
-        r_e = b0.w * inv;
+        r_z = k0.x * inv;
+        r_e = b0.x * inv;
       }
       if constexpr (GW > 1) group_rys<NR, 32>(xx, lane, 0, u, w);
       else group_rys<NR, G>(xx, in_group ? gl : G, lane - (in_group ? gl : 0), u, w);
@@ -275,11 +275,12 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
 #pragma unroll
           for (int i = 0; i < NR; ++i)
             if (i == r) { t2 = u[i]; wr = w[i]; }
-          const double QPd = d == 0 ? k0.x - b0.x : (d == 1 ? k0.y - b0.y : k0.z - b0.z);
-          const double PA = b1.z * (d == 0 ? b.Rx : (d == 1 ? b.Ry : b.Rz));
-          const double QC = k1.z * (d == 0 ? k.Rx : (d == 1 ? k.Ry : k.Rz));
+          const double Rb = d == 0 ? geom.Rab[0] : (d == 1 ? geom.Rab[1] : geom.Rab[2]);
+          const double Rk = d == 0 ? geom.Rcd[0] : (d == 1 ? geom.Rcd[1] : geom.Rcd[2]);
+          const double PA = b0.z * Rb, QC = k0.z * Rk;
+          const double QPd = fma(-b0.z, Rb, fma(k0.z, Rk, d == 0 ? geom.CA[0] : (d == 1 ? geom.CA[1] : geom.CA[2])));
           const double t2_rz = t2 * r_z, t2_re = t2 * r_e;
-          const double B10 = (1.0 - t2_rz) * b1.y, B01 = (1.0 - t2_re) * k1.y, B00 = 0.5 * t2 * inv;
+          const double B10 = (1.0 - t2_rz) * b0.w, B01 = (1.0 - t2_re) * k0.w, B00 = 0.5 * t2 * inv;
           const double c00 = PA + t2_rz * QPd, d00 = QC - t2_re * QPd;
           double* out = T2 + task * (D2 * D1P);
           // one ket column at a time: I[e][f + 1] from columns f and f - 1
@@ -334,8 +335,8 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
       if (++ik == nkp) { ik = 0; ++ib; }
     }
     group_sync();                                // the tables have been read, the density blocks written
-    const double Rab[3] = {b.Rx, b.Ry, b.Rz};
-    const double Rcd[3] = {k.Rx, k.Ry, k.Rz};
+    const double (&Rab)[3] = geom.Rab;
+    const double (&Rcd)[3] = geom.Rcd;
     if (act && has_f) {                          // column f: bra transfer, J~(f)
       double jt = 0.0, jt2 = 0.0;
       const double* pab = stage + NX * YS;

@@ -49,7 +49,7 @@ struct JKArgs {
   const long long* range;
   long long base, cap, first;
   const int4* jkrec;            // packed pair records (load_pair_jk)
-  const double2* pairR;
+  const double4* xyz4;          // atom positions (load_pair_jk)
   // unrestricted builds: the beta density and its J, K (else null); P, J, K above
   // are then the alpha ones.  want: bit 0 J, bit 1 K.
   const double* P2;
@@ -333,16 +333,15 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
     const bool active = in_list && sub == 0;          // the lane that digests and counts the entry
     const long long te = plan.item0[seg] + (in_list ? at : plan.count[seg] - 1) - a.base;
     const int2 qd = a.quartets[te];
-    const PairJK b = load_pair_jk(a.jkrec, a.pairR, qd.x);
-    const PairJK k = load_pair_jk(a.jkrec, a.pairR, qd.y);
+    const PairJK b = load_pair_jk(a.jkrec, a.xyz4, qd.x);
+    const PairJK k = load_pair_jk(a.jkrec, a.xyz4, qd.y);
     const bool any_same = b.atom_hi == b.atom_lo || k.atom_hi == k.atom_lo || b.atom_hi == k.atom_hi ||
                           b.atom_hi == k.atom_lo || b.atom_lo == k.atom_hi || b.atom_lo == k.atom_lo;
     const PrimPair* bp = any_same ? a.prim_full + b.full_off : a.prim_skip + b.skip_off;
     const PrimPair* kp = any_same ? a.prim_full + k.full_off : a.prim_skip + k.skip_off;
     const int nbp = any_same ? b.n_full : b.n_skip;
     const int nkp = any_same ? k.n_full : k.n_skip;
-    const double Rab[3] = {b.Rx, b.Ry, b.Rz};
-    const double Rcd[3] = {k.Rx, k.Ry, k.Rz};
+    const QuartetGeom geom = quartet_geom(b, k);
     // this lane's share of the primitive quartets
     const int npq = nbp * nkp;
     const int p0 = lg ? (int)((long long)npq * sub >> lg) : 0;
@@ -357,13 +356,13 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
       if (qd.x == qd.y) f *= 0.5;
       double I[Q::NA][Q::NB][Q::NC * Q::ND];
       T esfs[Q::NE][Q::NF];
-      accumulate_esfs<LA, LB, LC, LD, T>(bp, nbp, kp, nkp, p0, np, Rab, Rcd, esfs, rys_tab);
+      accumulate_esfs<LA, LB, LC, LD, T>(bp, nbp, kp, nkp, p0, np, geom, esfs, rys_tab);
       for (int o = 1; o < 1 << lg; o <<= 1)
 #pragma unroll
         for (int e = 0; e < Q::NE; ++e)
 #pragma unroll
           for (int q = 0; q < Q::NF; ++q) esfs[e][q] += __shfl_xor_sync(0xffffffffu, esfs[e][q], o);
-      hrr_quartet<LA, LB, LC, LD, T>(esfs, Rab, Rcd, I);
+      hrr_quartet<LA, LB, LC, LD, T>(esfs, geom.Rab, geom.Rcd, I);
       digest_jk<LA, LB, LC, LD, V>(a, mi, I, f, qd.x, b.cart_hi, b.cart_lo, k.cart_hi, k.cart_lo);
     } else {
       const unsigned mask = active ? a.qmask[te] : 0u;
@@ -375,11 +374,11 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
       const PrimPair* bmp[MB];
 #pragma unroll
       for (int m = 0; m < MB; ++m) {
-        bm[m] = load_pair_jk(a.jkrec, a.pairR, mid[m] >= 0 ? mid[m] : qd.x);
+        bm[m] = load_pair_jk(a.jkrec, a.xyz4, mid[m] >= 0 ? mid[m] : qd.x);
         bmp[m] = mid[m] < 0 ? nullptr : (any_same ? a.prim_full + bm[m].full_off : a.prim_skip + bm[m].skip_off);
       }
       T esfs[MB][Q::NE][Q::NF];
-      accumulate_esfs_fam<LA, LB, LC, LD, T, MB>(bp, nbp, kp, nkp, p0, np, Rab, Rcd, bmp, esfs, rys_tab);
+      accumulate_esfs_fam<LA, LB, LC, LD, T, MB>(bp, nbp, kp, nkp, p0, np, geom, bmp, esfs, rys_tab);
       for (int o = 1; o < 1 << lg; o <<= 1)
 #pragma unroll
         for (int m = 0; m < MB; ++m)
@@ -394,7 +393,7 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
         if (bm[m].same) f *= 0.5;
         if (mid[m] == qd.y) f *= 0.5;
         double I[Q::NA][Q::NB][Q::NC * Q::ND];
-        hrr_quartet<LA, LB, LC, LD, T>(esfs[m], Rab, Rcd, I);
+        hrr_quartet<LA, LB, LC, LD, T>(esfs[m], geom.Rab, geom.Rcd, I);
         digest_jk<LA, LB, LC, LD, V>(a, mi, I, f, mid[m] >= 0 ? mid[m] : qd.x, bm[m].cart_hi, bm[m].cart_lo,
                                      k.cart_hi, k.cart_lo);
       }

@@ -75,7 +75,7 @@ __constant__ unsigned char c_cidx[LCOMP + 1][LCOMP + 1][LCOMP + 1];
 // sm: this warp's scratch, i2d + 2 buf doubles (W_SMEM for s, p, d in shared memory,
 // WF_SCRATCH up to f).  Returns the number of primitive quartets.
 __device__ int warp_quartet(const WarpQuartet& q, const PrimPair* __restrict__ bp, int nbp,
-                            const PrimPair* __restrict__ kp, int nkp, const double* Rab, const double* Rcd,
+                            const PrimPair* __restrict__ kp, int nkp, const QuartetGeom& geo,
                             double* __restrict__ sm, double*& out, int i2d = W_I2D, int buf = W_BUF) {
   const int lane = threadIdx.x & 31;
   double* I2 = sm;                     // [3][nr][d1][d2]
@@ -85,19 +85,17 @@ __device__ int warp_quartet(const WarpQuartet& q, const PrimPair* __restrict__ b
   for (int k = lane; k < nef; k += 32) es[k] = 0.0;
   const int tsz = q.d1 * q.d2;
   for (int ib = 0; ib < nbp; ++ib) {
-    const double4 b0 = ldg256(bp + ib);
-    const double4 b1 = ldg256(&bp[ib].cc);
-    const double bcc = b1.x * TWOPI5ON2;
+    const PrimRegs b0 = load_prim(bp, ib);
+    const double bcc = b0.y * TWOPI5ON2;
     for (int ik = 0; ik < nkp; ++ik) {
-      const double4 k0 = ldg256(kp + ik);
-      const double4 k1 = ldg256(&kp[ik].cc);
-      const double kcc = k1.x;
-      const double zeta = b0.w, eta = k0.w;
+      const PrimRegs k0 = load_prim(kp, ik);
+      const double kcc = k0.y;
+      const double zeta = b0.x, eta = k0.x;
       const double sq = rsqrt_nr(zeta + eta);
       const double inv = sq * sq;
       const double rho = zeta * eta * inv;
-      const double QP[3] = {k0.x - b0.x, k0.y - b0.y, k0.z - b0.z};
-      const double xx = rho * (QP[0] * QP[0] + QP[1] * QP[1] + QP[2] * QP[2]);
+      const PrimGeom pg = prim_geom(b0, k0, geo);
+      const double xx = rho * (pg.QP[0] * pg.QP[0] + pg.QP[1] * pg.QP[1] + pg.QP[2] * pg.QP[2]);
       double u[WNR_MAX], w[WNR_MAX];
       switch (q.nr) {
         case 1: { double uu[1], ww[1]; rys_eval<1>(xx, uu, ww); u[0] = uu[0]; w[0] = ww[0]; } break;
@@ -119,9 +117,8 @@ __device__ int warp_quartet(const WarpQuartet& q, const PrimPair* __restrict__ b
         for (int i = 0; i < WNR_MAX; ++i)
           if (i == r) { t2 = u[i]; wr = w[i]; }
         const double t2_rz = t2 * r_z, t2_re = t2 * r_e;
-        const double B10 = (1.0 - t2_rz) * b1.y, B01 = (1.0 - t2_re) * k1.y, B00 = 0.5 * t2 * inv;
-        const double PA = b1.z * Rab[d], QC = k1.z * Rcd[d];
-        const double c00 = PA + t2_rz * QP[d], d00 = QC - t2_re * QP[d];
+        const double B10 = (1.0 - t2_rz) * b0.w, B01 = (1.0 - t2_re) * k0.w, B00 = 0.5 * t2 * inv;
+        const double c00 = pg.PA[d] + t2_rz * pg.QP[d], d00 = pg.QC[d] - t2_re * pg.QP[d];
         double* I = I2 + (d * q.nr + r) * tsz;
         I[0] = (d == 2) ? wr * scale : 1.0;
         if (q.d1 > 1) I[q.d2] = c00 * I[0];
@@ -170,7 +167,7 @@ __device__ int warp_quartet(const WarpQuartet& q, const PrimPair* __restrict__ b
         const int g = q.ff + c;
         const int cx2 = c_comp[0][g] + (dir == 0), cy2 = c_comp[1][g] + (dir == 1), cz2 = c_comp[2][g] + (dir == 2);
         const int gp = ncart_upto(cx2 + cy2 + cz2 - 1) + c_cidx[cx2][cy2][cz2] - q.ff;
-        dst[t] = src[(e * ncr + gp) * ny + y0] + Rcd[dir] * src[(e * ncr + c) * ny + y0];
+        dst[t] = src[(e * ncr + gp) * ny + y0] + geo.Rcd[dir] * src[(e * ncr + c) * ny + y0];
       }
       __syncwarp();
       double* tmp = src; src = dst; dst = tmp;
@@ -207,7 +204,7 @@ __device__ int warp_quartet(const WarpQuartet& q, const PrimPair* __restrict__ b
         const int g = q.fe + a;
         const int ax = c_comp[0][g] + (dir == 0), ay = c_comp[1][g] + (dir == 1), az = c_comp[2][g] + (dir == 2);
         const int gp = ncart_upto(ax + ay + az - 1) + c_cidx[ax][ay][az] - q.fe;
-        dst[t] = src[(gp * nb + b0) * ncd + r] + Rab[dir] * src[(a * nb + b0) * ncd + r];
+        dst[t] = src[(gp * nb + b0) * ncd + r] + geo.Rab[dir] * src[(a * nb + b0) * ncd + r];
       }
       __syncwarp();
       double* tmp = src; src = dst; dst = tmp;

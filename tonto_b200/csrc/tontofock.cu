@@ -100,14 +100,10 @@ __global__ void k_pair_prep(int n_pairs, PairRec* __restrict__ pairs, const doub
       const double ea = hi_is_a ? eh : el, eb = hi_is_a ? el : eh;
       const double prefac = same ? 1.0 : exp(-ea * (eb * r2) * inv);
       PrimPair q;
-      q.Px = (eh * A[0] + el * B[0]) * inv;
-      q.Py = (eh * A[1] + el * B[1]) * inv;
-      q.Pz = (eh * A[2] + el * B[2]) * inv;
       q.zeta = zeta;
       q.f = -el * inv;
       q.half_zinv = 0.5 * inv;
       q.cc = ch * cl * inv * prefac;      // c_a c_b / zeta x prefactor: see PrimPair
-      q.pad = 0.0;
       prim_full[pr.full_off + i] = q;
       if (!same && !(prefac < pair_cutoff)) prim_skip[pr.skip_off + k++] = q;
     }
@@ -135,7 +131,7 @@ __global__ void __launch_bounds__(32 * SCHWARZ_WARPS) k_schwarz(const int* __res
   const long long npq = (long long)pr.n_full * pr.n_full;
   const int p0 = (int)(npq * lane / 32), np = (int)(npq * (lane + 1) / 32) - p0;
   accumulate_esfs<LA, LB, LA, LB, double>(prim_full + pr.full_off, pr.n_full, prim_full + pr.full_off, pr.n_full, p0,
-                                          np, R, R, es);
+                                          np, QuartetGeom{{R[0], R[1], R[2]}, {R[0], R[1], R[2]}, {0.0, 0.0, 0.0}}, es);
 #pragma unroll
   for (int e = 0; e < Q::NE; ++e)
 #pragma unroll
@@ -573,7 +569,8 @@ __global__ void __launch_bounds__(32 * WARPS_PER_BLOCK) k_schwarz_warp(const int
     const PairRec pr = pairs[p];
     const double R[3] = {pr.Rx, pr.Ry, pr.Rz};
     double* I = nullptr;
-    warp_quartet(q, prim_full + pr.full_off, pr.n_full, prim_full + pr.full_off, pr.n_full, R, R, sm, I, i2d, wbuf);
+    warp_quartet(q, prim_full + pr.full_off, pr.n_full, prim_full + pr.full_off, pr.n_full,
+                 QuartetGeom{{R[0], R[1], R[2]}, {R[0], R[1], R[2]}, {0.0, 0.0, 0.0}}, sm, I, i2d, wbuf);
     double m = 0.0;
     for (int e = lane; e < MA * MB; e += 32) {
       const int ma = e / MB, mb = e % MB;
@@ -691,6 +688,7 @@ __global__ void __launch_bounds__(32 * ONE_EL_WARPS) k_one_electron(
     const MolInfo mi = mols[pr.mol];
     const PrimPair* pp = prim_full + pr.full_off;
     const double AB[3] = {pr.Rx, pr.Ry, pr.Rz};
+    const double* A = xyz + 3 * pr.atom_hi;
     const int nl = shell_nprim[pr.sh_lo];
     double s_c[NA][NB], t_c[NA][NB], v_c[NA][NB];
 #pragma unroll
@@ -742,8 +740,9 @@ __global__ void __launch_bounds__(32 * ONE_EL_WARPS) k_one_electron(
     for (int q0 = lane; q0 < n_work; q0 += 32) {
       const int p = q0 / mi.n_atom, at = mi.atom0 + q0 - p * mi.n_atom;
       const PrimPair q = pp[p];
-      const double PC[3] = {q.Px - xyz[3 * at], q.Py - xyz[3 * at + 1], q.Pz - xyz[3 * at + 2]};
       const double PA[3] = {q.f * AB[0], q.f * AB[1], q.f * AB[2]};
+      const double PC[3] = {PA[0] + (A[0] - xyz[3 * at]), PA[1] + (A[1] - xyz[3 * at + 1]),
+                            PA[2] + (A[2] - xyz[3 * at + 2])};
       const double x = q.zeta * (PC[0] * PC[0] + PC[1] * PC[1] + PC[2] * PC[2]);
       double u[NR], w[NR];
       RT::eval(one_el_tab, x, u, w);
@@ -1142,7 +1141,7 @@ struct tf_ctx {
   tf::DBuf<long long> d_fam_coff;                        // their member masks in d_cmask
   tf::DBuf<unsigned char> d_cmask;                       // recorded member mask per candidate ket
   tf::DBuf<int4> d_srec, d_jkrec;
-  tf::DBuf<double2> d_pairR;
+  tf::DBuf<double4> d_xyz4;                              // atom positions, 32 bytes each (load_pair_jk)
   tf::DBuf<long long> d_task_cand_off;
   tf::DBuf<long long> d_counts, d_offsets, d_group_offsets;
   tf::DBuf<tf::LaunchPlan> d_plans;                      // per group: its FP64 and its FP32 launch
@@ -1826,23 +1825,22 @@ static int setup_pairs(tf_ctx* c) {
   const std::vector<int>& sorted = c->lists.sorted;
   const std::vector<double>& simax = c->lists.simax;
   const std::vector<double>& sbmax = c->lists.sbmax;
-  // packed pair records of the ERI kernels (load_pair_jk)
+  // packed pair records and atom positions of the ERI kernels (load_pair_jk)
   {
+    std::vector<double4> x4(c->n_atom);
+    for (int i = 0; i < c->n_atom; ++i) x4[i] = make_double4(c->xyz[3 * i], c->xyz[3 * i + 1], c->xyz[3 * i + 2], 0.0);
+    TF_CUDA(c->d_xyz4.reserve(std::max<size_t>(x4.size(), 1)));
+    TF_CUDA(cudaMemcpy(c->d_xyz4.p, x4.data(), x4.size() * sizeof(double4), cudaMemcpyHostToDevice));
     std::vector<int4> jr(2 * c->n_pairs);
-    std::vector<double2> pr2(2 * c->n_pairs);
     for (long long p = 0; p < c->n_pairs; ++p) {
       const PairRec& q = c->pairs_h[p];
       if (q.n_full > 0xffff || q.n_skip > 0xffff) { set_error("too many primitive pairs in one shell pair"); return TF_EUNSUPPORTED; }
       jr[2 * p] = make_int4(q.cart_hi, q.cart_lo, q.full_off, q.skip_off);
       jr[2 * p + 1] = make_int4(q.atom_hi, q.atom_lo, q.n_full | (q.n_skip << 16),
                                 (int)((unsigned)q.mol | (q.sh_hi == q.sh_lo ? 0x80000000u : 0u)));
-      pr2[2 * p] = make_double2(q.Rx, q.Ry);
-      pr2[2 * p + 1] = make_double2(q.Rz, 0.0);
     }
     TF_CUDA(c->d_jkrec.reserve(std::max<size_t>(jr.size(), 1)));
-    TF_CUDA(c->d_pairR.reserve(std::max<size_t>(pr2.size(), 1)));
     TF_CUDA(cudaMemcpy(c->d_jkrec.p, jr.data(), jr.size() * sizeof(int4), cudaMemcpyHostToDevice));
-    TF_CUDA(cudaMemcpy(c->d_pairR.p, pr2.data(), pr2.size() * sizeof(double2), cudaMemcpyHostToDevice));
   }
   std::vector<int4> srec(sorted.size());
   for (size_t q = 0; q < sorted.size(); ++q) {
@@ -1920,7 +1918,7 @@ static int dispatch_jk(int la, int lb, int lc, int ld, const JKArgs& a, cudaStre
       launch_jk_d(key, a, s, fp32, variant) || launch_jk_f(key, a, s, fp32, variant))
     return TF_OK;
   const RowArgs r{a.quartets + (a.range ? 0 : a.first - a.base), a.n, a.prim_full, a.prim_skip, a.P, a.J, a.K, a.mols, a.prim_count, a.range, a.base,
-                  a.cap, a.jkrec, a.pairR, a.P2, a.J2, a.K2, a.want,
+                  a.cap, a.jkrec, a.xyz4, a.P2, a.J2, a.K2, a.want,
                   a.qcount ? a.qcount + (a.bucket32 ? NQCLS : 0) : nullptr, a.fx_lo};
   for (auto* launch : {launch_rows_d, launch_rows_fs, launch_rows_fd, launch_rows_ff}) {
     const int rc = launch(key, r, s);
@@ -2147,7 +2145,7 @@ static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* d
     cudaStream_t sg = branch_of(c, g, ns);
     JKArgs a{c->d_quartets.p, 0, c->d_pairs.p, c->d_prim_full.p, c->d_prim_skip.p, c->d_Pc.p, c->d_Jc.p,
              c->d_Kc.p, c->d_mols.p, c->d_prim_count.p, c->d_plans.p + 2 * g, c->d_group_offsets.p + 3 * g, 0,
-             c->graph_cap, 0, c->d_jkrec.p, c->d_pairR.p, dPb ? c->d_PcB.p : nullptr, dPb ? c->d_JcB.p : nullptr,
+             c->graph_cap, 0, c->d_jkrec.p, c->d_xyz4.p, dPb ? c->d_PcB.p : nullptr, dPb ? c->d_JcB.p : nullptr,
              dPb ? c->d_KcB.p : nullptr, want};
     a.qmask = c->d_qmask.p;
     a.fam_mem = c->d_fam_mem.p;
@@ -2396,7 +2394,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
       JKArgs a{c->d_quartets.p, goff[3 * g + 1] - goff[3 * g], c->d_pairs.p,
                c->d_prim_full.p, c->d_prim_skip.p, c->d_Pc.p, c->d_Jc.p, c->d_Kc.p, c->d_mols.p,
                c->d_prim_count.p, c->d_plans.p + 2 * g, nullptr, base, LLONG_MAX, goff[3 * g], c->d_jkrec.p,
-               c->d_pairR.p,
+               c->d_xyz4.p,
                dPb ? c->d_PcB.p : nullptr, dPb ? c->d_JcB.p : nullptr, dPb ? c->d_KcB.p : nullptr, want};
       a.qmask = c->d_qmask.p;
       a.fam_mem = c->d_fam_mem.p;
