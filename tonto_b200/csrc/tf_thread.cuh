@@ -96,6 +96,43 @@ constexpr int jk_threads() {
   return jk_min_blocks<LA, LB, LC, LD, V>() == 1 ? 256 : 128 * jk_min_blocks<LA, LB, LC, LD, V>();
 }
 
+// N consecutive doubles of a density row at a shell's first column: p, d and f shells start
+// on 32-byte boundaries and are padded to whole words (the context's Cartesian order).
+template <int N>
+__device__ __forceinline__ void load_row(const double* __restrict__ p, double (&v)[N]) {
+  if constexpr (N == 1) {
+    v[0] = __ldg(p);
+  } else {
+#pragma unroll
+    for (int i = 0; i < N; i += 4) {
+      const double4 x = ldg256(p + i);
+      v[i] = x.x;
+      if (i + 1 < N) v[i + 1] = x.y;
+      if (i + 2 < N) v[i + 2] = x.z;
+      if (i + 3 < N) v[i + 3] = x.w;
+    }
+  }
+}
+
+// Block (x, y) of the (symmetric) density, shells of NX and NY components at ox and oy,
+// read along the wider one: a gather touches a sector per lane and row, whatever of
+// its 32 bytes is used.
+template <int NX, int NY>
+__device__ __forceinline__ void load_block(const double* __restrict__ P, int n, int ox, int oy, double (&v)[NX][NY]) {
+  if constexpr (NY >= NX) {
+#pragma unroll
+    for (int x = 0; x < NX; ++x) load_row<NY>(P + (size_t)(ox + x) * n + oy, v[x]);
+  } else {
+#pragma unroll
+    for (int y = 0; y < NY; ++y) {
+      double r[NX];
+      load_row<NX>(P + (size_t)(oy + y) * n + ox, r);
+#pragma unroll
+      for (int x = 0; x < NX; ++x) v[x][y] = r[x];
+    }
+  }
+}
+
 // Digestion of one quartet's Cartesian integrals I into J and K with the coincidence
 // factor f (f = 0: the lane adds nothing but still takes part in the warp sums):
 // bid is the bra pair (lanes of one bra are summed together), ob/oa the bra's and
@@ -131,10 +168,7 @@ __device__ __forceinline__ void digest_jk(const JKArgs& a, const MolInfo& mi,
   const bool taila = lane == 31 || ((heada >> (lane + 1)) & 1u);
   auto digest_j = [&](const double* __restrict__ P, double* __restrict__ Jm) {
     double Pcd[Q::NC][Q::ND];
-#pragma unroll
-    for (int c = 0; c < Q::NC; ++c)
-#pragma unroll
-      for (int d = 0; d < Q::ND; ++d) Pcd[c][d] = __ldg(P + (size_t)(oc + c) * n + od + d);
+    load_block<Q::NC, Q::ND>(P, n, oc, od, Pcd);
 #pragma unroll
     for (int ia = 0; ia < Q::NA; ++ia)
 #pragma unroll
@@ -160,10 +194,7 @@ __device__ __forceinline__ void digest_jk(const JKArgs& a, const MolInfo& mi,
       }
     if (live) {
       double Pab[Q::NA][Q::NB];
-#pragma unroll
-      for (int ia = 0; ia < Q::NA; ++ia)
-#pragma unroll
-        for (int ib = 0; ib < Q::NB; ++ib) Pab[ia][ib] = __ldg(P + (size_t)(oa + ia) * n + ob + ib);
+      load_block<Q::NA, Q::NB>(P, n, oa, ob, Pab);
 #pragma unroll
       for (int c = 0; c < Q::NC; ++c)
 #pragma unroll
@@ -218,20 +249,28 @@ __device__ __forceinline__ void digest_jk(const JKArgs& a, const MolInfo& mi,
 #pragma unroll
       for (int d = 0; d < Q::ND; ++d) Kbd[ib][d] = 0.0;
     }
-#pragma unroll
-    for (int ib = 0; ib < Q::NB; ++ib) {
-#pragma unroll
-      for (int d = 0; d < Q::ND; ++d) Pbd[ib][d] = __ldg(P + (size_t)(ob + ib) * n + od + d);
-#pragma unroll
-      for (int c = 0; c < Q::NC; ++c) Pbc[ib][c] = __ldg(P + (size_t)(ob + ib) * n + oc + c);
-    }
+    load_block<Q::NB, Q::ND>(P, n, ob, od, Pbd);
+    load_block<Q::NB, Q::NC>(P, n, ob, oc, Pbc);
+    // (a, c) and (a, d): whole blocks when read along a, else row by row with a
+    constexpr bool ALONG_A_D = Q::NA > Q::ND, ALONG_A_C = Q::NA > Q::NC;
+    double PadA[ALONG_A_D ? Q::NA : 1][Q::ND], PacA[ALONG_A_C ? Q::NA : 1][Q::NC];
+    if constexpr (ALONG_A_D) load_block<Q::NA, Q::ND>(P, n, oa, od, PadA);
+    if constexpr (ALONG_A_C) load_block<Q::NA, Q::NC>(P, n, oa, oc, PacA);
 #pragma unroll
     for (int ia = 0; ia < Q::NA; ++ia) {
       double Pad[Q::ND], Pac[Q::NC];
+      if constexpr (ALONG_A_D) {
 #pragma unroll
-      for (int d = 0; d < Q::ND; ++d) Pad[d] = __ldg(P + (size_t)(oa + ia) * n + od + d);
+        for (int d = 0; d < Q::ND; ++d) Pad[d] = PadA[ia][d];
+      } else {
+        load_row<Q::ND>(P + (size_t)(oa + ia) * n + od, Pad);
+      }
+      if constexpr (ALONG_A_C) {
 #pragma unroll
-      for (int c = 0; c < Q::NC; ++c) Pac[c] = __ldg(P + (size_t)(oa + ia) * n + oc + c);
+        for (int c = 0; c < Q::NC; ++c) Pac[c] = PacA[ia][c];
+      } else {
+        load_row<Q::NC>(P + (size_t)(oa + ia) * n + oc, Pac);
+      }
 #pragma unroll
       for (int c = 0; c < Q::NC; ++c) {
         double s = 0.0;

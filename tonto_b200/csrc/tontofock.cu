@@ -201,6 +201,7 @@ __global__ void k_density_to_cart(BatchArgs b, const double* __restrict__ P, con
   const long long r = t - mi.cmat;
   const int p = (int)(r / mi.n_cart), q = (int)(r % mi.n_cart);
   const int sp = b.cart_shell[mi.cart0 + p], sq = b.cart_shell[mi.cart0 + q];
+  if (sp < 0 || sq < 0) { Pc[t] = 0.0; return; }       // padding
   const int ip = b.cart_local[mi.cart0 + p], iq = b.cart_local[mi.cart0 + q];
   const int lp = b.shell_l[sp], lq = b.shell_l[sq];
   const int fp = b.shell_first_bf[sp], fq = b.shell_first_bf[sq];
@@ -2521,15 +2522,26 @@ static int create_impl(const tf_basis* bases, int n_mol, const tf_options* opt, 
       c->shell_nprim.push_back(B->shell_nprim[s]);
       c->shell_first_bf.push_back(nb);
       c->shell_poff.push_back((int)c->exps.size() + np);
-      c->shell_cart.push_back(nc);
+      c->shell_cart.push_back(0);              // (below)
       const int nbf_s = (c->spherical && l >= 2) ? 2 * l + 1 : ncart(l);
       c->shell_nbf.push_back(nbf_s);
-      for (int i = 0; i < ncart(l); ++i) { cart_shell.push_back(mi.shell0 + s); cart_local.push_back(i); }
       for (int i = 0; i < nbf_s; ++i) { bf_shell.push_back(mi.shell0 + s); bf_local.push_back(i); }
       np += B->shell_nprim[s];
-      nc += ncart(l);
       nb += nbf_s;
     }
+    // Cartesian functions of the molecule, an order of this library's own: all s shells, then
+    // p, d and f shells, each p, d or f shell on a 32-byte boundary and padded to whole
+    // 32-byte words (4, 8 and 12 columns).  A shell's columns of a density row are then one to
+    // three load instructions and sectors, and the s columns a warp's kets touch are neighbours.
+    for (int l = 0; l <= LMAX_SUPPORTED; ++l)
+      for (int s = 0; s < B->n_shell; ++s) {
+        if (B->shell_l[s] != l) continue;
+        if (l > 0) while (nc % 4) { cart_shell.push_back(-1); cart_local.push_back(0); ++nc; }
+        c->shell_cart[mi.shell0 + s] = nc;
+        for (int i = 0; i < ncart(l); ++i) { cart_shell.push_back(mi.shell0 + s); cart_local.push_back(i); }
+        nc += ncart(l);
+      }
+    while (nc % 4) { cart_shell.push_back(-1); cart_local.push_back(0); ++nc; }
     c->exps.insert(c->exps.end(), B->exponents, B->exponents + np);
     c->coefs.insert(c->coefs.end(), B->coefficients, B->coefficients + np);
     c->xyz.insert(c->xyz.end(), B->xyz, B->xyz + 3 * B->n_atom);
