@@ -721,6 +721,9 @@ __device__ __forceinline__ void prim_quartet_vrr(const PrimRegs& B, const PrimRe
 // prefactor, the recurrence coefficients, the 2D recurrences and the (e0|f0)
 // products); P - Q in FP64 (a difference of positions), then the nodes and weights
 // themselves in FP64 from the FP64 tables, as for the FP64 path.
+// The order of every FP32 operation is written out (no contraction left to the compiler):
+// an incremental build is nearly all FP32 quartets, so a different rounding shows in its
+// result, and all kernel variants of a class should give the same one.
 template <int LA, int LB, int LC, int LD>
 __device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRegs& K, const QuartetGeom& g,
                                                  float (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
@@ -730,55 +733,70 @@ __device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRe
   const PrimGeom p = prim_geom(B, K, g);
   const float zeta = (float)B.x, eta = (float)K.x;
   const float half_zinv = (float)B.w, half_einv = (float)K.w;
-  const float sq = rsqrt_f32(zeta + eta);
-  const float inv = sq * sq;
-  const float rho = zeta * eta * inv;
+  const float sq = rsqrt_f32(__fadd_rn(zeta, eta));
+  const float inv = __fmul_rn(sq, sq);
+  const float rho = __fmul_rn(__fmul_rn(zeta, eta), inv);
   const float QP[3] = {(float)p.QP[0], (float)p.QP[1], (float)p.QP[2]};
-  const float xx = rho * (QP[0] * QP[0] + QP[1] * QP[1] + QP[2] * QP[2]);
+  const float xx = __fmul_rn(rho, __fmaf_rn(QP[2], QP[2], __fmaf_rn(QP[0], QP[0], __fmul_rn(QP[1], QP[1]))));
   double u[NR], w[NR];
   if (rys_smem) RysSmem<NR>::eval(rys_smem, (double)xx, u, w);
   else rys_eval<NR>((double)xx, u, w);
-  const float scale = (float)(B.y * K.y * TWOPI5ON2) * sq;
-  const float r_z = eta * inv;     // rho / zeta
-  const float r_e = zeta * inv;    // rho / eta
+  const float scale = __fmul_rn((float)(B.y * K.y * TWOPI5ON2), sq);
+  const float r_z = __fmul_rn(eta, inv);     // rho / zeta
+  const float r_e = __fmul_rn(zeta, inv);    // rho / eta
   const float PA[3] = {(float)p.PA[0], (float)p.PA[1], (float)p.PA[2]};
   const float QC[3] = {(float)p.QC[0], (float)p.QC[1], (float)p.QC[2]};
 #pragma unroll
   for (int r = 0; r < NR; ++r) {
     const float t2 = (float)u[r];
-    const float t2_rz = t2 * r_z, t2_re = t2 * r_e;
-    const float B10 = (1.0f - t2_rz) * half_zinv;
-    const float B01 = (1.0f - t2_re) * half_einv;
-    const float B00 = 0.5f * t2 * inv;
-    const float wt = (float)w[r] * scale;
+    const float t2_rz = __fmul_rn(t2, r_z), t2_re = __fmul_rn(t2, r_e);
+    const float B10 = __fmul_rn(__fsub_rn(1.0f, t2_rz), half_zinv);
+    const float B01 = __fmul_rn(__fsub_rn(1.0f, t2_re), half_einv);
+    const float B00 = __fmul_rn(__fmul_rn(0.5f, t2), inv);
+    const float wt = __fmul_rn((float)w[r], scale);
     float I[3][D1][D2];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
-      const float c00 = fmaf(t2_rz, QP[d], PA[d]);
-      const float d00 = fmaf(-t2_re, QP[d], QC[d]);
+      const float c00 = __fmaf_rn(t2_rz, QP[d], PA[d]);
+      const float d00 = __fmaf_rn(-t2_re, QP[d], QC[d]);
       I[d][0][0] = (d == 2) ? wt : 1.0f;
-      if (D1 > 1) I[d][1][0] = c00 * I[d][0][0];
+      if (D1 > 1) I[d][1][0] = d == 2 ? __fmul_rn(c00, wt) : c00;
 #pragma unroll
-      for (int e = 1; e + 1 < D1; ++e) I[d][e + 1][0] = c00 * I[d][e][0] + float(e) * B10 * I[d][e - 1][0];
+      for (int e = 1; e + 1 < D1; ++e)
+        I[d][e + 1][0] = d == 2 && D1 == 3 ? __fmaf_rn(B10, I[d][0][0], __fmul_rn(c00, I[d][1][0]))
+                                : __fmaf_rn(c00, I[d][e][0], __fmul_rn(__fmul_rn(float(e), B10), I[d][e - 1][0]));
 #pragma unroll
       for (int f = 0; f + 1 < D2; ++f) {
 #pragma unroll
         for (int e = 0; e < D1; ++e) {
-          float v = d00 * I[d][e][f];
-          if (f > 0) v += float(f) * B01 * I[d][e][f - 1];
-          if (e > 0) v += float(e) * B00 * I[d][e - 1][f];
+          const float i0 = I[d][e][f];
+          float v;
+          if (f > 0) {
+            v = __fmaf_rn(d00, i0, __fmul_rn(__fmul_rn(float(f), B01), I[d][e][f - 1]));
+            if (e > 0) v = __fmaf_rn(__fmul_rn(float(e), B00), I[d][e - 1][f], v);
+          } else if (e > 0) {
+            v = __fmaf_rn(d00, i0, __fmul_rn(__fmul_rn(float(e), B00), I[d][e - 1][f]));
+          } else {
+            v = __fmul_rn(d00, i0);
+          }
           I[d][e][f + 1] = v;
         }
       }
     }
-    static_for<Q::NE>([&](auto e) {
-      constexpr int ge = Q::FE + decltype(e)::value;
-      static_for<Q::NF>([&](auto f) {
-        constexpr int gf = Q::FF + decltype(f)::value;
-        esfs[decltype(e)::value][decltype(f)::value] +=
-            I[0][gx(ge)][gx(gf)] * I[1][gy(ge)][gy(gf)] * I[2][gz(ge)][gz(gf)];
+    if constexpr (Q::LAB == 1 && Q::LCD == 0) {      // one product per element, none rounded by itself
+      esfs[0][0] = __fmaf_rn(I[0][1][0], wt, esfs[0][0]);
+      esfs[1][0] = __fmaf_rn(I[1][1][0], wt, esfs[1][0]);
+      esfs[2][0] = __fmaf_rn(__fmaf_rn(t2_rz, QP[2], PA[2]), wt, esfs[2][0]);
+    } else {
+      static_for<Q::NE>([&](auto e) {
+        constexpr int ge = Q::FE + decltype(e)::value;
+        static_for<Q::NF>([&](auto f) {
+          constexpr int gf = Q::FF + decltype(f)::value;
+          float& es = esfs[decltype(e)::value][decltype(f)::value];
+          es = __fmaf_rn(__fmul_rn(I[0][gx(ge)][gx(gf)], I[1][gy(ge)][gy(gf)]), I[2][gz(ge)][gz(gf)], es);
+        });
       });
-    });
+    }
   }
 }
 

@@ -1252,10 +1252,11 @@ static BatchArgs batch_args(tf_ctx* c) {
 }
 
 // Lanes per quartet of a launch (LaunchPlan::lg).  A launch cannot end before its longest
-// quartet, so no lane should get more primitive quartets than its fair share of the
-// launch, taken over PLAN_LANES resident lanes (148 SMs, 12 warps) with a factor
-// 2 of slack, nor fewer than PLAN_MIN: beyond that the split costs more (one lane of
-// the sharers digests) than its shorter chain saves.  Measured, (ss|ss) and the whole
+// quartet, so no lane should get more primitive quartets than half its fair share of the
+// launch, taken over PLAN_LANES resident lanes (148 SMs, 12 warps), nor fewer than PLAN_MIN:
+// beyond that the split costs more (one lane of the sharers digests) than its shorter
+// chain saves.  (Shares of 2, 1, 1/2 and 1/4: (H2O)12 cc-pVDZ class by class 7.82, 7.05, 6.36 and
+// 6.21 ms, overlapped 5.01, 5.04, 5.04 and 5.14.)  Measured, (ss|ss) and the whole
 // build, one thread a quartet throughout -> split: (H2O)2 cc-pVTZ 1.32 -> 0.06 and 2.12 -> 0.87
 // ms, (H2O)3 6-31G(d) 0.35 -> 0.02 and 0.54 -> 0.31, (H2O)7 cc-pVDZ 1.77 -> 0.34 and 2.04 ->
 // 1.68; (H2O)32 cc-pVDZ, where few buckets are split, 72.7 -> 73.0 ms.
@@ -1299,7 +1300,7 @@ __global__ void __launch_bounds__(64) k_group_offsets(int n_groups, const int* _
   }
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) work += __shfl_xor_sync(0xffffffffu, work, o);
-  const double share = fmax((double)PLAN_MIN, 2.0 * work / PLAN_LANES);
+  const double share = fmax((double)PLAN_MIN, 0.5 * work / PLAN_LANES);
   long long start = 0;
 #pragma unroll
   for (int q = 0; q < 2; ++q) {
@@ -1626,6 +1627,27 @@ static void make_task_plan(const ClassLists& L, const std::vector<PairRec>& pair
   }
 }
 
+// pair class id -> (lh, ll)
+static void class_l(int k, int& lh, int& ll) {
+  lh = 0;
+  while ((lh + 1) * (lh + 2) / 2 <= k) ++lh;
+  ll = k - lh * (lh + 1) / 2;
+}
+
+// Kernel variant of a class pair that no autotuner has chosen one for.  Two and three quanta
+// with an ss or ps ket (the vertical-recurrence classes beyond (ps|ss)) have few live values for
+// their latency: 16 resident warps (bit 0) against 8; with a ps ket and an s on the bra
+// most of the time is K adds, merged over lanes first (bit 1).  The classes above spill
+// at 16 warps and (ss|ss), (ps|ss) run 20 without it.  Measured, (H2O)32 cc-pVDZ, variants 0
+// to 3 in ms: (ps|ps) 8.4 6.8 9.5 6.6, (ds|ps) 4.7 4.4 5.5 4.1, (pp|ps) 5.1 4.9 6.0 5.1, (pp|ss)
+// 4.4 3.2 5.3 3.5, (ds|ss) 3.7 2.9 4.7 3.2, (dp|ss) 2.0 1.5 2.5 1.7; (dp|ps) 2.8 5.2 4.0 5.5, (ps|ss)
+// 11.0 11.7 11.7 12.1, (ss|ss) 7.6 7.9 7.8 8.0.
+static int default_variant(int la, int lb, int lc, int ld) {
+  const int L = la + lb + lc + ld;
+  if (L < 2 || L > 3 || lc + ld > 1 || la > 2) return 0;
+  return lc == 1 && lb == 0 ? 3 : 1;
+}
+
 // Groups (class pairs p1 >= p2) of units (one per molecule having both classes);
 // tasks are (unit, bra position); with sharding this context keeps the tasks that
 // make_task_plan deals to its shard (Tonto's parallel do shares the bra pairs
@@ -1649,7 +1671,13 @@ static int build_tasks(tf_ctx* c) {
   }
   c->group_task0.push_back((int)tasks.size());
   c->n_tasks = (long long)tasks.size();
-  c->cls_variant.assign(c->group_cls.size(), 0);
+  c->cls_variant.resize(c->group_cls.size());
+  for (size_t g = 0; g < c->group_cls.size(); ++g) {
+    int l1h, l1l, l2h, l2l;
+    class_l(c->group_cls[g].x, l1h, l1l);
+    class_l(c->group_cls[g].y, l2h, l2l);
+    c->cls_variant[g] = default_variant(l1h, l1l, l2h, l2l);
+  }
   {                                    // start from the last autotuned choice on this device
     std::lock_guard<std::mutex> lock(g_variant_mutex);
     const auto it = g_variant_cache.find(c->device);
@@ -1902,13 +1930,6 @@ static void launch_one_electron(tf_ctx* c, int k, double* const* out, cudaStream
   k_one_electron<LA, LB><<<blocks, 32 * ONE_EL_WARPS, smem, s>>>(
       c->d_schwarz_ids.p + i0, n, c->d_pairs.p, c->d_mols.p, c->d_prim_full.p, c->d_xyz.p, c->d_Z.p,
       c->d_shell_nprim.p, c->d_shell_poff.p, c->d_exps.p, out[0], out[1], out[2]);
-}
-
-// pair class id -> (lh, ll)
-static void class_l(int k, int& lh, int& ll) {
-  lh = 0;
-  while ((lh + 1) * (lh + 2) / 2 <= k) ++lh;
-  ll = k - lh * (lh + 1) / 2;
 }
 
 // fp32: evaluate the 2D recurrences and (e0|f0) sums in FP32 (thread-per-quartet
