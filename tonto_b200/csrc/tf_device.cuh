@@ -32,33 +32,29 @@
 namespace tf {
 
 // ---------------------------------------------------------------------------
-// Reciprocal and reciprocal square root by Newton-Raphson iteration, seeded by
-// the PTX approximate instructions rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64
-// (about 20 correct bits).  Each step squares the relative error:
-//   1/x:       y <- y + y (1 - x y)
-//   1/sqrt(x): y <- y + y (1/2 - (x/2) y^2)
-// so two steps reach the double-precision rounding level (a few ulp; checked
-// against IEEE division and square root by tests/fast_math_check.cu).  Used for
-// the exponent sums, rho, the Boys-function ratio and 1/x of the asymptotic
-// rules: positive normal numbers far from the overflow range.
+// Reciprocal and reciprocal square root by one third-order step, seeded by the PTX
+// approximate instructions rcp.approx.ftz.f64 / rsqrt.approx.ftz.f64 (about 20 correct
+// bits).  With the residual e the truncated binomial series
+//   1/x:       e = 1 - x y,    y <- y + y (e + e^2)
+//   1/sqrt(x): e = 1 - x y^2,  y <- y + y e (1/2 + 3/8 e)
+// leaves an error of order e^3, some 2^-59, below the double-precision rounding (a few
+// ulp; checked against IEEE division and square root by tests/fast_math_check.cu): three
+// and five operations where two Newton steps take four and seven.  Used for the
+// exponent sums, rho, the Boys-function ratio and 1/x of the asymptotic rules: positive
+// normal numbers far from the overflow range.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ double rcp_nr(double x) {
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  double e = fma(-x, y, 1.0);
-  y = fma(y, e, y);
-  e = fma(-x, y, 1.0);
-  return fma(y, e, y);
+  const double e = fma(-x, y, 1.0);
+  return fma(y, fma(e, e, e), y);
 }
 
 __device__ __forceinline__ double rsqrt_nr(double x) {
   double y;
   asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
-  const double h = 0.5 * x;
-  double e = fma(-h * y, y, 0.5);
-  y = fma(y, e, y);
-  e = fma(-h * y, y, 0.5);
-  return fma(y, e, y);
+  const double e = fma(-x * y, y, 1.0);
+  return fma(y * e, fma(0.375, e, 0.5), y);
 }
 
 // ---------------------------------------------------------------------------
@@ -477,8 +473,11 @@ struct RysSmem<2> {
 
 // Boys functions F_0 .. F_M, M <= 3, of the classes evaluated by the vertical recurrence
 // (prim_quartet_vrr): the 8-term Taylor step of the grids above about the nearest point
-// k/8, one independent chain per order; beyond the grid (42, or 50 for M >= 2)
-// F_0 = sqrt(pi/x)/2 and F_{m+1} = (2m+1)/(2x) F_m, where exp(-x)/(2x) is below rounding.
+// k/8; beyond the grid (42, or 50 for M >= 2) F_0 = sqrt(pi/x)/2 and F_{m+1} = (2m+1)/(2x)
+// F_m, where exp(-x)/(2x) is below rounding.  M = 0, 1: the table holds F_j(k/8)/j!, the
+// coefficients of F_0 in d = k/8 - x; F_1 is that polynomial's derivative, one Horner scheme
+// for both (15 operations against 20 with the factors d/j).  M = 2, 3: one independent chain per
+// order, shorter in latency and no longer in operations.
 template <int M>
 struct BoysSmem {
   static constexpr bool WIDE = M >= 2;
@@ -486,8 +485,16 @@ struct BoysSmem {
   static constexpr int XMAX = WIDE ? TF_BOYS2_XMAX : TF_BOYS_XMAX;
   static constexpr int SIZE = NPTS * NM;
   static __device__ __forceinline__ void load(double* t) {
-    const double* g = WIDE ? tf_boys2_grid : tf_boys_grid;
-    for (int q = threadIdx.x; q < SIZE; q += blockDim.x) t[q] = g[q];
+    if constexpr (WIDE) {
+      for (int q = threadIdx.x; q < SIZE; q += blockDim.x) t[q] = tf_boys2_grid[q];
+    } else {
+      for (int q = threadIdx.x; q < SIZE; q += blockDim.x) {
+        const int j = q % NM;
+        const double f = j < 2 ? 1.0 : j == 2 ? 2.0 : j == 3 ? 6.0 : j == 4 ? 24.0 : j == 5 ? 120.0 : j == 6 ? 720.0
+                         : j == 7 ? 5040.0 : 40320.0;
+        t[q] = tf_boys_grid[q] / f;
+      }
+    }
   }
   static __device__ __forceinline__ void eval(const double* __restrict__ t, double x, double (&F)[M + 1]) {
     static_assert(M <= 3 && TF_BOYS_NTERM == 8, "grids of F_0 .. F_8 and F_0 .. F_10");
@@ -502,13 +509,29 @@ struct BoysSmem {
         f[2 * q] = v.x;
         f[2 * q + 1] = v.y;
       }
-      const double dj[8] = {0.0, d, d * 0.5, d * (1.0 / 3.0), d * 0.25, d * 0.2, d * (1.0 / 6.0), d * (1.0 / 7.0)};
+      if constexpr (M == 0) {
+        double p = f[7];
 #pragma unroll
-      for (int m = 0; m <= M; ++m) F[m] = f[m + 7];
+        for (int j = 6; j >= 0; --j) p = fma(p, d, f[j]);
+        F[0] = p;
+      } else if constexpr (M == 1) {
+        double p = fma(f[8], d, f[7]), q = f[8];       // value and derivative
 #pragma unroll
-      for (int j = 7; j >= 1; --j)
+        for (int j = 6; j >= 0; --j) {
+          q = fma(q, d, p);
+          p = fma(p, d, f[j]);
+        }
+        F[0] = p;
+        F[1] = q;
+      } else {
+        const double dj[8] = {0.0, d, d * 0.5, d * (1.0 / 3.0), d * 0.25, d * 0.2, d * (1.0 / 6.0), d * (1.0 / 7.0)};
 #pragma unroll
-        for (int m = 0; m <= M; ++m) F[m] = fma(dj[j], F[m], f[m + j - 1]);
+        for (int m = 0; m <= M; ++m) F[m] = f[m + 7];
+#pragma unroll
+        for (int j = 7; j >= 1; --j)
+#pragma unroll
+          for (int m = 0; m <= M; ++m) F[m] = fma(dj[j], F[m], f[m + j - 1]);
+      }
     } else {
       const double r = rsqrt_nr(x), ix = r * r;
       F[0] = tf_rys_hweight[rys_hoffset(1)] * r;
@@ -552,19 +575,30 @@ __device__ __forceinline__ QuartetGeom quartet_geom(const PairJK& b, const PairJ
   return QuartetGeom{{b.Rx, b.Ry, b.Rz}, {k.Rx, k.Ry, k.Rz}, {k.Ax - b.Ax, k.Ay - b.Ay, k.Az - b.Az}};
 }
 
-// P - A, Q - C and Q - P of a primitive quartet.
+// P - A, Q - C and Q - P of a primitive quartet; QA = Q - A of its ket, which a loop over
+// bras keeps.
 struct PrimGeom {
   double PA[3], QC[3], QP[3];
 };
-__device__ __forceinline__ PrimGeom prim_geom(const PrimRegs& B, const PrimRegs& K, const QuartetGeom& g) {
+struct KetPos {
+  double QA[3];
+};
+__device__ __forceinline__ KetPos ket_pos(const PrimRegs& K, const QuartetGeom& g) {
+  return KetPos{{fma(K.z, g.Rcd[0], g.CA[0]), fma(K.z, g.Rcd[1], g.CA[1]), fma(K.z, g.Rcd[2], g.CA[2])}};
+}
+__device__ __forceinline__ PrimGeom prim_geom(const PrimRegs& B, const PrimRegs& K, const KetPos& q,
+                                              const QuartetGeom& g) {
   PrimGeom r;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     r.PA[i] = B.z * g.Rab[i];
     r.QC[i] = K.z * g.Rcd[i];
-    r.QP[i] = fma(-B.z, g.Rab[i], fma(K.z, g.Rcd[i], g.CA[i]));
+    r.QP[i] = fma(-B.z, g.Rab[i], q.QA[i]);
   }
   return r;
+}
+__device__ __forceinline__ PrimGeom prim_geom(const PrimRegs& B, const PrimRegs& K, const QuartetGeom& g) {
+  return prim_geom(B, K, ket_pos(K, g), g);
 }
 
 // 1/x and 1/sqrt(x) in FP32 (the PTX approximate instructions, about 23 correct
@@ -693,11 +727,12 @@ __device__ __forceinline__ void boys_eval(const double* __restrict__ tab, double
 
 // One primitive quartet by the vertical recurrence.
 template <int LA, int LB, int LC, int LD>
-__device__ __forceinline__ void prim_quartet_vrr(const PrimRegs& B, const PrimRegs& K, const QuartetGeom& g,
+__device__ __forceinline__ void prim_quartet_vrr(const PrimRegs& B, const PrimRegs& K, const KetPos& q,
+                                                 const QuartetGeom& g,
                                                  double (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                  const double* __restrict__ tab) {
   constexpr int L = LA + LB + LC + LD;
-  const PrimGeom p = prim_geom(B, K, g);
+  const PrimGeom p = prim_geom(B, K, q, g);
   const double zeta = B.x, eta = K.x;
   const double sq = rsqrt_nr(zeta + eta);      // 1/sqrt(zeta + eta)
   const double inv = sq * sq, r_z = eta * inv, r_e = zeta * inv;
@@ -708,6 +743,12 @@ __device__ __forceinline__ void prim_quartet_vrr(const PrimRegs& B, const PrimRe
   double S[L + 1], WP[3], WQ[3];
 #pragma unroll
   for (int m = 0; m <= L; ++m) S[m] = F[m] * scale;
+  if constexpr (L == 1) {                      // one step: r_z with S[1] instead of with Q - P
+    const double s1 = r_z * S[1];
+#pragma unroll
+    for (int i = 0; i < 3; ++i) esfs[i][0] = fma(p.QP[i], s1, fma(p.PA[i], S[0], esfs[i][0]));
+    return;
+  }
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
     WP[i] = r_z * p.QP[i];
@@ -725,12 +766,13 @@ __device__ __forceinline__ void prim_quartet_vrr(const PrimRegs& B, const PrimRe
 // an incremental build is nearly all FP32 quartets, so a different rounding shows in its
 // result, and all kernel variants of a class should give the same one.
 template <int LA, int LB, int LC, int LD>
-__device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRegs& K, const QuartetGeom& g,
+__device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRegs& K, const KetPos& q,
+                                                 const QuartetGeom& g,
                                                  float (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                  const double* __restrict__ rys_smem) {
   using Q = Quartet<LA, LB, LC, LD>;
   constexpr int D1 = Q::LAB + 1, D2 = Q::LCD + 1, NR = Q::NROOT;
-  const PrimGeom p = prim_geom(B, K, g);
+  const PrimGeom p = prim_geom(B, K, q, g);
   const float zeta = (float)B.x, eta = (float)K.x;
   const float half_zinv = (float)B.w, half_einv = (float)K.w;
   const float sq = rsqrt_f32(__fadd_rn(zeta, eta));
@@ -803,18 +845,20 @@ __device__ __forceinline__ void prim_quartet_f32(const PrimRegs& B, const PrimRe
 // One primitive quartet: Rys nodes and weights, the 2D recurrences and the
 // (e0|f0) products, added to esfs.
 template <int LA, int LB, int LC, int LD, typename T>
-__device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& K, const QuartetGeom& g, T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
+__device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& K, const KetPos& q,
+                                             const QuartetGeom& g,
+                                             T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                              const double* __restrict__ rys_smem) {
   if constexpr (use_vrr<LA, LB, LC, LD, T>()) {
-    prim_quartet_vrr<LA, LB, LC, LD>(B, K, g, esfs, rys_smem);
+    prim_quartet_vrr<LA, LB, LC, LD>(B, K, q, g, esfs, rys_smem);
     return;
   } else if constexpr (std::is_same<T, float>::value) {
-    prim_quartet_f32<LA, LB, LC, LD>(B, K, g, esfs, rys_smem);
+    prim_quartet_f32<LA, LB, LC, LD>(B, K, q, g, esfs, rys_smem);
     return;
   } else {
   using Q = Quartet<LA, LB, LC, LD>;
   constexpr int D1 = Q::LAB + 1, D2 = Q::LCD + 1, NR = Q::NROOT;
-  const PrimGeom p = prim_geom(B, K, g);
+  const PrimGeom p = prim_geom(B, K, q, g);
   const double bcc = B.y * TWOPI5ON2, kcc = K.y;
   const double zeta = B.x, half_zinv = B.w;
   const double eta = K.x, half_einv = K.w;
@@ -880,7 +924,8 @@ __device__ __forceinline__ void prim_quartet(const PrimRegs& B, const PrimRegs& 
 template <int LA, int LB, int LC, int LD, typename T>
 __device__ __forceinline__ void accumulate_esfs(const PrimPair* __restrict__ bp, int nbp,
                                                 const PrimPair* __restrict__ kp, int nkp, int p0, int npq,
-                                                const QuartetGeom& g, T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
+                                                const QuartetGeom& g,
+                                                T (&esfs)[Quartet<LA, LB, LC, LD>::NE][Quartet<LA, LB, LC, LD>::NF],
                                                 const double* __restrict__ rys_smem = nullptr) {
   using Q = Quartet<LA, LB, LC, LD>;
 #pragma unroll
@@ -889,17 +934,25 @@ __device__ __forceinline__ void accumulate_esfs(const PrimPair* __restrict__ bp,
     for (int f = 0; f < Q::NF; ++f) esfs[e][f] = T(0);
   if (npq <= 0) return;
   int ik = p0 ? p0 / nbp : 0, ib = p0 - ik * nbp;
-  PrimRegs kc = load_prim(kp, ik);
+  // (the one-root classes, at 20 resident warps, have no registers for it)
+  constexpr bool KEEP = Q::LAB + Q::LCD >= 2;
+  PrimRegs k = load_prim(kp, ik);
+  KetPos q = ket_pos(k, g);
 #pragma unroll(kPrimUnroll)
   for (int p = 0; p < npq; ++p) {
     const PrimRegs b = load_prim(bp, ib);
-    const PrimRegs k = kc;
-    if (++ib == nbp) {
+    const bool last = ++ib == nbp;             // the ket's last bra: its successor is loaded meanwhile
+    PrimRegs kc = k;
+    if (last) {
       ib = 0;
       ++ik;
       if (ik < nkp) kc = load_prim(kp, ik);
     }
-    prim_quartet<LA, LB, LC, LD, T>(b, k, g, esfs, rys_smem);
+    prim_quartet<LA, LB, LC, LD, T>(b, k, KEEP ? q : ket_pos(k, g), g, esfs, rys_smem);
+    if (last) {
+      k = kc;
+      if (KEEP) q = ket_pos(k, g);
+    }
   }
 }
 
@@ -1025,15 +1078,19 @@ __device__ __forceinline__ void accumulate_esfs_fam(const PrimPair* __restrict__
       for (int f = 0; f < Q::NF; ++f) esfs[m][e][f] = T(0);
   if (npq <= 0) return;
   int ik = p0 ? p0 / nbp : 0, ib = p0 - ik * nbp;
-  PrimRegs kc = load_prim(kp, ik);
+  // (the one-root classes, at 20 resident warps, have no registers for it)
+  constexpr bool KEEP = Q::LAB + Q::LCD >= 2;
+  PrimRegs k = load_prim(kp, ik);
+  KetPos q = ket_pos(k, g);
   for (int p = 0; p < npq; ++p) {
     PrimRegs b = load_prim(bp, ib);
     double cb[MB];
 #pragma unroll
     for (int m = 0; m < MB; ++m) cb[m] = bm[m] ? __ldg(&bm[m][ib].cc) : 0.0;
     b.y = 1.0;
-    const PrimRegs k = kc;
-    if (++ib == nbp) {
+    const bool last = ++ib == nbp;
+    PrimRegs kc = k;
+    if (last) {
       ib = 0;
       ++ik;
       if (ik < nkp) kc = load_prim(kp, ik);
@@ -1043,7 +1100,11 @@ __device__ __forceinline__ void accumulate_esfs_fam(const PrimPair* __restrict__
     for (int e = 0; e < Q::NE; ++e)
 #pragma unroll
       for (int f = 0; f < Q::NF; ++f) one[e][f] = T(0);
-    prim_quartet<LA, LB, LC, LD, T>(b, k, g, one, rys_smem);
+    prim_quartet<LA, LB, LC, LD, T>(b, k, KEEP ? q : ket_pos(k, g), g, one, rys_smem);
+    if (last) {
+      k = kc;
+      if (KEEP) q = ket_pos(k, g);
+    }
 #pragma unroll
     for (int m = 0; m < MB; ++m) {
       const T w = T(cb[m]);

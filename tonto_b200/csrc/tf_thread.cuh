@@ -133,6 +133,38 @@ __device__ __forceinline__ void load_block(const double* __restrict__ P, int n, 
   }
 }
 
+// Sums of N <= 32 values over the warp: at each of the five steps a lane keeps half of its
+// values and gets its partner's sums of those, so that about N + 5 exchanges do the work of
+// 5 N.  On return v[0] is the warp's sum of value e, the returned index (N or more: none).
+template <int N>
+__device__ __forceinline__ int warp_sums(double (&v)[N]) {
+  static_assert(N >= 1 && N <= 32, "at most a value per lane");
+  const int lane = threadIdx.x & 31;
+  int e = 0;
+  static_for<5>([&](auto ss) {
+    constexpr int st = decltype(ss)::value, o = 16 >> st;
+    constexpr int P2 = N <= 1 ? 1 : N <= 2 ? 2 : N <= 4 ? 4 : N <= 8 ? 8 : N <= 16 ? 16 : 32;
+    constexpr int held = (P2 >> st) > 1 ? (P2 >> st) : 1;
+    constexpr int valid = held < N ? held : N;               // held values that exist in some lane
+    const bool up = lane & o;
+    if constexpr (held > 1) {
+      constexpr int h = held / 2;
+#pragma unroll
+      for (int i = 0; i < h; ++i) {
+        const double lo = i < valid ? v[i] : 0.0, hi = i + h < valid ? v[i + h < N ? i + h : 0] : 0.0;
+        const double got = __shfl_xor_sync(0xffffffffu, up ? lo : hi, o);
+        if (i < N) v[i] = (up ? hi : lo) + got;
+      }
+      if (up) e += h;
+    } else {
+      v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+    }
+  });
+  // lanes that took part in the last, unsplit steps hold the same sum: one of them adds it
+  constexpr int P2 = N <= 1 ? 1 : N <= 2 ? 2 : N <= 4 ? 4 : N <= 8 ? 8 : N <= 16 ? 16 : 32;
+  return (lane & (32 / P2 - 1)) == 0 ? e : 32;
+}
+
 // Digestion of one quartet's Cartesian integrals I into J and K with the coincidence
 // factor f (f = 0: the lane adds nothing but still takes part in the warp sums):
 // bid is the bra pair (lanes of one bra are summed together), ob/oa the bra's and
@@ -169,6 +201,7 @@ __device__ __forceinline__ void digest_jk(const JKArgs& a, const MolInfo& mi,
   auto digest_j = [&](const double* __restrict__ P, double* __restrict__ Jm) {
     double Pcd[Q::NC][Q::ND];
     load_block<Q::NC, Q::ND>(P, n, oc, od, Pcd);
+    double Jab[Q::NA * Q::NB];
 #pragma unroll
     for (int ia = 0; ia < Q::NA; ++ia)
 #pragma unroll
@@ -178,20 +211,29 @@ __device__ __forceinline__ void digest_jk(const JKArgs& a, const MolInfo& mi,
         for (int c = 0; c < Q::NC; ++c)
 #pragma unroll
           for (int d = 0; d < Q::ND; ++d) s += I[ia][ib][c * Q::ND + d] * Pcd[c][d];
-        s *= f;
-        if (uni) {
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-          if (lane == 0 && s != 0.0) fock_add<FX>(Jm + (size_t)(oa + ia) * n + ob + ib, s, a.fx_lo);
-        } else {                       // idle lanes join the last run with s = 0
-#pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const double t = __shfl_up_sync(0xffffffffu, s, o);
-            if (lane - o >= sega) s += t;
-          }
-          if (taila && s != 0.0) fock_add<FX>(Jm + (size_t)(oa + ia) * n + ob + ib, s, a.fx_lo);
-        }
+        Jab[ia * Q::NB + ib] = s * f;
       }
+    if (uni) {
+      static_for<(Q::NA * Q::NB + 31) / 32>([&](auto cc) {
+        constexpr int e0 = 32 * decltype(cc)::value, m = Q::NA * Q::NB - e0 < 32 ? Q::NA * Q::NB - e0 : 32;
+        double v[m];
+#pragma unroll
+        for (int i = 0; i < m; ++i) v[i] = Jab[e0 + i];
+        const int i = warp_sums<m>(v), e = e0 + i;
+        if (i < m && v[0] != 0.0) fock_add<FX>(Jm + (size_t)(oa + e / Q::NB) * n + ob + e % Q::NB, v[0], a.fx_lo);
+      });
+    } else {                           // idle lanes join the last run with s = 0
+#pragma unroll
+      for (int e = 0; e < Q::NA * Q::NB; ++e) {
+        double s = Jab[e];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const double t = __shfl_up_sync(0xffffffffu, s, o);
+          if (lane - o >= sega) s += t;
+        }
+        if (taila && s != 0.0) fock_add<FX>(Jm + (size_t)(oa + e / Q::NB) * n + ob + e % Q::NB, s, a.fx_lo);
+      }
+    }
     if (live) {
       double Pab[Q::NA][Q::NB];
       load_block<Q::NA, Q::NB>(P, n, oa, ob, Pab);
