@@ -21,7 +21,8 @@
 #include <utility>
 #include <type_traits>
 
-#define TF_RYS_CONST __device__ const
+// (32-byte aligned: a polynomial's twelve coefficients are three 32-byte loads)
+#define TF_RYS_CONST __device__ const __align__(32)
 // the asymptotic-rule tables in the constant bank: read at compile-time indices,
 // they become immediate operands instead of global loads
 #define TF_RYS_SMALL_CONST __constant__ const

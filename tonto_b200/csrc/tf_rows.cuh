@@ -49,6 +49,8 @@ struct RowArgs {
   int want;                     // bit 0 J, bit 1 K
   unsigned long long* qcount;   // quartets counted per class (the launch's FP64 or FP32 half)
   long long fx_lo;              // deterministic builds: offset of the lo words (fock_add), else 0
+  long long groups;             // lane groups of the full grid (see k_jk_rows)
+  long long expect;             // entries the launch will probably have (chooses the instantiation)
 };
 
 template <int LA, int LB, int LC, int LD>
@@ -59,15 +61,17 @@ struct RowCfg {
   static constexpr int GW = (Q::NF + 31) / 32;           // warps per quartet
   static constexpr int G = GW == 1 ? Q::NF : 32 * GW;    // lanes per quartet
   static constexpr int QPW = GW == 1 ? 32 / G : 1;       // quartets per warp (GW > 1: per block)
-  static constexpr int D1P = (D1 + 1) & ~1;              // a table column, whole 16-byte words
-  static constexpr int T2D = 3 * NR * D2 * D1P;
+  // a 2D table's column and the table itself, odd: lanes that read several columns or write
+  // several tables hit different banks (as do a warp's groups, per_group)
+  static constexpr int CS = D1 | 1, TS = (CS * D2) | 1;
+  static constexpr int T2D = 3 * NR * TS;
   // row stride (odd: rows on different banks): the row, or in its place the row's K shares
   __host__ __device__ static constexpr int rs(int ns) { return cmax(Q::NF, 2 * NY * ns) | 1; }
   static constexpr int YS = NY | 1;
-  __host__ __device__ static constexpr int area(int ns) { return (cmax(T2D, NAB * rs(ns)) + 1) & ~1; }
+  __host__ __device__ static constexpr int area(int ns) { return cmax(T2D, NAB * rs(ns)); }
   // per density: P(a|b, c|d), P(ab), P(cd), J~
   static constexpr int STAGE = NX * YS + NAB + NCD + Q::NF;
-  __host__ __device__ static constexpr int per_group(int ns) { return area(ns) + ((ns * STAGE + 1) & ~1); }
+  __host__ __device__ static constexpr int per_group(int ns) { return (area(ns) + ns * STAGE) | 1; }
 };
 
 struct CompBytes {
@@ -137,6 +141,7 @@ __device__ __forceinline__ double bra_value(const double (&es)[NE], const double
 // first lane.
 template <int N, int G>
 __device__ __forceinline__ void group_rys(double x, int gl, int gbase, double (&u)[N], double (&w)[N]) {
+  static_assert(TF_RYS_NCOEF == 12 && rys_offset(N) % 4 == 0, "three 32-byte words a polynomial");
   constexpr int NF2 = 2 * N, PER = (NF2 + G - 1) / G;
   constexpr int XMAX = rys_xmax(N), OFF = rys_offset(N), HOFF = rys_hoffset(N);
   const bool tab = x < (double)XMAX;
@@ -149,9 +154,10 @@ __device__ __forceinline__ void group_rys(double x, int gl, int gbase, double (&
     double v = 0.0;
     if (tab && f < NF2) {
       const double* cf = tf_rys_coef + OFF + j * (NF2 * TF_RYS_NCOEF) + f * TF_RYS_NCOEF;
-      v = __ldg(cf + TF_RYS_DEG);
-#pragma unroll
-      for (int k = TF_RYS_DEG - 1; k >= 0; --k) v = fma(v, s, __ldg(cf + k));
+      const double4 c2 = ldg256(cf + 8), c1 = ldg256(cf + 4), c0 = ldg256(cf);
+      v = fma(fma(fma(c2.w, s, c2.z), s, c2.y), s, c2.x);
+      v = fma(fma(fma(fma(v, s, c1.w), s, c1.z), s, c1.y), s, c1.x);
+      v = fma(fma(fma(fma(v, s, c0.w), s, c0.z), s, c0.y), s, c0.x);
     }
     val[q] = v;
   }
@@ -176,15 +182,20 @@ __device__ __forceinline__ void fock_add_rt(double* addr, double v, long long fx
   else fock_add<false>(addr, v, 0);
 }
 
-template <int LA, int LB, int LC, int LD, int WPB>
+// SHARED: a list with fewer quartets than the GPU has lane groups; several groups of a warp
+// share a quartet.  Each takes every share-th primitive quartet, their (e0|f0) columns are
+// summed by shuffles, the first group transfers them and all lanes take rows: (H2O)2 STO-3G's
+// 81-primitive (pp|pp) quartets 66 -> 28 us, (H2O)2 cc-pVTZ (ff|ps) 93 -> 44.  An instantiation of
+// its own: with run-time lane counts (H2O)32's (pp|pp) took 2.97 instead of 2.55 ms.
+template <int LA, int LB, int LC, int LD, int WPB, bool SHARED>
 __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
   using C = RowCfg<LA, LB, LC, LD>;
   using Q = typename C::Q;
-  constexpr int G = C::G, GW = C::GW, QPW = C::QPW, NR = C::NR, D1 = C::D1, D2 = C::D2, D1P = C::D1P;
+  constexpr int G = C::G, GW = C::GW, QPW = C::QPW, NR = C::NR, D1 = C::D1, D2 = C::D2;
   constexpr int NE = Q::NE, NF = Q::NF, NA = Q::NA, NB = Q::NB, NC = Q::NC, ND = Q::ND;
   constexpr int NAB = C::NAB, NCD = C::NCD, NY = C::NY, NX = C::NX, YS = C::YS;
   static_assert(GW == 1 || GW == WPB, "a quartet wider than a warp takes a block");
-  extern __shared__ __align__(16) double smem[];
+  extern __shared__ double smem[];
   const int ns = a.P2 ? 2 : 1;
   const int rs = C::rs(ns);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -197,21 +208,31 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
   const bool in_group = GW > 1 || gq < QPW;
   const int gl = GW > 1 ? (int)threadIdx.x : (in_group ? lane - gq * G : 0x40000000);
   const int slot = GW > 1 ? 0 : warp * QPW + (in_group ? gq : 0);
-  double* const T2 = smem + (size_t)slot * C::per_group(ns);      // 2D tables, then the rows
-  double* const X = T2;
-  double* const stage = T2 + C::area(ns);
+  double* const T2 = smem + (size_t)slot * C::per_group(ns);      // the group's 2D tables
   const bool has_f = in_group && gl < NF;
-  const int gf = Q::FF + (has_f ? gl : 0);
-  const int fx = g_comp_bytes.x[gf], fy = g_comp_bytes.y[gf], fz = g_comp_bytes.z[gf];
-  const long long nslots = GW > 1 ? gridDim.x : (long long)gridDim.x * WPB;   // warps or blocks at work
-  unsigned long long nprim = 0, nquart = 0;
   const int2* quartets = a.quartets;
   long long nq = a.n;
   resolve_range(a.range, a.base, a.cap, quartets, nq);
-  for (long long base = (GW > 1 ? (long long)blockIdx.x : (long long)blockIdx.x * WPB + warp) * QPW; base < nq;
-       base += nslots * QPW) {
-    const long long t = base + (in_group ? gq : 0);
-    const bool act = in_group && t < nq;
+  if (nq <= 0) return;
+  // (from the list length and the full grid alone, so that a deterministic build does not
+  // depend on the launch)
+  const int share = SHARED ? (int)max(1LL, min((long long)QPW, a.groups / nq)) : 1;
+  const int per_warp = QPW / share;                    // quartets of a warp at a time
+  const int qs = in_group ? gq / share : 0, member = in_group ? gq - qs * share : 0;
+  const bool used = in_group && qs < per_warp;
+  const int ql = used ? member * G + gl : 0x40000000;  // lane within the quartet, and its lanes
+  const int QL = share * G;
+  const int gf = Q::FF + (has_f ? gl : 0);
+  const int fx = g_comp_bytes.x[gf], fy = g_comp_bytes.y[gf], fz = g_comp_bytes.z[gf];
+  const long long nslots = GW > 1 ? gridDim.x : (long long)gridDim.x * WPB;   // warps or blocks at work
+  // the quartet's rows and density blocks, in its first group's area
+  double* const X = smem + (size_t)(slot - member) * C::per_group(ns);
+  double* const stage = X + C::area(ns);
+  unsigned long long nprim = 0, nquart = 0;
+  for (long long base = (GW > 1 ? (long long)blockIdx.x : (long long)blockIdx.x * WPB + warp) * per_warp; base < nq;
+       base += nslots * per_warp) {
+    const long long t = base + qs;
+    const bool act = used && t < nq;
     const int2 qd = act ? quartets[t] : make_int2(0, 0);
     const PairJK b = load_pair_jk(a.jkrec, a.xyz4, qd.x);
     const PairJK k = load_pair_jk(a.jkrec, a.xyz4, qd.y);
@@ -222,7 +243,7 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
     const int nbp = any_same ? b.n_full : b.n_skip;
     const int nkp = any_same ? k.n_full : k.n_skip;
     const int npq = act ? nbp * nkp : 0;
-    if (act && gl == 0) { nprim += (unsigned long long)npq; nquart += 1; }
+    if (act && ql == 0) { nprim += (unsigned long long)npq; nquart += 1; }
     const MolInfo mi = a.mols[act ? b.mol : 0];
     const int n = mi.n_cart;
     const int oa = b.cart_hi, ob = b.cart_lo, oc = k.cart_hi, od = k.cart_lo;
@@ -231,24 +252,27 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
       for (int s = 0; s < ns; ++s) {
         const double* __restrict__ P = (s ? a.P2 : a.P) + mi.cmat;
         double* st = stage + s * C::STAGE;
-        for (int e = gl; e < NX * NY; e += G) {
+        for (int e = ql; e < NX * NY; e += QL) {
           const int x = e / NY, y = e - x * NY;
           const int row = x < NA ? oa + x : ob + x - NA, col = y < NC ? oc + y : od + y - NC;
           st[x * YS + y] = __ldg(P + (size_t)row * n + col);
         }
-        for (int e = gl; e < NAB; e += G) st[NX * YS + e] = __ldg(P + (size_t)(oa + e / NB) * n + ob + e % NB);
-        for (int e = gl; e < NCD; e += G)
+        for (int e = ql; e < NAB; e += QL) st[NX * YS + e] = __ldg(P + (size_t)(oa + e / NB) * n + ob + e % NB);
+        for (int e = ql; e < NCD; e += QL)
           st[NX * YS + NAB + e] = __ldg(P + (size_t)(oc + e / ND) * n + od + e % ND);
       }
     }
-    const int maxnpq = GW > 1 ? npq : (int)__reduce_max_sync(0xffffffffu, npq);
+    const int mine = npq > member ? (npq - member + share - 1) / share : 0;   // this group's primitive quartets
+    const int maxnpq = GW > 1 ? npq : (int)__reduce_max_sync(0xffffffffu, mine);
     const QuartetGeom geom = quartet_geom(b, k);
     double es[NE];
 #pragma unroll
     for (int e = 0; e < NE; ++e) es[e] = 0.0;
-    int ib = 0, ik = 0;
+    int ib = 0, ik = member;
     for (int p = 0; p < maxnpq; ++p) {
-      const bool v = p < npq;
+      const bool v = p < mine;
+      if constexpr (SHARED)
+        while (v && ik >= nkp) { ik -= nkp; ++ib; }
       double u[NR], w[NR];
       double4 b0 = make_double4(1, 0, 0, 0), k0 = make_double4(1, 0, 0, 0);
       double inv = 0.0, r_z = 0.0, r_e = 0.0, scale = 0.0, xx = 0.0;
@@ -282,7 +306,7 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
           const double t2_rz = t2 * r_z, t2_re = t2 * r_e;
           const double B10 = (1.0 - t2_rz) * b0.w, B01 = (1.0 - t2_re) * k0.w, B00 = 0.5 * t2 * inv;
           const double c00 = PA + t2_rz * QPd, d00 = QC - t2_re * QPd;
-          double* out = T2 + task * (D2 * D1P);
+          double* out = T2 + task * C::TS;
           // one ket column at a time: I[e][f + 1] from columns f and f - 1
           double I0[D1], I1[D1];
           I0[0] = d == 2 ? wr * scale : 1.0;
@@ -305,7 +329,7 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
             for (int e = 0; e < D1; ++e) {
               I1[e] = I0[e];
               I0[e] = nx[e];
-              out[(f + 1) * D1P + e] = nx[e];
+              out[(f + 1) * C::CS + e] = nx[e];
             }
           }
         }
@@ -314,16 +338,17 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
       if (v && has_f) {
 #pragma unroll
         for (int r = 0; r < NR; ++r) {
-          double cxv[D1P], cyv[D1P], czv[D1P];
-          const double2* tx = reinterpret_cast<const double2*>(T2 + ((0 * NR + r) * D2 + fx) * D1P);
-          const double2* ty = reinterpret_cast<const double2*>(T2 + ((1 * NR + r) * D2 + fy) * D1P);
-          const double2* tz = reinterpret_cast<const double2*>(T2 + ((2 * NR + r) * D2 + fz) * D1P);
+          // (8-byte loads: lanes that share a word are served together, half a warp at a
+          // time; 16-byte ones a quarter warp at a time, measured 2-4 cycles against 0.6-1.3)
+          double cxv[D1], cyv[D1], czv[D1];
+          const double* tx = T2 + (0 * NR + r) * C::TS + fx * C::CS;
+          const double* ty = T2 + (1 * NR + r) * C::TS + fy * C::CS;
+          const double* tz = T2 + (2 * NR + r) * C::TS + fz * C::CS;
 #pragma unroll
-          for (int e = 0; e < D1P / 2; ++e) {
-            const double2 vx = tx[e], vy = ty[e], vz = tz[e];
-            cxv[2 * e] = vx.x; cxv[2 * e + 1] = vx.y;
-            cyv[2 * e] = vy.x; cyv[2 * e + 1] = vy.y;
-            czv[2 * e] = vz.x; czv[2 * e + 1] = vz.y;
+          for (int e = 0; e < D1; ++e) {
+            cxv[e] = tx[e];
+            cyv[e] = ty[e];
+            czv[e] = tz[e];
           }
           static_for<NE>([&](auto ee) {
             constexpr int e = decltype(ee)::value;
@@ -332,12 +357,24 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
           });
         }
       }
-      if (++ik == nkp) { ik = 0; ++ib; }
+      if constexpr (SHARED) ik += share;
+      else if (++ik == nkp) { ik = 0; ++ib; }
     }
     group_sync();                                // the tables have been read, the density blocks written
+    if constexpr (SHARED) {                      // the sharing groups' sums, halving
+      for (int o = share; o > 1; o = (o + 1) / 2) {
+        const int h = (o + 1) / 2;
+        const bool add = used && member + h < o;
+#pragma unroll
+        for (int e = 0; e < NE; ++e) {
+          const double x = __shfl_sync(0xffffffffu, es[e], (lane + h * G) & 31);
+          if (add) es[e] += x;
+        }
+      }
+    }
     const double (&Rab)[3] = geom.Rab;
     const double (&Rcd)[3] = geom.Rcd;
-    if (act && has_f) {                          // column f: bra transfer, J~(f)
+    if (act && has_f && member == 0) {           // column f: bra transfer, J~(f)
       double jt = 0.0, jt2 = 0.0;
       const double* pab = stage + NX * YS;
       static_for<NA>([&](auto aa) {
@@ -359,7 +396,7 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
     if (k.same) f *= 0.5;
     if (qd.x == qd.y) f *= 0.5;
     if (act) {
-      for (int r = gl; r < NAB; r += G) {        // row ab: ket transfer, J(ab), the row's shares of K
+      for (int r = ql; r < NAB; r += QL) {        // row ab: ket transfer, J(ab), the row's shares of K
         const int ia = r / NB, ibb = r - ia * NB;
         double* row = X + r * rs;
         double g[1][NF], I[1][NC][ND];
@@ -416,7 +453,7 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
         for (int s = 0; s < ns; ++s) {
           const double* jt = stage + s * C::STAGE + NX * YS + NAB + NCD;
           double* Jm = (s ? a.J2 : a.J) + mi.cmat;
-          for (int cd = gl; cd < NCD; cd += G) {
+          for (int cd = ql; cd < NCD; cd += QL) {
             const int c = cd / ND, d = cd - c * ND;
             double sum = 0.0;
 #pragma unroll
@@ -440,7 +477,7 @@ __global__ void __launch_bounds__(32 * WPB) k_jk_rows(RowArgs a) {
       for (int s = 0; s < ns; ++s) {
         double* Km = (s ? a.K2 : a.K) + mi.cmat;
         const double* part = X + 2 * NY * s;
-        for (int e = gl; e < NX * NY; e += G) {
+        for (int e = ql; e < NX * NY; e += QL) {
           const int x = e / NY, y = e - x * NY;
           double sum = 0.0;
           if (x < NA) {
@@ -488,14 +525,18 @@ static bool launch_rows_t(const RowArgs& a, cudaStream_t s) {
   constexpr int WPB = rows_wpb<LA, LB, LC, LD>();
   constexpr int QPB = C::GW > 1 ? 1 : C::QPW * WPB;
   const size_t smem = (size_t)QPB * C::per_group(a.P2 ? 2 : 1) * sizeof(double);
+  constexpr bool CAN_SHARE = C::QPW > 1;
   static int per_sm[2] = {-1, -1};            // restricted, unrestricted
   if (per_sm[1] < 0) {
-    if (cudaFuncSetAttribute(k_jk_rows<LA, LB, LC, LD, WPB>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)(QPB * C::per_group(2) * sizeof(double))) != cudaSuccess)
+    const int top = (int)(QPB * C::per_group(2) * sizeof(double));
+    if (cudaFuncSetAttribute(k_jk_rows<LA, LB, LC, LD, WPB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, top) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(k_jk_rows<LA, LB, LC, LD, WPB, CAN_SHARE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             top) != cudaSuccess)
       return false;
     for (int u = 0; u < 2; ++u) {
       int nb = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_jk_rows<LA, LB, LC, LD, WPB>, 32 * WPB,
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_jk_rows<LA, LB, LC, LD, WPB, false>, 32 * WPB,
                                                     (size_t)QPB * C::per_group(1 + u) * sizeof(double));
       per_sm[u] = nb < 1 ? 1 : nb;
     }
@@ -504,9 +545,16 @@ static bool launch_rows_t(const RowArgs& a, cudaStream_t s) {
   int dev = 0, nsm = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const long long full = (long long)nsm * per_sm[a.P2 ? 1 : 0], need = (a.n + QPB - 1) / QPB;
+  RowArgs r = a;
+  const long long full = (long long)nsm * per_sm[a.P2 ? 1 : 0];
+  r.groups = full * QPB;
+  // sharing groups where the list is expected to leave half of them idle; always in a
+  // deterministic build, whose sums must not depend on an expectation
+  const bool shared = CAN_SHARE && (a.fx_lo || 2 * a.expect <= r.groups);
+  const long long per_block = shared ? WPB : QPB, need = (a.n + per_block - 1) / per_block;
   const long long blocks = a.range || need > full ? full : need;
-  k_jk_rows<LA, LB, LC, LD, WPB><<<(unsigned)blocks, 32 * WPB, smem, s>>>(a);
+  if (shared) k_jk_rows<LA, LB, LC, LD, WPB, CAN_SHARE><<<(unsigned)blocks, 32 * WPB, smem, s>>>(r);
+  else k_jk_rows<LA, LB, LC, LD, WPB, false><<<(unsigned)blocks, 32 * WPB, smem, s>>>(r);
   return true;
 }
 

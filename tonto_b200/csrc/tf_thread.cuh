@@ -64,6 +64,7 @@ struct JKArgs {
   int fam;                      // bra-family capacity of the launch's kernel (1: none)
   int bucket32;                 // 1: the launch covers the FP32 buckets
   long long fx_lo;              // deterministic builds: offset of the lo words (fock_add), else 0
+  long long expect;             // entries the launch will probably have (the lane-group kernels' choice)
 };
 
 

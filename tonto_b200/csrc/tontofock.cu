@@ -1941,7 +1941,7 @@ static int dispatch_jk(int la, int lb, int lc, int ld, const JKArgs& a, cudaStre
     return TF_OK;
   const RowArgs r{a.quartets + (a.range ? 0 : a.first - a.base), a.n, a.prim_full, a.prim_skip, a.P, a.J, a.K, a.mols, a.prim_count, a.range, a.base,
                   a.cap, a.jkrec, a.xyz4, a.P2, a.J2, a.K2, a.want,
-                  a.qcount ? a.qcount + (a.bucket32 ? NQCLS : 0) : nullptr, a.fx_lo};
+                  a.qcount ? a.qcount + (a.bucket32 ? NQCLS : 0) : nullptr, a.fx_lo, 0, a.expect};
   for (auto* launch : {launch_rows_d, launch_rows_fs, launch_rows_fd, launch_rows_ff}) {
     const int rc = launch(key, r, s);
     if (rc > 0) return TF_OK;
@@ -2179,6 +2179,9 @@ static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* d
     a32.plan = c->d_plans.p + 2 * g + 1;
     a32.range = c->d_group_offsets.p + 3 * g + 1;
     a32.bucket32 = 1;
+    const int cid = qclass_id(l1h, l1l, l2h, l2l);           // the last build's counts
+    a.expect = (long long)c->pin->pc[NQCLS + 1 + cid];
+    a32.expect = (long long)c->pin->pc[2 * NQCLS + 1 + cid];
     rc = dispatch_jk(l1h, l1l, l2h, l2l, a, sg, false, jk_variant(c, g));
     if (rc != TF_OK) return rc;
     kernels++;
@@ -2429,6 +2432,8 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
       a32.first = goff[3 * g + 1];
       a32.n = goff[3 * g + 2] - goff[3 * g + 1];
       a32.bucket32 = 1;
+      a.expect = a.n;
+      a32.expect = a32.n;
       if (a.n > 0) {
         rc = dispatch_jk(l1h, l1l, l2h, l2l, a, sg, false, jk_variant(c, g));
         if (rc != TF_OK) return rc;
