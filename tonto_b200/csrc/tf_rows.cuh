@@ -18,10 +18,10 @@
 // layout reads every integral from shared memory once (the row read), where transfers and
 // digestion element by element in shared memory read each about ten times.  Measured,
 // class-by-class builds, against that form of the kernels: (H2O)32 cc-pVDZ (dp|dp) 1.22 ->
-// 0.82 ms, (dd|pp) 1.26 -> 0.56, (dd|dp) 1.01 -> 0.29, (pp|pp) 3.77 -> 3.28, (dp|pp) 3.44 ->
-// 2.84, (dd|ps) 1.61 -> 1.81, (dp|ds) unchanged at 2.25.  For the f classes, against one warp
-// a quartet with run-time angular momenta in global scratch: (H2O)5 cc-pVTZ (fd|dp) 3.26 ->
-// 0.14 ms, (fp|ps) 5.07 -> 0.42, (ff|ff) 1.08 -> 0.06, the whole build 85 -> 8.5 ms.
+// 0.72 ms, (dd|pp) 1.26 -> 0.56, (dd|dp) 1.01 -> 0.28, (dp|pp) 3.44 -> 2.77.  For the f classes,
+// against one warp a quartet with run-time angular momenta in global scratch: (H2O)5 cc-pVTZ
+// (fd|dp) 3.26 -> 0.14 ms, (ff|ff) 1.08 -> 0.02.  The classes of tf_jk_l*.cu come here with
+// short lists only (dispatch_jk has both sides' times).
 #pragma once
 #include "tf_device.cuh"
 

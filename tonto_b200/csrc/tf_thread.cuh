@@ -544,9 +544,9 @@ static void launch_jk(const JKArgs& a, cudaStream_t s, bool fp32, int variant) {
   launch_jk_m<LA, LB, LC, LD, 1>(a, s, fp32, variant);
 }
 
-// Classes with an f shell: FP64 for the FP32 buckets too, and the two instantiations that
-// differ in their results' bits only (deterministic or not): their launches are too small
-// a share of a build for the register-bounded variants to matter.
+// Classes whose (e0|f0) block and integrals do not fit a thread's registers: FP64 for the
+// FP32 buckets too, and the two instantiations that differ in their results' bits only
+// (deterministic or not; a register-bounded variant would spill more).
 template <int LA, int LB, int LC, int LD>
 static void launch_jk_f64(const JKArgs& a, cudaStream_t s, bool, int variant) {
   if (variant & 4) launch_jk_t<LA, LB, LC, LD, double, 6, 1>(a, s);
@@ -557,6 +557,8 @@ static void launch_jk_f64(const JKArgs& a, cudaStream_t s, bool, int variant) {
 bool launch_jk_ss(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
 bool launch_jk_ps(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
 bool launch_jk_d(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+bool launch_jk_l(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+bool launch_jk_l2(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
 bool launch_jk_f(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
 
 }  // namespace tf

@@ -1939,6 +1939,23 @@ static int dispatch_jk(int la, int lb, int lc, int ld, const JKArgs& a, cudaStre
   if (launch_jk_ss(key, a, s, fp32, variant) || launch_jk_ps(key, a, s, fp32, variant) ||
       launch_jk_d(key, a, s, fp32, variant) || launch_jk_f(key, a, s, fp32, variant))
     return TF_OK;
+  // Both kinds of kernel exist for the classes of up to a hundred elements (e0|f0) and for the
+  // ps kets (three lanes to a lane group).  One thread a quartet, spilling to L1, issues a third
+  // of the lane groups' instructions, but its quartet takes 30 to 120 us however few there
+  // are, where groups that share one take 15 to 45.  Measured, thread and rows in ms at n
+  // quartets: (pp|pp) 0.035 / 0.029 at 202, 0.037 / 0.048 at 2454, 1.23 / 2.61 at 2.8 M; (dd|ps)
+  // 0.041 / 0.015 at 605, 0.051 / 0.072 at 7251, 0.62 / 1.78 at 0.9 M; (ff|ps) 0.119 / 0.043 at 812,
+  // 0.170 / 0.213 at 13970; (fp|ps) 0.150 / 0.394 at 177 k.  Larger blocks never gain: (dp|pp) 3.00
+  // / 2.77 at 3.4 M, (fp|ds) 0.29 / 0.26, (fs|dp) 0.33 / 0.22, (dp|dp) 2.36 / 0.72.  Alone the two
+  // cross at one to two thousand; in overlapped branches later, as a short list's launch takes
+  // fewer warps from its neighbours: (H2O)2 cc-pVTZ, lists of 700 to 17000, 0.90 ms with the line
+  // at 1500, 0.86 at 7000, 0.85 at 8192; (H2O)6 6-31G(d) unrestricted 0.745, 0.743, 0.745, and 0.757
+  // at 30000.  A deterministic build's bits must not depend on an expectation: always the
+  // thread kernels.
+  constexpr long long ROWS_BELOW = 8192;
+  if ((a.fx_lo || a.expect >= ROWS_BELOW) &&
+      (launch_jk_l(key, a, s, fp32, variant) || launch_jk_l2(key, a, s, fp32, variant)))
+    return TF_OK;
   const RowArgs r{a.quartets + (a.range ? 0 : a.first - a.base), a.n, a.prim_full, a.prim_skip, a.P, a.J, a.K, a.mols, a.prim_count, a.range, a.base,
                   a.cap, a.jkrec, a.xyz4, a.P2, a.J2, a.K2, a.want,
                   a.qcount ? a.qcount + (a.bucket32 ? NQCLS : 0) : nullptr, a.fx_lo, 0, a.expect};
@@ -2303,8 +2320,9 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
         class_l(c->group_cls[g].y, l2h, l2l);
         JKArgs none{};
         none.fam = c->group_fam[g];
-        for (int fp32 = 0; fp32 < 2; ++fp32) {
-          const int rc = dispatch_jk(l1h, l1l, l2h, l2l, none, s, fp32 != 0, jk_variant(c, g));
+        for (int i = 0; i < 4; ++i) {         // FP64 and FP32, a short and a long list expected
+          none.expect = i & 2 ? LLONG_MAX / 4 : 0;
+          const int rc = dispatch_jk(l1h, l1l, l2h, l2l, none, s, i & 1, jk_variant(c, g));
           if (rc != TF_OK) return rc;
         }
       }
