@@ -2320,9 +2320,12 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
         class_l(c->group_cls[g].y, l2h, l2l);
         JKArgs none{};
         none.fam = c->group_fam[g];
-        for (int i = 0; i < 4; ++i) {         // FP64 and FP32, a short and a long list expected
-          none.expect = i & 2 ? LLONG_MAX / 4 : 0;
-          const int rc = dispatch_jk(l1h, l1l, l2h, l2l, none, s, i & 1, jk_variant(c, g));
+        none.fx_lo = fx_offset(c);
+        if (c->group_task0[g + 1] == c->group_task0[g]) continue;
+        const int cid = qclass_id(l1h, l1l, l2h, l2l);
+        for (int fp32 = 0; fp32 <= (mixed ? 1 : 0); ++fp32) {   // the kernels the capture will launch, as
+          none.expect = (long long)c->pin->pc[(1 + fp32) * NQCLS + 1 + cid];   // each costs a first load
+          const int rc = dispatch_jk(l1h, l1l, l2h, l2l, none, s, fp32 != 0, jk_variant(c, g));
           if (rc != TF_OK) return rc;
         }
       }
