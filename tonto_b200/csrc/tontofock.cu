@@ -1244,6 +1244,15 @@ static int join_branches(tf_ctx* c, int ns) {
   return TF_OK;
 }
 
+// Host-to-device copy on the context's stream.  (A plain cudaMemcpy from pageable memory may
+// return before its transfer has landed, and the context's non-blocking streams do not wait
+// for the legacy stream it runs on.)  Pageable sources are read when this returns; src must
+// stay valid until the next synchronisation of the stream where the caller may have pinned it.
+template <typename T>
+static cudaError_t upload(tf_ctx* c, T* dst, const T* src, size_t n) {
+  return cudaMemcpyAsync(dst, src, n * sizeof(T), cudaMemcpyHostToDevice, c->stream);
+}
+
 static BatchArgs batch_args(tf_ctx* c) {
   return BatchArgs{c->d_mols.p,       c->n_mol,          c->d_cmat_off.p,     c->d_bmat_off.p,
                    c->d_pmax_off.p,   c->d_cart_shell.p, c->d_cart_local.p,   c->d_bf_shell.p,
@@ -1855,12 +1864,12 @@ static int setup_pairs(tf_ctx* c) {
   const std::vector<double>& simax = c->lists.simax;
   const std::vector<double>& sbmax = c->lists.sbmax;
   // packed pair records and atom positions of the ERI kernels (load_pair_jk)
+  std::vector<double4> x4(c->n_atom);
+  std::vector<int4> jr(2 * c->n_pairs);
   {
-    std::vector<double4> x4(c->n_atom);
     for (int i = 0; i < c->n_atom; ++i) x4[i] = make_double4(c->xyz[3 * i], c->xyz[3 * i + 1], c->xyz[3 * i + 2], 0.0);
     TF_CUDA(c->d_xyz4.reserve(std::max<size_t>(x4.size(), 1)));
-    TF_CUDA(cudaMemcpy(c->d_xyz4.p, x4.data(), x4.size() * sizeof(double4), cudaMemcpyHostToDevice));
-    std::vector<int4> jr(2 * c->n_pairs);
+    TF_CUDA(upload(c, c->d_xyz4.p, x4.data(), x4.size()));
     for (long long p = 0; p < c->n_pairs; ++p) {
       const PairRec& q = c->pairs_h[p];
       if (q.n_full > 0xffff || q.n_skip > 0xffff) { set_error("too many primitive pairs in one shell pair"); return TF_EUNSUPPORTED; }
@@ -1869,7 +1878,7 @@ static int setup_pairs(tf_ctx* c) {
                                 (int)((unsigned)q.mol | (q.sh_hi == q.sh_lo ? 0x80000000u : 0u)));
     }
     TF_CUDA(c->d_jkrec.reserve(std::max<size_t>(jr.size(), 1)));
-    TF_CUDA(cudaMemcpy(c->d_jkrec.p, jr.data(), jr.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    TF_CUDA(upload(c, c->d_jkrec.p, jr.data(), jr.size()));
   }
   std::vector<int4> srec(sorted.size());
   for (size_t q = 0; q < sorted.size(); ++q) {
@@ -1891,14 +1900,13 @@ static int setup_pairs(tf_ctx* c) {
     TF_CUDA(c->d_cn.reserve(std::max<size_t>(L.cn.size(), 1)));
     TF_CUDA(c->d_fam_mem.reserve(std::max<size_t>(c->fams.members.size(), 1)));
     if (!L.csorted.empty()) {
-      TF_CUDA(cudaMemcpy(c->d_csorted.p, L.csorted.data(), L.csorted.size() * sizeof(int), cudaMemcpyHostToDevice));
-      TF_CUDA(cudaMemcpy(c->d_cimax.p, L.cimax.data(), L.cimax.size() * sizeof(double), cudaMemcpyHostToDevice));
-      TF_CUDA(cudaMemcpy(c->d_cxstart.p, L.cxstart.data(), L.cxstart.size() * sizeof(int), cudaMemcpyHostToDevice));
-      TF_CUDA(cudaMemcpy(c->d_cn.p, L.cn.data(), L.cn.size() * sizeof(int), cudaMemcpyHostToDevice));
+      TF_CUDA(upload(c, c->d_csorted.p, L.csorted.data(), L.csorted.size()));
+      TF_CUDA(upload(c, c->d_cimax.p, L.cimax.data(), L.cimax.size()));
+      TF_CUDA(upload(c, c->d_cxstart.p, L.cxstart.data(), L.cxstart.size()));
+      TF_CUDA(upload(c, c->d_cn.p, L.cn.data(), L.cn.size()));
     }
     if (!c->fams.members.empty())
-      TF_CUDA(cudaMemcpy(c->d_fam_mem.p, c->fams.members.data(), c->fams.members.size() * sizeof(int4),
-                         cudaMemcpyHostToDevice));
+      TF_CUDA(upload(c, c->d_fam_mem.p, c->fams.members.data(), c->fams.members.size()));
   }
   TF_CUDA(c->d_srec.reserve(std::max<size_t>(srec.size(), 1)));
   TF_CUDA(cudaMemcpyAsync(c->d_srec.p, srec.data(), srec.size() * sizeof(int4), cudaMemcpyHostToDevice, c->stream));
@@ -2607,15 +2615,6 @@ static int create_impl(const tf_basis* bases, int n_mol, const tf_options* opt, 
     c->n_atom += B->n_atom;
   }
   if (c->cmat_off[n_mol] > (1LL << 36)) { delete c; set_error("batch too large"); return TF_EUNSUPPORTED; }
-  {
-    if (cudaMemcpyToSymbol(c_U, g_tables.U, sizeof(g_tables.U)) != cudaSuccess ||
-        cudaMemcpyToSymbol(c_comp, g_tables.comp, sizeof(g_tables.comp)) != cudaSuccess ||
-        cudaMemcpyToSymbol(c_cidx, g_tables.cidx, sizeof(g_tables.cidx)) != cudaSuccess ||
-        cudaFuncSetAttribute(k_schwarz_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             WARPS_PER_BLOCK * W_SMEM * (int)sizeof(double)) != cudaSuccess) {
-      delete c; set_error("constant upload"); return TF_ECUDA;
-    }
-  }
 #define TF_TRY(x)                               \
   do {                                          \
     int r__ = (x);                              \
@@ -2623,7 +2622,7 @@ static int create_impl(const tf_basis* bases, int n_mol, const tf_options* opt, 
   } while (0)
   auto up = [&](auto& buf, const auto& v) -> int {
     if (buf.reserve(std::max<size_t>(v.size(), 1)) != cudaSuccess) { set_error("device allocation"); return TF_ENOMEM; }
-    if (!v.empty() && cudaMemcpy(buf.p, v.data(), v.size() * sizeof(v[0]), cudaMemcpyHostToDevice) != cudaSuccess) {
+    if (!v.empty() && upload(c, buf.p, v.data(), v.size()) != cudaSuccess) {
       set_error("upload"); return TF_ECUDA;
     }
     return TF_OK;
@@ -2633,6 +2632,14 @@ static int create_impl(const tf_basis* bases, int n_mol, const tf_options* opt, 
       cudaEventCreate(&c->ev2) != cudaSuccess ||
       cudaEventCreateWithFlags(&c->order_ev, cudaEventDisableTiming) != cudaSuccess) {
     tf_ctx_destroy(c); set_error("stream/event creation"); return TF_ECUDA;
+  }
+  const cudaMemcpyKind h2d = cudaMemcpyHostToDevice;
+  if (cudaMemcpyToSymbolAsync(c_U, g_tables.U, sizeof(g_tables.U), 0, h2d, c->stream) != cudaSuccess ||
+      cudaMemcpyToSymbolAsync(c_comp, g_tables.comp, sizeof(g_tables.comp), 0, h2d, c->stream) != cudaSuccess ||
+      cudaMemcpyToSymbolAsync(c_cidx, g_tables.cidx, sizeof(g_tables.cidx), 0, h2d, c->stream) != cudaSuccess ||
+      cudaFuncSetAttribute(k_schwarz_warp, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           WARPS_PER_BLOCK * W_SMEM * (int)sizeof(double)) != cudaSuccess) {
+    tf_ctx_destroy(c); set_error("constant upload"); return TF_ECUDA;
   }
   TF_TRY(up(c->d_mols, c->mols));
   TF_TRY(up(c->d_cmat_off, c->cmat_off));
@@ -2704,7 +2711,7 @@ int tf_set_geometry(tf_ctx* c, const double* xyz) {
   int rc = set_device(c);
   if (rc) return rc;
   c->xyz.assign(xyz, xyz + 3 * c->n_atom);
-  TF_CUDA(cudaMemcpy(c->d_xyz.p, c->xyz.data(), c->xyz.size() * sizeof(double), cudaMemcpyHostToDevice));
+  TF_CUDA(upload(c, c->d_xyz.p, c->xyz.data(), c->xyz.size()));
   c->geometry_ready = false;
   return setup_pairs(c);
 }
@@ -2729,7 +2736,8 @@ int tf_set_molecule_cutoffs(tf_ctx* c, const double* cutoffs) {
   if (c->d_mol_cut.reserve(c->n_mol) != cudaSuccess) { cudaGetLastError(); set_error("device allocation"); return TF_ENOMEM; }
   // builds are synchronous, so no captured or running build reads the array now; a
   // captured graph reads the new values at its next replay
-  TF_CUDA(cudaMemcpy(c->d_mol_cut.p, cutoffs, c->n_mol * sizeof(double), cudaMemcpyHostToDevice));
+  TF_CUDA(upload(c, c->d_mol_cut.p, cutoffs, c->n_mol));
+  TF_CUDA(cudaStreamSynchronize(c->stream));   // the caller's array is free again
   c->use_mol_cut = true;
   return TF_OK;
 }
@@ -3201,6 +3209,7 @@ static int noalloc_setup(int dev, NoAllocScratch** out) {
     // constant tables (component order, spherical matrices) for this device
     TF_CUDA(cudaMemcpyToSymbol(c_U, g_tables.U, sizeof(g_tables.U)));
     TF_CUDA(cudaMemcpyToSymbol(c_comp, g_tables.comp, sizeof(g_tables.comp)));
+    TF_CUDA(cudaStreamSynchronize(cudaStreamLegacy));   // landed, for callers on non-blocking streams
     g_noalloc_ptr[dev] = static_cast<NoAllocScratch*>(ptr);
   }
   *out = g_noalloc_ptr[dev];
