@@ -21,7 +21,7 @@ PEAK_LIB = os.path.join(HERE, "libtf_peak.so")
 
 SOURCES = ["tontofock.cu", "tf_jk_ss.cu", "tf_jk_ps.cu", "tf_jk_d.cu", "tf_jk_f.cu", "tf_jk_l.cu", "tf_jk_l2.cu", "tf_rows_d.cu",
            "tf_rows_fs.cu", "tf_rows_fd.cu", "tf_rows_ff.cu", "tf_mlp.cu"]
-DEPS = SOURCES + ["tf_device.cuh", "tf_thread.cuh", "tf_rows.cuh", "tf_warp.cuh", "rys_tables.inc", "boys_table.inc", "boys2_table.inc",
+DEPS = SOURCES + ["tf_device.cuh", "tf_thread.cuh", "tf_rows.cuh", "tf_warp.cuh", "tf_host.h", "rys_tables.inc", "boys_table.inc", "boys2_table.inc",
         os.path.join("..", "..", "include", "tontofock.h"), os.path.join("..", "..", "include", "tontofock_guess.h")]
 
 

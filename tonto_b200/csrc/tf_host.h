@@ -1,0 +1,60 @@
+// tf_host.h — host-side helpers of the library that hold no device code: they take the
+// runtime calls they make as a parameter, so that a host program can check them.
+#pragma once
+#include <cstddef>
+#include <vector>
+
+namespace tf {
+
+// A set of launches spread over branch streams.  fork() lets branches 1 .. n - 1 (side) wait
+// for the earlier work of the context's stream (branch 0); join() lets that stream wait for
+// them.  A scope that is left early, by an error between the two, joins as well: the
+// context's next call orders itself after the context's stream alone, so a branch that was
+// never joined could still be writing into its buffers.
+// Rt: static record(event, stream) and wait(stream, event), both with Status results.
+template <typename Rt>
+class BranchFork {
+  using Stream = typename Rt::Stream;
+  using Event = typename Rt::Event;
+  using Status = typename Rt::Status;
+
+ public:
+  BranchFork(Stream main, const std::vector<Stream>& side, Event fork_ev, const std::vector<Event>& join_ev, int n)
+      : main_(main), side_(side), fork_ev_(fork_ev), join_ev_(join_ev), n_(n) {}
+  BranchFork(const BranchFork&) = delete;
+  BranchFork& operator=(const BranchFork&) = delete;
+  ~BranchFork() { join(); }
+
+  Status fork() {
+    if (n_ <= 1) return Status{};
+    const Status r = Rt::record(fork_ev_, main_);
+    if (r != Status{}) return r;
+    for (int i = 0; i + 1 < n_; ++i) {
+      const Status w = Rt::wait(side_[i], fork_ev_);
+      if (w != Status{}) return w;
+      forked_ = i + 1;
+    }
+    return Status{};
+  }
+
+  Status join() {
+    Status first{};
+    for (int i = 0; i < forked_; ++i) {
+      Status r = Rt::record(join_ev_[i], side_[i]);
+      if (r == Status{}) r = Rt::wait(main_, join_ev_[i]);
+      if (first == Status{}) first = r;
+    }
+    forked_ = 0;
+    return first;
+  }
+
+ private:
+  Stream main_;
+  const std::vector<Stream>& side_;
+  Event fork_ev_;
+  const std::vector<Event>& join_ev_;
+  int n_;
+  int forked_ = 0;                     // side branches that wait for the context's stream and are not joined yet
+};
+
+}  // namespace tf

@@ -19,6 +19,7 @@
 #include "tf_warp.cuh"
 #include "tf_thread.cuh"
 #include "tf_rows.cuh"
+#include "tf_host.h"
 #include "../../include/tontofock.h"
 
 #include <cub/cub.cuh>
@@ -1224,25 +1225,19 @@ static int ensure_branches(tf_ctx* c, int n) {
 // 6.1, 6.2 and 6.3 ms; (H2O)32 cc-pVDZ 81.4, 76.8, 76.9, 76.2 and 76.4 ms.
 constexpr int DEFAULT_BRANCHES = 6;
 
-// Branches of the current schedule, and the start and end of a set of class launches on
-// them: the branches wait for the context stream's earlier work, and the context stream
-// then waits for the branches.
+// Branches of the current schedule, and a set of class launches on n of them.
 static int sched_branches(const tf_ctx* c) { return std::max(1, std::min(c->sched_streams, 1 + (int)c->side.size())); }
 
-static int fork_branches(tf_ctx* c, int ns) {
-  if (ns <= 1) return TF_OK;
-  TF_CUDA(cudaEventRecord(c->fork_ev, c->stream));
-  for (int i = 0; i + 1 < ns; ++i) TF_CUDA(cudaStreamWaitEvent(c->side[i], c->fork_ev, 0));
-  return TF_OK;
-}
-
-static int join_branches(tf_ctx* c, int ns) {
-  for (int i = 0; i + 1 < ns; ++i) {
-    TF_CUDA(cudaEventRecord(c->join_ev[i], c->side[i]));
-    TF_CUDA(cudaStreamWaitEvent(c->stream, c->join_ev[i], 0));
-  }
-  return TF_OK;
-}
+struct CudaRt {
+  using Stream = cudaStream_t;
+  using Event = cudaEvent_t;
+  using Status = cudaError_t;
+  static cudaError_t record(cudaEvent_t e, cudaStream_t s) { return cudaEventRecord(e, s); }
+  static cudaError_t wait(cudaStream_t s, cudaEvent_t e) { return cudaStreamWaitEvent(s, e, 0); }
+};
+struct Fork : BranchFork<CudaRt> {
+  Fork(tf_ctx* c, int n) : BranchFork<CudaRt>(c->stream, c->side, c->fork_ev, c->join_ev, n) {}
+};
 
 // Host-to-device copy on the context's stream.  (A plain cudaMemcpy from pageable memory may
 // return before its transfer has landed, and the context's non-blocking streams do not wait
@@ -1803,7 +1798,18 @@ static int setup_pairs(tf_ctx* c) {
   // the classes' launches overlap on the build's branch streams (each ends in a tail of its
   // longest contractions); the f classes share one scratch area and stay on the context's
   TF_TRY_RC(ensure_branches(c, DEFAULT_BRANCHES));
-  TF_TRY_RC(fork_branches(c, DEFAULT_BRANCHES));
+  // pair classes with an f shell: the warp path in global scratch (two blocks of
+  // WARPS_PER_BLOCK warps per SM)
+  long long f_warps = 0;
+  if (cls_start[NPAIRCLS] > cls_start[pair_class(3, 0)]) {
+    int dev = 0, nsm = 148;
+    TF_CUDA(cudaGetDevice(&dev));
+    TF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+    f_warps = (long long)nsm * 2 * WARPS_PER_BLOCK;
+    TF_CUDA(c->d_wscratch.reserve((size_t)f_warps * WF_SCRATCH));
+  }
+  Fork branches(c, DEFAULT_BRANCHES);
+  TF_CUDA(branches.fork());
   auto branch = [&](int k) { return k == 0 ? c->stream : c->side[(k - 1) % (DEFAULT_BRANCHES - 1)]; };
 #define TF_SCHWARZ(LH, LL)                                                                                  \
   {                                                                                                         \
@@ -1824,24 +1830,17 @@ static int setup_pairs(tf_ctx* c) {
                          WARPS_PER_BLOCK * W_SMEM * sizeof(double), branch(k)>>>(
             c->d_schwarz_ids.p + cls_start[k], nk, c->d_pairs.p, c->d_prim_full.p, c->spherical, lh, ll, nullptr);
     }
-  // pair classes with an f shell: the warp path in global scratch (two blocks of
-  // WARPS_PER_BLOCK warps per SM)
-  if (cls_start[NPAIRCLS] > cls_start[pair_class(3, 0)]) {
-    int dev = 0, nsm = 148;
-    TF_CUDA(cudaGetDevice(&dev));
-    TF_CUDA(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-    const long long warps = (long long)nsm * 2 * WARPS_PER_BLOCK;
-    TF_CUDA(c->d_wscratch.reserve((size_t)warps * WF_SCRATCH));
+  if (f_warps > 0) {
     for (int ll = 0; ll <= 3; ++ll) {
       const int k = pair_class(3, ll);
       const int nk = cls_start[k + 1] - cls_start[k];
       if (nk > 0)
-        k_schwarz_warp<<<(unsigned)std::min<long long>(warps / WARPS_PER_BLOCK, (nk + WARPS_PER_BLOCK - 1) / WARPS_PER_BLOCK),
+        k_schwarz_warp<<<(unsigned)std::min<long long>(f_warps / WARPS_PER_BLOCK, (nk + WARPS_PER_BLOCK - 1) / WARPS_PER_BLOCK),
                          32 * WARPS_PER_BLOCK, 0, c->stream>>>(c->d_schwarz_ids.p + cls_start[k], nk, c->d_pairs.p,
                                                               c->d_prim_full.p, c->spherical, 3, ll, c->d_wscratch.p);
     }
   }
-  TF_TRY_RC(join_branches(c, DEFAULT_BRANCHES));
+  TF_CUDA(branches.join());
   TF_CUDA(cudaGetLastError());
   TF_CUDA(cudaMemcpyAsync(c->pairs_h.data(), c->d_pairs.p, c->n_pairs * sizeof(PairRec), cudaMemcpyDeviceToHost,
                           c->stream));
@@ -2183,7 +2182,8 @@ static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* d
   // the graph (the autotuner's choice), so that one class's tail overlaps another
   // class's start; J and K are summed with atomics, so the order is free
   const int ns = sched_branches(c);
-  TF_TRY_RC(fork_branches(c, ns));
+  Fork branches(c, ns);
+  TF_CUDA(branches.fork());
   for (int g = 0; g < ng; ++g) {
     if (c->group_task0[g + 1] == c->group_task0[g]) continue;   // no molecule has this class pair
     int l1h, l1l, l2h, l2l;
@@ -2216,7 +2216,7 @@ static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* d
       kernels++;
     }
   }
-  TF_TRY_RC(join_branches(c, ns));
+  TF_CUDA(branches.join());
   return enqueue_finalize(c, dJ, dK, dJb, dKb, kernels);
 }
 
@@ -2438,7 +2438,8 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
                             c->d_quartets.p, s, kernels);
       if (rc) return rc;
     }
-    TF_TRY_RC(fork_branches(c, ns));
+    Fork branches(c, ns);
+    TF_CUDA(branches.fork());
     for (int g = g0; g < g1; ++g) {
       int l1h, l1l, l2h, l2l;
       class_l(c->group_cls[g].x, l1h, l1l);
@@ -2475,7 +2476,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
       }
       if (timed) TF_CUDA(cudaEventRecord(c->cls_ev[2 * g + 1], s));
     }
-    TF_TRY_RC(join_branches(c, ns));
+    TF_CUDA(branches.join());
   }
   (void)nq_total;
   rc = enqueue_finalize(c, dJ, dK, dJb, dKb, kernels);
@@ -3100,7 +3101,8 @@ int tf_one_electron(tf_ctx* c, const double* Z, double* S, double* T, double* V)
   // Cartesian blocks into the (reused) Cartesian accumulators, then to the basis
   double* const in[3] = {c->d_Jc.p, c->d_Kc.p, c->d_Pc.p};
   TF_TRY_RC(ensure_branches(c, DEFAULT_BRANCHES));
-  TF_TRY_RC(fork_branches(c, DEFAULT_BRANCHES));
+  Fork branches(c, DEFAULT_BRANCHES);
+  TF_CUDA(branches.fork());
 #define TF_ONE_EL(LH, LL)                                                                                  \
   launch_one_electron<LH, LL>(c, pair_class(LH, LL), in,                                                   \
                               pair_class(LH, LL) == 0 ? s : c->side[(pair_class(LH, LL) - 1) % (DEFAULT_BRANCHES - 1)])
@@ -3108,7 +3110,7 @@ int tf_one_electron(tf_ctx* c, const double* Z, double* S, double* T, double* V)
   TF_ONE_EL(2, 2); TF_ONE_EL(3, 0); TF_ONE_EL(3, 1); TF_ONE_EL(3, 2); TF_ONE_EL(3, 3);
 #undef TF_ONE_EL
   TF_CUDA(cudaGetLastError());
-  TF_TRY_RC(join_branches(c, DEFAULT_BRANCHES));
+  TF_CUDA(branches.join());
   const long long n2 = c->bmat_off[c->n_mol];
   const BatchArgs bt = batch_args(c);
   double* const outs[3] = {S, T, V};
