@@ -1,7 +1,9 @@
 // tf_host.h — host-side helpers of the library that hold no device code: they take the
 // runtime calls they make as a parameter, so that a host program can check them.
 #pragma once
+#include <atomic>
 #include <cstddef>
+#include <mutex>
 #include <vector>
 
 namespace tf {
@@ -55,6 +57,37 @@ class BranchFork {
   const std::vector<Event>& join_ev_;
   int n_;
   int forked_ = 0;                     // side branches that wait for the context's stream and are not joined yet
+};
+
+// A value per device, made at the first use on that device: a kernel's launch set-up, which
+// holds for one device (function attributes are per device), not for the process.  Several
+// threads may ask at once; a value is seen only when it is complete.
+template <typename V>
+class PerDevice {
+  static constexpr int MAX_DEVICES = 64;
+
+ public:
+  // make(V&) -> bool: false, it failed (it is tried again at the next use).
+  template <typename Make>
+  bool get(int device, V& out, Make&& make) {
+    if (device < 0 || device >= MAX_DEVICES) return make(out);     // beyond the table: not kept
+    if (!ready_[device].load(std::memory_order_acquire)) {
+      std::lock_guard<std::mutex> lock(mutex_);
+      if (!ready_[device].load(std::memory_order_relaxed)) {
+        V v{};
+        if (!make(v)) return false;
+        value_[device] = v;
+        ready_[device].store(true, std::memory_order_release);
+      }
+    }
+    out = value_[device];
+    return true;
+  }
+
+ private:
+  std::mutex mutex_;
+  std::atomic<bool> ready_[MAX_DEVICES] = {};
+  V value_[MAX_DEVICES] = {};
 };
 
 }  // namespace tf

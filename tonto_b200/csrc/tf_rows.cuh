@@ -24,6 +24,9 @@
 // short lists only (dispatch_jk has both sides' times).
 #pragma once
 #include "tf_device.cuh"
+#include "tf_host.h"
+
+#include <algorithm>
 
 namespace tf {
 
@@ -518,7 +521,8 @@ constexpr int rows_wpb() {
   return C::GW > 1 ? C::GW : C::QPW * C::per_group(1) * 8 > 12288 ? 1 : 4;
 }
 
-// Launches the class (false: out of its limits).  n <= 0 without a range only sets up.
+// Launches the class (false: the launch could not be set up, which is done once per device).
+// n <= 0 without a range only sets up.
 template <int LA, int LB, int LC, int LD>
 static bool launch_rows_t(const RowArgs& a, cudaStream_t s) {
   using C = RowCfg<LA, LB, LC, LD>;
@@ -526,27 +530,35 @@ static bool launch_rows_t(const RowArgs& a, cudaStream_t s) {
   constexpr int QPB = C::GW > 1 ? 1 : C::QPW * WPB;
   const size_t smem = (size_t)QPB * C::per_group(a.P2 ? 2 : 1) * sizeof(double);
   constexpr bool CAN_SHARE = C::QPW > 1;
-  static int per_sm[2] = {-1, -1};            // restricted, unrestricted
-  if (per_sm[1] < 0) {
+  struct Resident {
+    long long blocks[2];                      // restricted, unrestricted
+  };
+  static PerDevice<Resident> resident;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  Resident r_dev{};
+  const bool ready = resident.get(dev, r_dev, [&](Resident& v) {
     const int top = (int)(QPB * C::per_group(2) * sizeof(double));
-    if (cudaFuncSetAttribute(k_jk_rows<LA, LB, LC, LD, WPB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, top) !=
+    int nsm = 0;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(k_jk_rows<LA, LB, LC, LD, WPB, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, top) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_jk_rows<LA, LB, LC, LD, WPB, CAN_SHARE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              top) != cudaSuccess)
       return false;
     for (int u = 0; u < 2; ++u) {
       int nb = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_jk_rows<LA, LB, LC, LD, WPB, false>, 32 * WPB,
-                                                    (size_t)QPB * C::per_group(1 + u) * sizeof(double));
-      per_sm[u] = nb < 1 ? 1 : nb;
+      if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_jk_rows<LA, LB, LC, LD, WPB, false>, 32 * WPB,
+                                                        (size_t)QPB * C::per_group(1 + u) * sizeof(double)) != cudaSuccess)
+        return false;
+      v.blocks[u] = (long long)nsm * std::max(nb, 1);
     }
-  }
+    return true;
+  });
+  if (!ready) return false;
   if (a.n <= 0 && !a.range) return true;
-  int dev = 0, nsm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
   RowArgs r = a;
-  const long long full = (long long)nsm * per_sm[a.P2 ? 1 : 0];
+  const long long full = r_dev.blocks[a.P2 ? 1 : 0];
   r.groups = full * QPB;
   // sharing groups where the list is expected to leave half of them idle; always in a
   // deterministic build, whose sums must not depend on an expectation

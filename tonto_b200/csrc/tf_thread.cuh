@@ -3,6 +3,7 @@
 // classes are shared out over translation units (tf_jk_*.cu), which build in parallel.
 #pragma once
 #include "tf_device.cuh"
+#include "tf_host.h"
 
 #include <algorithm>
 
@@ -484,81 +485,85 @@ __global__ void __launch_bounds__(jk_threads<LA, LB, LC, LD, V>(), 1) k_jk(JKArg
   count_quartets(a, qclass_id(LA, LB, LC, LD), nprim, nquart);
 }
 
-// Launch set-up (shared-memory attribute, resident blocks per SM), done once per
-// kernel and before any graph capture: a zero-sized, range-less JKArgs only sets up.
+// Launch set-up (shared-memory attribute, resident blocks of the GPU), done once per
+// kernel and device and before any graph capture: a JKArgs without a plan only sets up.
+// false: the set-up failed.
 template <int LA, int LB, int LC, int LD, typename T, int V, int MB>
-static void launch_jk_t(const JKArgs& a, cudaStream_t s) {
+static bool launch_jk_t(const JKArgs& a, cudaStream_t s) {
   constexpr int thr = jk_threads<LA, LB, LC, LD, V>();
   constexpr size_t smem = RootTable<LA, LB, LC, LD, T>::SIZE * sizeof(double);
-  static int blocks_per_sm = -1;
-  if (blocks_per_sm < 0) {
-    cudaFuncSetAttribute(k_jk<LA, LB, LC, LD, T, V, MB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    {                                  // shared storage for one block, the rest to L1
-      int dev = 0, per_sm = 0;
-      cudaGetDevice(&dev);
-      cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-      const int pct = per_sm > 0 ? std::min(100, (int)((smem + 2048) * 100 / per_sm) + 1) : 100;
-      cudaFuncSetAttribute(k_jk<LA, LB, LC, LD, T, V, MB>, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
-    }
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks_per_sm, k_jk<LA, LB, LC, LD, T, V, MB>, thr, smem);
-    if (blocks_per_sm < 1) blocks_per_sm = 1;
-  }
-  if (!a.plan) return;
-  int dev = 0, nsm = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  const long long full = (long long)nsm * blocks_per_sm;
+  static PerDevice<long long> resident;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return false;
+  long long full = 0;
+  const bool ready = resident.get(dev, full, [&](long long& blocks) {
+    auto* const kernel = k_jk<LA, LB, LC, LD, T, V, MB>;
+    int nsm = 0, per_sm = 0, nb = 0;
+    if (cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&per_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+      return false;
+    // shared storage for one block, the rest to L1
+    const int pct = per_sm > 0 ? std::min(100, (int)((smem + 2048) * 100 / per_sm) + 1) : 100;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct) != cudaSuccess ||
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, thr, smem) != cudaSuccess)
+      return false;
+    blocks = (long long)nsm * std::max(nb, 1);
+    return true;
+  });
+  if (!ready) return false;
+  if (!a.plan) return true;
   // (n known: at most a warp an entry)
   const long long blocks = a.range ? full : std::min<long long>((a.n * 32 + thr - 1) / thr, full);
   k_jk<LA, LB, LC, LD, T, V, MB><<<(unsigned)blocks, thr, smem, s>>>(a);
+  return true;
 }
 
 template <int LA, int LB, int LC, int LD, int V, int MB>
-static void launch_jk_v(const JKArgs& a, cudaStream_t s, bool fp32) {
-  if (fp32) launch_jk_t<LA, LB, LC, LD, float, V, MB>(a, s);
-  else launch_jk_t<LA, LB, LC, LD, double, V, MB>(a, s);
+static bool launch_jk_v(const JKArgs& a, cudaStream_t s, bool fp32) {
+  return fp32 ? launch_jk_t<LA, LB, LC, LD, float, V, MB>(a, s) : launch_jk_t<LA, LB, LC, LD, double, V, MB>(a, s);
 }
 
 template <int LA, int LB, int LC, int LD, int MB>
-static void launch_jk_m(const JKArgs& a, cudaStream_t s, bool fp32, int variant) {
+static bool launch_jk_m(const JKArgs& a, cudaStream_t s, bool fp32, int variant) {
   switch (variant & 7) {
-    case 1: launch_jk_v<LA, LB, LC, LD, 1, MB>(a, s, fp32); break;
-    case 2: launch_jk_v<LA, LB, LC, LD, 2, MB>(a, s, fp32); break;
-    case 3: launch_jk_v<LA, LB, LC, LD, 3, MB>(a, s, fp32); break;
-    case 4: case 6: launch_jk_v<LA, LB, LC, LD, 6, MB>(a, s, fp32); break;   // deterministic: always bit 2
-    case 5: case 7: launch_jk_v<LA, LB, LC, LD, 7, MB>(a, s, fp32); break;
-    default: launch_jk_v<LA, LB, LC, LD, 0, MB>(a, s, fp32); break;
+    case 1: return launch_jk_v<LA, LB, LC, LD, 1, MB>(a, s, fp32);
+    case 2: return launch_jk_v<LA, LB, LC, LD, 2, MB>(a, s, fp32);
+    case 3: return launch_jk_v<LA, LB, LC, LD, 3, MB>(a, s, fp32);
+    case 4: case 6: return launch_jk_v<LA, LB, LC, LD, 6, MB>(a, s, fp32);   // deterministic: always bit 2
+    case 5: case 7: return launch_jk_v<LA, LB, LC, LD, 7, MB>(a, s, fp32);
+    default: return launch_jk_v<LA, LB, LC, LD, 0, MB>(a, s, fp32);
   }
 }
 
 // The bra-family kernel of the class (fam_cap_l) when the launch is a family group.
 template <int LA, int LB, int LC, int LD>
-static void launch_jk(const JKArgs& a, cudaStream_t s, bool fp32, int variant) {
+static bool launch_jk(const JKArgs& a, cudaStream_t s, bool fp32, int variant) {
   constexpr int CAP = fam_cap_l(LA, LB, LC, LD);
   if constexpr (CAP > 1) {
-    if (a.fam > 1) {
-      launch_jk_m<LA, LB, LC, LD, CAP>(a, s, fp32, variant);
-      return;
-    }
+    if (a.fam > 1) return launch_jk_m<LA, LB, LC, LD, CAP>(a, s, fp32, variant);
   }
-  launch_jk_m<LA, LB, LC, LD, 1>(a, s, fp32, variant);
+  return launch_jk_m<LA, LB, LC, LD, 1>(a, s, fp32, variant);
 }
 
 // Classes whose (e0|f0) block and integrals do not fit a thread's registers: FP64 for the
 // FP32 buckets too, and the two instantiations that differ in their results' bits only
 // (deterministic or not; a register-bounded variant would spill more).
 template <int LA, int LB, int LC, int LD>
-static void launch_jk_f64(const JKArgs& a, cudaStream_t s, bool, int variant) {
-  if (variant & 4) launch_jk_t<LA, LB, LC, LD, double, 6, 1>(a, s);
-  else launch_jk_t<LA, LB, LC, LD, double, 0, 1>(a, s);
+static bool launch_jk_f64(const JKArgs& a, cudaStream_t s, bool, int variant) {
+  return variant & 4 ? launch_jk_t<LA, LB, LC, LD, double, 6, 1>(a, s) : launch_jk_t<LA, LB, LC, LD, double, 0, 1>(a, s);
 }
 
-// The classes of one translation unit each (tf_jk_*.cu); false: not a class of that unit.
-bool launch_jk_ss(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
-bool launch_jk_ps(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
-bool launch_jk_d(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
-bool launch_jk_l(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
-bool launch_jk_l2(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
-bool launch_jk_f(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+// The classes of one translation unit each (tf_jk_*.cu); 1: launched, 0: not a class of
+// that unit, -1: the launch could not be set up.
+int launch_jk_ss(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+int launch_jk_ps(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+int launch_jk_d(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+int launch_jk_l(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+int launch_jk_l2(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+int launch_jk_f(int key, const JKArgs& a, cudaStream_t s, bool fp32, int variant);
+
+#define TF_JK_CASE(LAUNCH, A, B, C, D) \
+  case class_key(A, B, C, D): return LAUNCH<A, B, C, D>(a, s, fp32, variant) ? 1 : -1;
 
 }  // namespace tf

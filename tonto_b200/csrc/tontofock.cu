@@ -1943,9 +1943,14 @@ static void launch_one_electron(tf_ctx* c, int k, double* const* out, cudaStream
 // classes up to d shells); roots, weights, transfers and the Fock accumulation stay FP64.
 static int dispatch_jk(int la, int lb, int lc, int ld, const JKArgs& a, cudaStream_t s, bool fp32, int variant = 0) {
   const int key = class_key(la, lb, lc, ld);
-  if (launch_jk_ss(key, a, s, fp32, variant) || launch_jk_ps(key, a, s, fp32, variant) ||
-      launch_jk_d(key, a, s, fp32, variant) || launch_jk_f(key, a, s, fp32, variant))
-    return TF_OK;
+  auto status = [](int rc) {
+    if (rc > 0) return TF_OK;
+    cudaGetLastError();
+    set_error("launch set-up of a quartet kernel");
+    return TF_ECUDA;
+  };
+  for (auto* launch : {launch_jk_ss, launch_jk_ps, launch_jk_d, launch_jk_f})
+    if (const int rc = launch(key, a, s, fp32, variant)) return status(rc);
   // Both kinds of kernel exist for the classes of up to a hundred elements (e0|f0) and for the
   // ps kets (three lanes to a lane group).  One thread a quartet, spilling to L1, issues a third
   // of the lane groups' instructions, but its quartet takes 30 to 120 us however few there
@@ -1960,17 +1965,14 @@ static int dispatch_jk(int la, int lb, int lc, int ld, const JKArgs& a, cudaStre
   // at 30000.  A deterministic build's bits must not depend on an expectation: always the
   // thread kernels.
   constexpr long long ROWS_BELOW = 8192;
-  if ((a.fx_lo || a.expect >= ROWS_BELOW) &&
-      (launch_jk_l(key, a, s, fp32, variant) || launch_jk_l2(key, a, s, fp32, variant)))
-    return TF_OK;
+  if (a.fx_lo || a.expect >= ROWS_BELOW)
+    for (auto* launch : {launch_jk_l, launch_jk_l2})
+      if (const int rc = launch(key, a, s, fp32, variant)) return status(rc);
   const RowArgs r{a.quartets + (a.range ? 0 : a.first - a.base), a.n, a.prim_full, a.prim_skip, a.P, a.J, a.K, a.mols, a.prim_count, a.range, a.base,
                   a.cap, a.jkrec, a.xyz4, a.P2, a.J2, a.K2, a.want,
                   a.qcount ? a.qcount + (a.bucket32 ? NQCLS : 0) : nullptr, a.fx_lo, 0, a.expect};
-  for (auto* launch : {launch_rows_d, launch_rows_fs, launch_rows_fd, launch_rows_ff}) {
-    const int rc = launch(key, r, s);
-    if (rc > 0) return TF_OK;
-    if (rc < 0) { set_error("launch set-up of a lane-group kernel"); return TF_ECUDA; }
-  }
+  for (auto* launch : {launch_rows_d, launch_rows_fs, launch_rows_fd, launch_rows_ff})
+    if (const int rc = launch(key, r, s)) return status(rc);
   set_error("quartet class not built");
   return TF_EUNSUPPORTED;
 }
