@@ -2785,8 +2785,29 @@ int tf_autotune(tf_ctx* c, const double* dP, double* dJ, double* dK, int flags, 
   if (rc) return rc;
   TF_CUDA(cudaDeviceSynchronize());    // dP may still be being written on any of the caller's streams
   TF_TRY_RC(ensure_branches(c, max_streams));
-  c->sched_tuned = true;
-  const bool use_graph = c->use_graph;
+  // the context's own settings, put back unless everything below succeeds
+  struct Trial {
+    tf_ctx* c;
+    bool keep = false, use_graph, tuned;
+    int streams;
+    std::vector<int> stream_of, variant;
+    explicit Trial(tf_ctx* ctx)
+        : c(ctx), use_graph(ctx->use_graph), tuned(ctx->sched_tuned), streams(ctx->sched_streams),
+          stream_of(ctx->sched_stream_of), variant(ctx->cls_variant) {}
+    void schedule_back() {
+      c->sched_tuned = tuned;
+      c->sched_streams = streams;
+      c->sched_stream_of = stream_of;
+    }
+    ~Trial() {
+      c->use_graph = use_graph;
+      if (!keep) {
+        schedule_back();
+        c->cls_variant = variant;
+      }
+      drop_graph(c);
+    }
+  } trial(c);
   tf_tune res{};
   const int ng = (int)c->group_cls.size();
   // launch-bound variant of each class pair's kernel: class-by-class builds with
@@ -2799,7 +2820,7 @@ int tf_autotune(tf_ctx* c, const double* dP, double* dJ, double* dK, int flags, 
     std::fill(c->cls_variant.begin(), c->cls_variant.end(), v);
     for (int rep = 0; rep < 2; ++rep) {
       rc = build_jk_device(c, dP, dJ, dK, flags);
-      if (rc) { c->use_graph = use_graph; return rc; }
+      if (rc) return rc;
     }
     for (int g = 0; g < ng; ++g) {
       float ms = 0.f;
@@ -2814,13 +2835,8 @@ int tf_autotune(tf_ctx* c, const double* dP, double* dJ, double* dK, int flags, 
     c->cls_variant[g] = best_v;
     if (best_v) res.variant_classes++;
   }
-  {                                    // later contexts on this device start from this choice
-    std::lock_guard<std::mutex> lock(g_variant_mutex);
-    g_variant_cache[c->device] = c->cls_variant;
-  }
   // class-pair times from a class-by-class build with the chosen variants
   rc = build_jk_device(c, dP, dJ, dK, flags);
-  c->use_graph = use_graph;
   if (rc) return rc;
   res.direct_ms = c->stats.build_ms;
   std::vector<double> t(ng, 0.0);
@@ -2836,8 +2852,8 @@ int tf_autotune(tf_ctx* c, const double* dP, double* dJ, double* dK, int flags, 
   double best_ms = 1e300;
   std::vector<int> best_of(ng, 0);
   if (c->graph_cap > 0) {
-    const bool saved = c->use_graph;
     c->use_graph = true;
+    c->sched_tuned = true;
     for (int ns = 1; ns <= max_streams; ++ns) {
       std::vector<double> load(ns, 0.0);
       std::vector<int> of(ng, 0);
@@ -2852,18 +2868,23 @@ int tf_autotune(tf_ctx* c, const double* dP, double* dJ, double* dK, int flags, 
       double ms = 1e300;
       for (int rep = 0; rep < 4; ++rep) {
         rc = build_jk_device(c, dP, dJ, dK, flags);
-        if (rc) { c->use_graph = saved; return rc; }
+        if (rc) return rc;
         if (rep > 0 && c->stats.graph) ms = std::min(ms, c->stats.build_ms);
       }
       res.ms[ns - 1] = ms;
       res.candidates = ns;
       if (ms < best_ms * 0.99) { best_ms = ms; best = ns; best_of = of; }
     }
-    c->use_graph = saved;
+    c->sched_streams = best;
+    c->sched_stream_of = best_of;
+  } else {
+    trial.schedule_back();             // a chunked list: no graph, so no schedule was timed
   }
-  c->sched_streams = best;
-  c->sched_stream_of = best_of;
-  drop_graph(c);
+  trial.keep = true;
+  {                                    // later contexts on this device start from these variants
+    std::lock_guard<std::mutex> lock(g_variant_mutex);
+    g_variant_cache[c->device] = c->cls_variant;
+  }
   res.streams = best;
   c->tune = res;
   if (out) *out = res;
