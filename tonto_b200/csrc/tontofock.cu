@@ -1079,6 +1079,74 @@ struct PinnedStage {
   }
 };
 
+// A captured build.  The caller's arrays (densities, J, K) appear in a few of its nodes, whose
+// parameters are changed when a call brings other arrays: a setting takes some microseconds,
+// a capture with its instantiation 0.9 ms, longer than a small build itself ((H2O)2 cc-pVDZ
+// 0.28 ms).  The captured graph is kept, as it names the nodes of the executable one.
+struct BuildIO {
+  const double* P[2] = {nullptr, nullptr};     // alpha (or total) and beta
+  double* J[2] = {nullptr, nullptr};
+  double* K[2] = {nullptr, nullptr};
+  bool operator==(const BuildIO& o) const {
+    return P[0] == o.P[0] && P[1] == o.P[1] && J[0] == o.J[0] && J[1] == o.J[1] && K[0] == o.K[0] && K[1] == o.K[1];
+  }
+};
+
+struct BuildGraph {
+  cudaGraph_t graph = nullptr;
+  cudaGraphExec_t exec = nullptr;
+  cudaGraphNode_t density[2] = {nullptr, nullptr}, pmax = nullptr, finalize[2] = {nullptr, nullptr};
+  BuildIO io;                                  // the arrays that the nodes hold
+  bool mixed = false, mol_cut = false;         // mol_cut: the list passes read per-molecule cutoffs
+  int want = 3;
+  double cutoff = 0.0;
+  int kernels = 0;
+
+  void drop() {
+    if (exec) cudaGraphExecDestroy(exec);
+    if (graph) cudaGraphDestroy(graph);
+    *this = BuildGraph{};
+  }
+  cudaError_t set_io(const BuildIO& to);
+};
+
+// The node that a launch just captured on s became.
+static cudaError_t captured_node(cudaStream_t s, cudaGraphNode_t* node) {
+  cudaStreamCaptureStatus st;
+  const cudaGraphNode_t* deps = nullptr;
+  size_t n = 0;
+  const cudaError_t e = cudaStreamGetCaptureInfo_v2(s, &st, nullptr, nullptr, &deps, &n);
+  if (e != cudaSuccess) return e;
+  if (st != cudaStreamCaptureStatusActive || n != 1) return cudaErrorStreamCaptureInvalidated;
+  *node = deps[0];
+  return cudaSuccess;
+}
+
+// Parameters first, first + 1, .. of a kernel node set to the given pointers.
+static cudaError_t set_pointers(cudaGraphExec_t exec, cudaGraphNode_t node, int n_params, int first,
+                                std::initializer_list<const double*> pointers) {
+  cudaKernelNodeParams kp{};
+  const cudaError_t e = cudaGraphKernelNodeGetParams(node, &kp);
+  if (e != cudaSuccess) return e;
+  std::vector<void*> args(kp.kernelParams, kp.kernelParams + n_params);
+  std::vector<const double*> value(pointers);
+  for (size_t i = 0; i < value.size(); ++i) args[first + i] = &value[i];
+  kp.kernelParams = args.data();
+  return cudaGraphExecKernelNodeSetParams(exec, node, &kp);
+}
+
+cudaError_t BuildGraph::set_io(const BuildIO& to) {
+  const int spins = to.P[1] ? 2 : 1;
+  for (int i = 0; i < spins; ++i) {
+    cudaError_t e = set_pointers(exec, density[i], 4, 1, {to.P[i]});                 // k_density_to_cart
+    if (e == cudaSuccess) e = set_pointers(exec, finalize[i], 6, 3, {to.J[i], to.K[i]});   // k_finalize
+    if (e != cudaSuccess) return e;
+  }
+  const cudaError_t e = set_pointers(exec, pmax, 6, 1, {to.P[0], to.P[1]});          // k_pmax
+  if (e == cudaSuccess) io = to;
+  return e;
+}
+
 }  // namespace tf
 
 // ===========================================================================
@@ -1158,18 +1226,7 @@ struct tf_ctx {
   // graph builds
   bool use_graph = true;
   long long graph_cap = 0;                               // list entries a captured build may use
-  cudaGraphExec_t graph_exec = nullptr;
-  const double* graph_key_P = nullptr;
-  double* graph_key_J = nullptr;
-  double* graph_key_K = nullptr;
-  const double* graph_key_Pb = nullptr;       // unrestricted builds: the beta arrays (else null)
-  double* graph_key_Jb = nullptr;
-  double* graph_key_Kb = nullptr;
-  bool graph_key_mixed = false;
-  int graph_key_want = 3;
-  double graph_key_cutoff = 0.0;
-  bool graph_key_mol_cut = false;             // the captured list passes read per-molecule cutoffs
-  int graph_kernels = 0;
+  tf::BuildGraph graphs[2];                              // restricted, unrestricted
   // class schedule: graph branches and the branch of each class pair, set by the
   // autotuner or, until it has run, at each capture (default_schedule)
   bool sched_tuned = false;
@@ -1188,9 +1245,7 @@ struct tf_ctx {
 namespace tf {
 
 static void drop_graph(tf_ctx* c) {
-  if (c->graph_exec) cudaGraphExecDestroy(c->graph_exec);
-  c->graph_exec = nullptr;
-  c->graph_key_P = nullptr;
+  for (BuildGraph& g : c->graphs) g.drop();
 }
 
 static int set_device(tf_ctx* c) {
@@ -2048,16 +2103,19 @@ static int launch_list(tf_ctx* c, ListArgs a, long long t0, long long t1, long l
 // Density transform, pair maxima, quartet counts, their scan and the per-group
 // (start, FP32 start, end) offsets on the device: the part of a build shared by
 // the dynamic and the graph paths.
+// rec: the graph being captured (null: none), which notes the nodes that hold dP and dPb.
 static int enqueue_counts(tf_ctx* c, const double* dP, const double* dPb, bool mixed, long long cap, ListArgs& la,
-                          int& kernels) {
+                          int& kernels, BuildGraph* rec = nullptr) {
   cudaStream_t s = c->stream;
   const BatchArgs bt = batch_args(c);
   const long long nc2 = c->cmat_off[c->n_mol], ns2 = c->pmax_off[c->n_mol];
   const unsigned gc = (unsigned)std::max<long long>(1, (nc2 + 255) / 256);
   k_density_to_cart<<<gc, 256, 0, s>>>(bt, dP, nullptr, c->d_Pc.p);
+  if (rec) TF_CUDA(captured_node(s, &rec->density[0]));
   kernels++;
   if (dPb) {                                   // unrestricted: the beta density too
     k_density_to_cart<<<gc, 256, 0, s>>>(bt, dPb, nullptr, c->d_PcB.p);
+    if (rec) TF_CUDA(captured_node(s, &rec->density[1]));
     kernels++;
   }
   TF_CUDA(cudaMemsetAsync(c->d_pglob.p, 0, c->n_mol * sizeof(unsigned long long), s));
@@ -2065,6 +2123,7 @@ static int enqueue_counts(tf_ctx* c, const double* dP, const double* dPb, bool m
   TF_CUDA(cudaMemsetAsync(c->d_prim_count.p, 0, BUILD_COUNTERS * sizeof(unsigned long long), s));
   k_pmax<<<(unsigned)std::max<long long>(1, (ns2 + 255) / 256), 256, 0, s>>>(bt, dP, dPb, c->d_pmax.p, c->d_pglob.p,
                                                                              c->d_prim_count.p + NQCLS);
+  if (rec) TF_CUDA(captured_node(s, &rec->pmax));
   kernels++;
   la = ListArgs{c->d_tasks.p,    0,           c->n_tasks,    c->d_units.p, c->d_unit_group.p, c->d_group_task0.p,
                 c->d_sorted.p,   c->d_sorted_imax.p, c->d_sorted_bmax.p, c->d_srec.p, c->d_pairs.p,  c->d_mols.p,
@@ -2103,15 +2162,18 @@ static int enqueue_counts(tf_ctx* c, const double* dP, const double* dPb, bool m
   return TF_OK;
 }
 
-static int enqueue_finalize(tf_ctx* c, double* dJ, double* dK, double* dJb, double* dKb, int& kernels) {
+static int enqueue_finalize(tf_ctx* c, double* dJ, double* dK, double* dJb, double* dKb, int& kernels,
+                            BuildGraph* rec = nullptr) {
   cudaStream_t s = c->stream;
   const BatchArgs bt = batch_args(c);
   const long long nb2 = c->bmat_off[c->n_mol];
   const unsigned gb = (unsigned)std::max<long long>(1, (nb2 + 255) / 256);
   k_finalize<<<gb, 256, 0, s>>>(bt, c->d_Jc.p, c->d_Kc.p, dJ, dK, fx_offset(c));
+  if (rec) TF_CUDA(captured_node(s, &rec->finalize[0]));
   kernels++;
   if (dKb) {                                   // unrestricted: the beta J and K
     k_finalize<<<gb, 256, 0, s>>>(bt, c->d_JcB.p, c->d_KcB.p, dJb, dKb, fx_offset(c));
+    if (rec) TF_CUDA(captured_node(s, &rec->finalize[1]));
     kernels++;
   }
   TF_CUDA(cudaGetLastError());
@@ -2168,11 +2230,12 @@ static cudaStream_t branch_of(const tf_ctx* c, int g, int ns) {
 // build whose list is longer is detected on the host after the graph (the
 // ranges are clamped, so nothing is written out of bounds) and re-run on the
 // dynamic path with a larger buffer.
-static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* dK, const double* dPb, double* dJb,
-                              double* dKb, bool mixed, int want, int& kernels) {
+static int enqueue_graph_body(tf_ctx* c, const BuildIO& io, bool mixed, int want, BuildGraph& rec) {
   cudaStream_t s = c->stream;
+  const double* const dPb = io.P[1];
+  int& kernels = rec.kernels;
   ListArgs la;
-  int rc = enqueue_counts(c, dP, dPb, mixed, c->graph_cap, la, kernels);
+  int rc = enqueue_counts(c, io.P[0], dPb, mixed, c->graph_cap, la, kernels, &rec);
   if (rc) return rc;
   ListArgs lw = la;
   lw.out_cap = c->graph_cap;
@@ -2219,7 +2282,7 @@ static int enqueue_graph_body(tf_ctx* c, const double* dP, double* dJ, double* d
     }
   }
   TF_CUDA(branches.join());
-  return enqueue_finalize(c, dJ, dK, dJb, dKb, kernels);
+  return enqueue_finalize(c, io.J[0], io.K[0], io.J[1], io.K[1], kernels, &rec);
 }
 
 // Statistics of the finished build from the pinned read-backs and the events.
@@ -2316,14 +2379,17 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
     }
   }
   // graph path: once a dynamic build has sized the list buffer and set up every
-  // launch, later builds with the same arrays replay one captured graph
+  // launch, later builds of its kind replay one captured graph, whatever their arrays
   if (c->use_graph && c->graph_cap > 0) {
-    const bool same = c->graph_exec && c->graph_key_P == dP && c->graph_key_J == dJ && c->graph_key_K == dK &&
-                      c->graph_key_Pb == dPb && c->graph_key_Jb == dJb && c->graph_key_Kb == dKb &&
-                      c->graph_key_mixed == mixed && c->graph_key_cutoff == c->opt.eri_schwarz_cutoff &&
-                      c->graph_key_want == want && c->graph_key_mol_cut == c->use_mol_cut;
-    if (!same) {
-      drop_graph(c);
+    BuildGraph& G = c->graphs[dPb ? 1 : 0];
+    BuildIO io;
+    io.P[0] = dP; io.J[0] = dJ; io.K[0] = dK;
+    if (dPb) { io.P[1] = dPb; io.J[1] = dJb; io.K[1] = dKb; }
+    const bool same = G.exec && G.mixed == mixed && G.cutoff == c->opt.eri_schwarz_cutoff && G.want == want &&
+                      G.mol_cut == c->use_mol_cut;
+    if (!same || (!(G.io == io) && G.set_io(io) != cudaSuccess)) {
+      cudaGetLastError();
+      G.drop();
       for (int g = 0; g < ng; ++g) {         // launch set-up of every class, outside the capture
         int l1h, l1l, l2h, l2l;
         class_l(c->group_cls[g].x, l1h, l1l);
@@ -2340,31 +2406,30 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
         }
       }
       TF_TRY_RC(default_schedule(c, nullptr));
-      int kernels = 0;
-      cudaGraph_t graph = nullptr;
       TF_CUDA(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-      int rc = enqueue_graph_body(c, dP, dJ, dK, dPb, dJb, dKb, mixed, want, kernels);
-      cudaError_t ce = cudaStreamEndCapture(s, &graph);
-      if (rc != TF_OK) { if (graph) cudaGraphDestroy(graph); return rc; }
-      if (ce != cudaSuccess) { set_error(cudaGetErrorString(ce)); return TF_ECUDA; }
-      ce = cudaGraphInstantiate(&c->graph_exec, graph, 0);
-      cudaGraphDestroy(graph);
-      if (ce != cudaSuccess) { c->graph_exec = nullptr; set_error(cudaGetErrorString(ce)); return TF_ECUDA; }
-      c->graph_key_P = dP; c->graph_key_J = dJ; c->graph_key_K = dK;
-      c->graph_key_Pb = dPb; c->graph_key_Jb = dJb; c->graph_key_Kb = dKb;
-      c->graph_key_mixed = mixed;
-      c->graph_key_cutoff = c->opt.eri_schwarz_cutoff;
-      c->graph_key_want = want;
-      c->graph_key_mol_cut = c->use_mol_cut;
-      c->graph_kernels = kernels;
+      int rc = enqueue_graph_body(c, io, mixed, want, G);
+      cudaError_t ce = cudaStreamEndCapture(s, &G.graph);
+      if (rc == TF_OK && ce == cudaSuccess) ce = cudaGraphInstantiate(&G.exec, G.graph, 0);
+      if (rc == TF_OK && ce != cudaSuccess) { set_error(cudaGetErrorString(ce)); rc = TF_ECUDA; }
+      if (rc != TF_OK) {
+        cudaGetLastError();
+        if (ce != cudaSuccess) G.exec = nullptr;
+        G.drop();
+        return rc;
+      }
+      G.io = io;
+      G.mixed = mixed;
+      G.cutoff = c->opt.eri_schwarz_cutoff;
+      G.want = want;
+      G.mol_cut = c->use_mol_cut;
     }
     TF_CUDA(cudaEventRecord(c->ev0, s));
-    TF_CUDA(cudaGraphLaunch(c->graph_exec, s));
+    TF_CUDA(cudaGraphLaunch(G.exec, s));
     TF_CUDA(cudaEventRecord(c->ev2, s));
     TF_CUDA(cudaStreamSynchronize(s));
     const long long total = c->pin->goff[3 * ng];
-    if (total <= c->graph_cap) return finish_stats(c, c->graph_kernels, true);
-    drop_graph(c);                          // list outgrew the buffer: redo this build dynamically
+    if (total <= c->graph_cap) return finish_stats(c, G.kernels, true);
+    drop_graph(c);                          // the list outgrew the buffer: redo this build dynamically
   }
   int kernels = 0;
   TF_CUDA(cudaEventRecord(c->ev0, s));
