@@ -1101,6 +1101,7 @@ struct BuildGraph {
   int want = 3;
   double cutoff = 0.0;
   int kernels = 0;
+  std::vector<long long> expect[2];            // per class: FP64 and FP32 entries its launches were chosen for
 
   void drop() {
     if (exec) cudaGraphExecDestroy(exec);
@@ -1145,6 +1146,33 @@ cudaError_t BuildGraph::set_io(const BuildIO& to) {
   const cudaError_t e = set_pointers(exec, pmax, 6, 1, {to.P[0], to.P[1]});          // k_pmax
   if (e == cudaSuccess) io = to;
   return e;
+}
+
+// Longest lists (contracted quartets per class, FP64 and FP32 halves) and most primitive
+// quartets that the context's FP64 and mixed builds have had.  A captured build is launched
+// for these, not for the build before it, which may have been of another kind: after the
+// short lists of a density change, (H2O)5 cc-pVTZ full builds took 6.7 ms on the kernels for
+// short lists instead of 6.1, after a nearly empty build 7.5.
+struct ListMarks {
+  bool any = false;
+  std::vector<long long> n[2] = {std::vector<long long>(NQCLS, 0), std::vector<long long>(NQCLS, 0)};
+  std::vector<double> prim = std::vector<double>(NQCLS, 0.0);
+
+  void add(const unsigned long long* pc) {
+    any = true;
+    for (int k = 0; k < NQCLS; ++k) {
+      for (int h = 0; h < 2; ++h) n[h][k] = std::max(n[h][k], (long long)pc[(1 + h) * NQCLS + 1 + k]);
+      prim[k] = std::max(prim[k], (double)pc[k]);
+    }
+  }
+};
+
+// Expected FP64 (half 0) or FP32 (half 1) entries of class k in a build of the given kind;
+// marks: FP64 builds', mixed builds'.  Before the first mixed build either half may hold all.
+static long long expected_entries(const ListMarks (&marks)[2], bool mixed, int half, int k) {
+  if (mixed && marks[1].any) return marks[1].n[half][k];
+  const long long all = std::max(marks[0].n[0][k], marks[1].n[0][k] + marks[1].n[1][k]);
+  return mixed || half == 0 ? all : 0;
 }
 
 }  // namespace tf
@@ -1227,6 +1255,7 @@ struct tf_ctx {
   bool use_graph = true;
   long long graph_cap = 0;                               // list entries a captured build may use
   tf::BuildGraph graphs[2];                              // restricted, unrestricted
+  tf::ListMarks marks[2];                                // FP64 builds, mixed builds
   // class schedule: graph branches and the branch of each class pair, set by the
   // autotuner or, until it has run, at each capture (default_schedule)
   bool sched_tuned = false;
@@ -2188,21 +2217,19 @@ static int enqueue_finalize(tf_ctx* c, double* dJ, double* dK, double* dJb, doub
 // Class schedule of a build that no autotuner has chosen one for: the class pairs over
 // DEFAULT_BRANCHES branches, longest first, each to the least-loaded branch, by the FLOP
 // model at the given list lengths (goff: start, FP32 start and end per group) with eight
-// primitive quartets per entry, or, goff null, at the counts of the last build.
+// primitive quartets per entry, or, goff null, at the marks of the builds so far.
 static int default_schedule(tf_ctx* c, const long long* goff) {
   if (c->sched_tuned) return TF_OK;
   TF_TRY_RC(ensure_branches(c, DEFAULT_BRANCHES));
   const int ng = (int)c->group_cls.size();
-  const unsigned long long* pc = c->pin->pc;
   std::vector<double> cost(ng, 1.0);
   for (int g = 0; g < ng; ++g) {
     int l1h, l1l, l2h, l2l;
     class_l(c->group_cls[g].x, l1h, l1l);
     class_l(c->group_cls[g].y, l2h, l2l);
     const int cid = qclass_id(l1h, l1l, l2h, l2l);
-    const double nq = goff ? (double)(goff[3 * g + 2] - goff[3 * g])
-                           : (double)pc[NQCLS + 1 + cid] + (double)pc[2 * NQCLS + 1 + cid];
-    cost[g] += class_flops(l1h, l1l, l2h, l2l, nq, goff ? 8.0 * nq : (double)pc[cid]);
+    const double nq = goff ? (double)(goff[3 * g + 2] - goff[3 * g]) : (double)expected_entries(c->marks, false, 0, cid);
+    cost[g] += class_flops(l1h, l1l, l2h, l2l, nq, goff ? 8.0 * nq : std::max(c->marks[0].prim[cid], c->marks[1].prim[cid]));
   }
   std::vector<int> order(ng);
   std::iota(order.begin(), order.end(), 0);
@@ -2269,9 +2296,9 @@ static int enqueue_graph_body(tf_ctx* c, const BuildIO& io, bool mixed, int want
     a32.plan = c->d_plans.p + 2 * g + 1;
     a32.range = c->d_group_offsets.p + 3 * g + 1;
     a32.bucket32 = 1;
-    const int cid = qclass_id(l1h, l1l, l2h, l2l);           // the last build's counts
-    a.expect = (long long)c->pin->pc[NQCLS + 1 + cid];
-    a32.expect = (long long)c->pin->pc[2 * NQCLS + 1 + cid];
+    const int cid = qclass_id(l1h, l1l, l2h, l2l);
+    a.expect = rec.expect[0][cid];
+    a32.expect = rec.expect[1][cid];
     rc = dispatch_jk(l1h, l1l, l2h, l2l, a, sg, false, jk_variant(c, g));
     if (rc != TF_OK) return rc;
     kernels++;
@@ -2285,8 +2312,20 @@ static int enqueue_graph_body(tf_ctx* c, const BuildIO& io, bool mixed, int want
   return enqueue_finalize(c, io.J[0], io.K[0], io.J[1], io.K[1], kernels, &rec);
 }
 
+// Whether a class's list was more than twice as long as its captured launches were chosen for
+// (below two thousand entries both kinds of kernel take tens of microseconds): the next
+// build captures anew, for the marks that this one left.  Lists that became shorter keep
+// the kernels for long ones, which cost a few per cent there, and a context that
+// alternates full builds and changes does not capture each time.
+static bool outgrown(const BuildGraph& G, const unsigned long long* pc) {
+  for (int h = 0; h < 2; ++h)
+    for (int k = 0; k < NQCLS; ++k)
+      if ((long long)pc[(1 + h) * NQCLS + 1 + k] > 2 * std::max<long long>(G.expect[h][k], 1024)) return true;
+  return false;
+}
+
 // Statistics of the finished build from the pinned read-backs and the events.
-static int finish_stats(tf_ctx* c, int kernels, bool graph, bool timed = false) {
+static int finish_stats(tf_ctx* c, int kernels, bool mixed, bool graph, bool timed = false) {
   const int ng = (int)c->group_cls.size();
   const long long* goff = c->pin->goff;
   const unsigned long long* pc = c->pin->pc;
@@ -2294,6 +2333,7 @@ static int finish_stats(tf_ctx* c, int kernels, bool graph, bool timed = false) 
     set_error("the density has non-finite elements (NaN or infinity)");
     return TF_EINVAL;
   }
+  c->marks[mixed ? 1 : 0].add(pc);
   float ms_all = 0.f, ms_eri = 0.f;
   TF_CUDA(cudaEventElapsedTime(&ms_all, c->ev0, c->ev2));
   double npq = 0.0, flops = 0.0, n_all = 0.0, n_fp32 = 0.0;
@@ -2390,6 +2430,10 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
     if (!same || (!(G.io == io) && G.set_io(io) != cudaSuccess)) {
       cudaGetLastError();
       G.drop();
+      for (int h = 0; h < 2; ++h) {
+        G.expect[h].resize(NQCLS);
+        for (int k = 0; k < NQCLS; ++k) G.expect[h][k] = expected_entries(c->marks, mixed, h, k);
+      }
       for (int g = 0; g < ng; ++g) {         // launch set-up of every class, outside the capture
         int l1h, l1l, l2h, l2l;
         class_l(c->group_cls[g].x, l1h, l1l);
@@ -2400,7 +2444,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
         if (c->group_task0[g + 1] == c->group_task0[g]) continue;
         const int cid = qclass_id(l1h, l1l, l2h, l2l);
         for (int fp32 = 0; fp32 <= (mixed ? 1 : 0); ++fp32) {   // the kernels the capture will launch, as
-          none.expect = (long long)c->pin->pc[(1 + fp32) * NQCLS + 1 + cid];   // each costs a first load
+          none.expect = G.expect[fp32][cid];                    // each costs a first load
           const int rc = dispatch_jk(l1h, l1l, l2h, l2l, none, s, fp32 != 0, jk_variant(c, g));
           if (rc != TF_OK) return rc;
         }
@@ -2428,7 +2472,11 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
     TF_CUDA(cudaEventRecord(c->ev2, s));
     TF_CUDA(cudaStreamSynchronize(s));
     const long long total = c->pin->goff[3 * ng];
-    if (total <= c->graph_cap) return finish_stats(c, G.kernels, true);
+    if (total <= c->graph_cap) {
+      const int rc = finish_stats(c, G.kernels, mixed, true);
+      if (rc == TF_OK && outgrown(G, c->pin->pc)) G.drop();
+      return rc;
+    }
     drop_graph(c);                          // the list outgrew the buffer: redo this build dynamically
   }
   int kernels = 0;
@@ -2550,7 +2598,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
   if (rc) return rc;
   TF_CUDA(cudaEventRecord(c->ev2, s));
   TF_CUDA(cudaStreamSynchronize(s));
-  return finish_stats(c, kernels, false, timed);
+  return finish_stats(c, kernels, mixed, false, timed);
 }
 
 // Checks of one molecule's basis description, made before any device call: every
@@ -2963,6 +3011,7 @@ int tf_set_shard(tf_ctx* c, int index, int count) {
   if (rc) return rc;
   c->shard_index = index;
   c->shard_count = count;
+  for (ListMarks& m : c->marks) m = ListMarks{};   // another share of the tasks: other lists
   return c->geometry_ready ? build_tasks(c) : TF_OK;
 }
 
