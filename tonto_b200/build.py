@@ -3,6 +3,13 @@
     python -m tonto_b200.build
 
 The library is written next to this file so that it travels with the source tree.
+
+A process loads a source's kernels when it first launches one of them, in time that goes with
+their size: with line tables the library unpacks to 177 MB, without to 53 MB.  So line tables
+are built in only when asked for (TF_LINEINFO=1 with --force, for a profile by source line),
+and the kernels are stored unpacked.  Measured in fresh processes, median ms of context
+creation and first build, line tables (packed) -> neither: (H2O)2 cc-pVDZ 17.3 + 83.8 ->
+8.0 + 15.6; minima for (H2O)2 STO-3G 61 -> 17, (H2O)2 cc-pVTZ 139 -> 35.
 """
 
 from __future__ import annotations
@@ -22,7 +29,7 @@ PEAK_LIB = os.path.join(HERE, "libtf_peak.so")
 SOURCES = ["tontofock.cu", "tf_jk_ss.cu", "tf_jk_ps.cu", "tf_jk_d.cu", "tf_jk_f.cu", "tf_jk_l.cu", "tf_jk_l2.cu", "tf_rows_d.cu",
            "tf_rows_fs.cu", "tf_rows_fd.cu", "tf_rows_ff.cu", "tf_mlp.cu"]
 DEPS = SOURCES + ["tf_device.cuh", "tf_thread.cuh", "tf_rows.cuh", "tf_warp.cuh", "tf_host.h", "rys_tables.inc", "boys_table.inc", "boys2_table.inc",
-        os.path.join("..", "..", "include", "tontofock.h"), os.path.join("..", "..", "include", "tontofock_guess.h")]
+        os.path.join("..", "build.py"), os.path.join("..", "..", "include", "tontofock.h"), os.path.join("..", "..", "include", "tontofock_guess.h")]
 
 
 def nvcc() -> str:
@@ -33,7 +40,8 @@ def nvcc() -> str:
 
 
 def flags() -> list:
-    return ["-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
+    lineinfo = ["-lineinfo"] if os.environ.get("TF_LINEINFO", "0") != "0" else []
+    return ["-gencode", "arch=compute_100a,code=sm_100a", *lineinfo, "--compress-mode=none", "-O3", "-std=c++17",
             "--expt-relaxed-constexpr", "-Xcompiler", "-fPIC", "-shared"]
 
 
