@@ -117,8 +117,8 @@ typedef struct tf_class_stats {
   int l[4];                          /* la >= lb, lc >= ld, pair class (la lb) >= (lc ld) */
   double quartets, prim_quartets;    /* contracted and primitive quartets computed */
   double flops;                      /* algorithmic FLOPs */
-  double ms;                         /* device time of the launch (CUDA events; 0 unless tf_set_graph
-                                        is off: only then do the launches follow one another) */
+  double ms;                         /* device time of the launch (CUDA events; 0 for graph builds).
+                                        Launches of direct builds overlap unless tf_set_graph is off */
 } tf_class_stats;
 
 typedef struct tf_ctx tf_ctx;

@@ -2324,8 +2324,11 @@ static bool outgrown(const BuildGraph& G, const unsigned long long* pc) {
   return false;
 }
 
-// Statistics of the finished build from the pinned read-backs and the events.
-static int finish_stats(tf_ctx* c, int kernels, bool mixed, bool graph, bool timed = false) {
+// Statistics of the finished build from the pinned read-backs and the events.  chunk: the
+// class pairs at which a direct build's chunks start and the last one ends (null: a graph);
+// overlap: its class launches ran on several branches.
+static int finish_stats(tf_ctx* c, int kernels, bool mixed, const std::vector<int>* chunk = nullptr,
+                        bool overlap = false) {
   const int ng = (int)c->group_cls.size();
   const long long* goff = c->pin->goff;
   const unsigned long long* pc = c->pin->pc;
@@ -2334,7 +2337,8 @@ static int finish_stats(tf_ctx* c, int kernels, bool mixed, bool graph, bool tim
     return TF_EINVAL;
   }
   c->marks[mixed ? 1 : 0].add(pc);
-  float ms_all = 0.f, ms_eri = 0.f;
+  float ms_all = 0.f, ms_eri = 0.f, lo = 0.f, hi = 0.f;
+  int chunk_end = 0;
   TF_CUDA(cudaEventElapsedTime(&ms_all, c->ev0, c->ev2));
   double npq = 0.0, flops = 0.0, n_all = 0.0, n_fp32 = 0.0;
   c->cls_stats.clear();
@@ -2353,10 +2357,23 @@ static int finish_stats(tf_ctx* c, int kernels, bool mixed, bool graph, bool tim
     npq += p;
     const double fl = class_flops(l1h, l1l, l2h, l2l, (double)nq, p);
     flops += fl;
-    float ms = 0.f;                       // per-class device time: class-by-class builds only
-    if (timed) {
+    float ms = 0.f;                       // per-class device time: direct builds only
+    if (chunk) {
       TF_CUDA(cudaEventElapsedTime(&ms, c->cls_ev[2 * g], c->cls_ev[2 * g + 1]));
-      ms_eri += ms;
+      if (overlap) {                      // the time of a chunk's launches: first start to last end
+        float start = 0.f;
+        TF_CUDA(cudaEventElapsedTime(&start, c->ev0, c->cls_ev[2 * g]));
+        if (g >= chunk_end) {
+          ms_eri += hi - lo;
+          lo = start;
+          hi = start;
+          chunk_end = *std::upper_bound(chunk->begin(), chunk->end() - 1, g);
+        }
+        lo = std::min(lo, start);
+        hi = std::max(hi, start + ms);
+      } else {
+        ms_eri += ms;
+      }
     }
     tf_class_stats cs;
     cs.l[0] = l1h; cs.l[1] = l1l; cs.l[2] = l2h; cs.l[3] = l2l;
@@ -2367,13 +2384,13 @@ static int finish_stats(tf_ctx* c, int kernels, bool mixed, bool graph, bool tim
     c->cls_stats.push_back(cs);
   }
   c->stats.build_ms = ms_all;
-  c->stats.eri_ms = timed ? ms_eri : ms_all;
+  c->stats.eri_ms = chunk ? ms_eri + (hi - lo) : ms_all;
   c->stats.quartets = n_all;
   c->stats.quartets_fp32 = n_fp32;
   c->stats.prim_quartets = npq;
   c->stats.flops = flops;
   c->stats.kernels = kernels;
-  c->stats.graph = graph ? 1 : 0;
+  c->stats.graph = chunk ? 0 : 1;
   return TF_OK;
 }
 
@@ -2473,7 +2490,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
     TF_CUDA(cudaStreamSynchronize(s));
     const long long total = c->pin->goff[3 * ng];
     if (total <= c->graph_cap) {
-      const int rc = finish_stats(c, G.kernels, mixed, true);
+      const int rc = finish_stats(c, G.kernels, mixed);
       if (rc == TF_OK && outgrown(G, c->pin->pc)) G.drop();
       return rc;
     }
@@ -2533,11 +2550,10 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
     drop_graph(c);
     c->graph_cap = 0;
   }
-  // class-by-class builds proper (tf_set_graph 0) time each class pair's launches, so
+  // class-by-class builds proper (tf_set_graph 0) time each class pair's launches by itself, so
   // these follow one another; a build that only stands in for a graph build overlaps them
-  const bool timed = !c->use_graph;
-  if (!timed) TF_TRY_RC(default_schedule(c, goff.data()));
-  const int ns = timed ? 1 : sched_branches(c);
+  if (c->use_graph) TF_TRY_RC(default_schedule(c, goff.data()));
+  const int ns = c->use_graph ? sched_branches(c) : 1;
   for (size_t ci = 0; ci + 1 < chunk.size(); ++ci) {
     const int g0 = chunk[ci], g1 = chunk[ci + 1];
     const long long base = goff[3 * g0], nq = goff[3 * (g1 - 1) + 2] - base;
@@ -2560,7 +2576,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
       class_l(c->group_cls[g].x, l1h, l1l);
       class_l(c->group_cls[g].y, l2h, l2l);
       const cudaStream_t sg = branch_of(c, g, ns);
-      if (timed) TF_CUDA(cudaEventRecord(c->cls_ev[2 * g], s));
+      TF_CUDA(cudaEventRecord(c->cls_ev[2 * g], sg));
       JKArgs a{c->d_quartets.p, goff[3 * g + 1] - goff[3 * g], c->d_pairs.p,
                c->d_prim_full.p, c->d_prim_skip.p, c->d_Pc.p, c->d_Jc.p, c->d_Kc.p, c->d_mols.p,
                c->d_prim_count.p, c->d_plans.p + 2 * g, nullptr, base, LLONG_MAX, goff[3 * g], c->d_jkrec.p,
@@ -2589,7 +2605,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
         if (rc != TF_OK) return rc;
         kernels++;
       }
-      if (timed) TF_CUDA(cudaEventRecord(c->cls_ev[2 * g + 1], s));
+      TF_CUDA(cudaEventRecord(c->cls_ev[2 * g + 1], sg));
     }
     TF_CUDA(branches.join());
   }
@@ -2598,7 +2614,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
   if (rc) return rc;
   TF_CUDA(cudaEventRecord(c->ev2, s));
   TF_CUDA(cudaStreamSynchronize(s));
-  return finish_stats(c, kernels, mixed, false, timed);
+  return finish_stats(c, kernels, mixed, &chunk, ns > 1);
 }
 
 // Checks of one molecule's basis description, made before any device call: every
