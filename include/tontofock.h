@@ -206,7 +206,7 @@ typedef struct tf_tune {
   int candidates;                    /* schedules timed (1 .. max_streams branches) */
   double ms[8];                      /* best graph build time of each candidate */
   double direct_ms;                  /* the class-by-class build used for the class times */
-  int variant_classes;               /* class pairs whose kernel runs a variant other than the default */
+  int variant_classes;               /* class pairs whose kernel runs a variant other than 0 */
 } tf_tune;
 
 /* Autotuner for the kernels and the class schedule of graph builds.  It first waits
@@ -228,7 +228,8 @@ int tf_autotune(tf_ctx* ctx, const double* dP, double* dJ, double* dK, int flags
 
 /* Run every class pair's thread kernel in one variant (0 .. 3, as tf_autotune
  * numbers them: bit 0 more resident warps, bit 1 exchange atomics summed over lanes
- * first) until the next tf_autotune or tf_set_kernel_variant.  A deterministic
+ * first) until the next tf_autotune or tf_set_kernel_variant.  The classes beyond
+ * (dd|ss), (dp|ps), (ds|pp) and (ds|ds) have one kernel each, in every variant.  A deterministic
  * context always sums over lanes first (bit 1), whatever the variant.
  * Results do not depend on it beyond summation order (deterministic contexts: not at
  * all).  No reference counterpart. */

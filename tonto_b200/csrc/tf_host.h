@@ -59,6 +59,12 @@ class BranchFork {
   int forked_ = 0;                     // side branches that wait for the context's stream and are not joined yet
 };
 
+// Whether a class (la lb|lc ld) has kernel variants to choose from: the thread kernels of up to
+// d shells (launch_jk).  The others run one kernel whatever the variant's lower bits.
+constexpr bool has_variants(int la, int lb, int lc, int ld) {
+  return la <= 2 && (lc + ld == 0 || (lc + ld == 1 && la + lb <= 3) || (lc + ld == 2 && la == 2 && lb == 0));
+}
+
 // A value per device, made at the first use on that device: a kernel's launch set-up, which
 // holds for one device (function attributes are per device), not for the process.  Several
 // threads may ask at once; a value is seen only when it is complete.

@@ -2958,9 +2958,13 @@ int tf_autotune(tf_ctx* c, const double* dP, double* dJ, double* dK, int flags, 
     }
   }
   for (int g = 0; g < ng; ++g) {
+    int l1h, l1l, l2h, l2l;
+    class_l(c->group_cls[g].x, l1h, l1l);
+    class_l(c->group_cls[g].y, l2h, l2l);
     int best_v = 0;
-    for (int v = 1; v < JK_VARIANTS; ++v)
-      if (tv[v][g] < tv[best_v][g] * 0.98) best_v = v;
+    if (has_variants(l1h, l1l, l2h, l2l))
+      for (int v = 1; v < JK_VARIANTS; ++v)
+        if (tv[v][g] < tv[best_v][g] * 0.98) best_v = v;
     c->cls_variant[g] = best_v;
     if (best_v) res.variant_classes++;
   }
