@@ -1158,12 +1158,10 @@ struct ListMarks {
   std::vector<long long> n[2] = {std::vector<long long>(NQCLS, 0), std::vector<long long>(NQCLS, 0)};
   std::vector<double> prim = std::vector<double>(NQCLS, 0.0);
 
-  void add(const unsigned long long* pc) {
+  void add(const unsigned long long* pc, int k) {
     any = true;
-    for (int k = 0; k < NQCLS; ++k) {
-      for (int h = 0; h < 2; ++h) n[h][k] = std::max(n[h][k], (long long)pc[(1 + h) * NQCLS + 1 + k]);
-      prim[k] = std::max(prim[k], (double)pc[k]);
-    }
+    for (int h = 0; h < 2; ++h) n[h][k] = std::max(n[h][k], (long long)pc[(1 + h) * NQCLS + 1 + k]);
+    prim[k] = std::max(prim[k], (double)pc[k]);
   }
 };
 
@@ -1249,6 +1247,10 @@ struct tf_ctx {
   tf::DBuf<unsigned char> d_scan_tmp;
   std::vector<cudaEvent_t> cls_ev;                       // start and end of each group's launches
   std::vector<tf_class_stats> cls_stats;
+  // a direct build's device times, read from its events when they are asked for: the group of
+  // every entry of cls_stats, the end of its chunk, and whether the launches overlapped
+  bool times_pending = false, times_overlap = false;
+  std::vector<int> times_group, times_chunk_end;
   std::vector<double> max_I_tonto;                       // per molecule, Tonto pair order
   tf_stats stats{};
   // graph builds
@@ -2317,10 +2319,16 @@ static int enqueue_graph_body(tf_ctx* c, const BuildIO& io, bool mixed, int want
 // build captures anew, for the marks that this one left.  Lists that became shorter keep
 // the kernels for long ones, which cost a few per cent there, and a context that
 // alternates full builds and changes does not capture each time.
-static bool outgrown(const BuildGraph& G, const unsigned long long* pc) {
-  for (int h = 0; h < 2; ++h)
-    for (int k = 0; k < NQCLS; ++k)
+static bool outgrown(const tf_ctx* c, const BuildGraph& G) {
+  const unsigned long long* pc = c->pin->pc;
+  for (const int2& cls : c->group_cls) {
+    int l1h, l1l, l2h, l2l;
+    class_l(cls.x, l1h, l1l);
+    class_l(cls.y, l2h, l2l);
+    const int k = qclass_id(l1h, l1l, l2h, l2l);
+    for (int h = 0; h < 2; ++h)
       if ((long long)pc[(1 + h) * NQCLS + 1 + k] > 2 * std::max<long long>(G.expect[h][k], 1024)) return true;
+  }
   return false;
 }
 
@@ -2336,12 +2344,14 @@ static int finish_stats(tf_ctx* c, int kernels, bool mixed, const std::vector<in
     set_error("the density has non-finite elements (NaN or infinity)");
     return TF_EINVAL;
   }
-  c->marks[mixed ? 1 : 0].add(pc);
-  float ms_all = 0.f, ms_eri = 0.f, lo = 0.f, hi = 0.f;
-  int chunk_end = 0;
+  float ms_all = 0.f;
   TF_CUDA(cudaEventElapsedTime(&ms_all, c->ev0, c->ev2));
   double npq = 0.0, flops = 0.0, n_all = 0.0, n_fp32 = 0.0;
   c->cls_stats.clear();
+  c->times_group.clear();
+  c->times_chunk_end.clear();
+  c->times_pending = chunk != nullptr;
+  c->times_overlap = overlap;
   const unsigned long long* q64 = pc + NQCLS + 1;        // contracted (member) quartets per class
   const unsigned long long* q32 = q64 + NQCLS;
   for (int g = 0; g < ng; ++g) {
@@ -2350,6 +2360,7 @@ static int finish_stats(tf_ctx* c, int kernels, bool mixed, const std::vector<in
     class_l(c->group_cls[g].x, l1h, l1l);
     class_l(c->group_cls[g].y, l2h, l2l);
     const int cid = qclass_id(l1h, l1l, l2h, l2l);
+    c->marks[mixed ? 1 : 0].add(pc, cid);
     const double nq = (double)q64[cid] + (double)q32[cid];
     n_all += nq;
     n_fp32 += (double)q32[cid];
@@ -2357,34 +2368,20 @@ static int finish_stats(tf_ctx* c, int kernels, bool mixed, const std::vector<in
     npq += p;
     const double fl = class_flops(l1h, l1l, l2h, l2l, (double)nq, p);
     flops += fl;
-    float ms = 0.f;                       // per-class device time: direct builds only
     if (chunk) {
-      TF_CUDA(cudaEventElapsedTime(&ms, c->cls_ev[2 * g], c->cls_ev[2 * g + 1]));
-      if (overlap) {                      // the time of a chunk's launches: first start to last end
-        float start = 0.f;
-        TF_CUDA(cudaEventElapsedTime(&start, c->ev0, c->cls_ev[2 * g]));
-        if (g >= chunk_end) {
-          ms_eri += hi - lo;
-          lo = start;
-          hi = start;
-          chunk_end = *std::upper_bound(chunk->begin(), chunk->end() - 1, g);
-        }
-        lo = std::min(lo, start);
-        hi = std::max(hi, start + ms);
-      } else {
-        ms_eri += ms;
-      }
+      c->times_group.push_back(g);
+      c->times_chunk_end.push_back(*std::upper_bound(chunk->begin(), chunk->end() - 1, g));
     }
     tf_class_stats cs;
     cs.l[0] = l1h; cs.l[1] = l1l; cs.l[2] = l2h; cs.l[3] = l2l;
     cs.quartets = (double)nq;
     cs.prim_quartets = p;
     cs.flops = fl;
-    cs.ms = ms;
+    cs.ms = 0.0;
     c->cls_stats.push_back(cs);
   }
   c->stats.build_ms = ms_all;
-  c->stats.eri_ms = chunk ? ms_eri + (hi - lo) : ms_all;
+  c->stats.eri_ms = chunk ? 0.0 : ms_all;
   c->stats.quartets = n_all;
   c->stats.quartets_fp32 = n_fp32;
   c->stats.prim_quartets = npq;
@@ -2392,6 +2389,38 @@ static int finish_stats(tf_ctx* c, int kernels, bool mixed, const std::vector<in
   c->stats.kernels = kernels;
   c->stats.graph = chunk ? 0 : 1;
   return TF_OK;
+}
+
+// Per-class device times of the last direct build and their sum or, where launches overlapped,
+// the time from a chunk's first start to its last end, summed over the chunks.
+static void resolve_times(tf_ctx* c) {
+  if (!c->times_pending) return;
+  c->times_pending = false;
+  double sum = 0.0;
+  float lo = 0.f, hi = 0.f;
+  int chunk_end = 0;
+  for (size_t i = 0; i < c->cls_stats.size(); ++i) {
+    const int g = c->times_group[i];
+    float ms = 0.f, start = 0.f;
+    if (cudaEventElapsedTime(&ms, c->cls_ev[2 * g], c->cls_ev[2 * g + 1]) != cudaSuccess ||
+        cudaEventElapsedTime(&start, c->ev0, c->cls_ev[2 * g]) != cudaSuccess) {
+      cudaGetLastError();
+      continue;
+    }
+    c->cls_stats[i].ms = ms;
+    if (!c->times_overlap) {
+      sum += ms;
+      continue;
+    }
+    if (g >= chunk_end) {
+      sum += hi - lo;
+      lo = hi = start;
+      chunk_end = c->times_chunk_end[i];
+    }
+    lo = std::min(lo, start);
+    hi = std::max(hi, start + ms);
+  }
+  c->stats.eri_ms = sum + (hi - lo);
 }
 
 // One J/K build for every molecule of the context: dP, dJ, dK are the
@@ -2484,6 +2513,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
       G.want = want;
       G.mol_cut = c->use_mol_cut;
     }
+    c->times_pending = false;              // (ev0 is recorded anew)
     TF_CUDA(cudaEventRecord(c->ev0, s));
     TF_CUDA(cudaGraphLaunch(G.exec, s));
     TF_CUDA(cudaEventRecord(c->ev2, s));
@@ -2491,12 +2521,13 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
     const long long total = c->pin->goff[3 * ng];
     if (total <= c->graph_cap) {
       const int rc = finish_stats(c, G.kernels, mixed);
-      if (rc == TF_OK && outgrown(G, c->pin->pc)) G.drop();
+      if (rc == TF_OK && outgrown(c, G)) G.drop();
       return rc;
     }
     drop_graph(c);                          // the list outgrew the buffer: redo this build dynamically
   }
   int kernels = 0;
+  c->times_pending = false;              // the events are recorded anew
   TF_CUDA(cudaEventRecord(c->ev0, s));
   ListArgs la;
   int rc = enqueue_counts(c, dP, dPb, mixed, LLONG_MAX, la, kernels);
@@ -3458,12 +3489,14 @@ int tf_one_electron_noalloc(const tf_basis* B, const double* Z, double* dS, doub
 
 int tf_last_stats(const tf_ctx* c, tf_stats* s) {
   if (!c || !s) return TF_EINVAL;
+  tf::resolve_times(const_cast<tf_ctx*>(c));
   *s = c->stats;
   return TF_OK;
 }
 
 int tf_last_class_stats(const tf_ctx* c, tf_class_stats* out, int max) {
   if (!c || (!out && max > 0)) return TF_EINVAL;
+  tf::resolve_times(const_cast<tf_ctx*>(c));
   const int n = (int)c->cls_stats.size();
   for (int i = 0; i < n && i < max; ++i) out[i] = c->cls_stats[i];
   return n;
