@@ -1,5 +1,5 @@
 // tf_rows.cuh — lane-group quartets for the classes whose (e0|f0) block does not fit one
-// thread: the ket pairs beyond the thread kernels of tontofock.cu (pp, dp, dd, and
+// thread: the ket pairs beyond the thread kernels of tf_thread.cuh (pp, dp, dd, and
 // every class with an f shell except those whose ket block is small).
 //
 // A group of lanes computes one contracted quartet: NF <= 32 lanes (the ket's (f0|

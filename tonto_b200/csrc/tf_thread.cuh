@@ -9,7 +9,7 @@
 
 namespace tf {
 
-constexpr int LMAX_SUPPORTED = 3;                 // s, p, d, f shells (f: the warp path)
+constexpr int LMAX_SUPPORTED = 3;                 // s, p, d, f shells
 constexpr int NPAIRCLS = (LMAX_SUPPORTED + 1) * (LMAX_SUPPORTED + 2) / 2;
 constexpr int NQCLS = 625;                        // (la lb lc ld) counter slots, l <= 4
 // Counters of a build, zeroed with it and read back after it: primitive quartets per
@@ -19,12 +19,13 @@ constexpr int BUILD_COUNTERS = 3 * NQCLS + 1;
 __host__ __device__ constexpr int pair_class(int lh, int ll) { return lh * (lh + 1) / 2 + ll; }
 __host__ __device__ constexpr int qclass_id(int la, int lb, int lc, int ld) { return ((la * 5 + lb) * 5 + lc) * 5 + ld; }
 // Bra-family members the thread kernel of a class holds at once (accumulator
-// capacity), for the classes where evaluating a bra family's primitive quartets once
-// measured faster on (H2O)32 cc-pVDZ: (ss|ss) 9.36 -> 8.36 ms, (ds|ss) 3.87 -> 3.63 ms.
-// (ps|ss), (ps|ps) and (ds|ps) measured slower with it (13.33 -> 13.45, 8.55 -> 8.90
-// and 4.29 -> 5.63 ms: the extra accumulators cost registers and the coefficient
-// loads and products every primitive quartet, and few of their bras are families),
-// so they, like every other class, take one member per list entry (capacity 1).
+// capacity), for the classes that evaluate a bra family's primitive quartets once.
+// Measured on (H2O)32 cc-pVDZ, one member per entry -> families: (ss|ss) 7.65 -> 7.21 ms,
+// (ds|ss) 2.72 -> 2.84, the build 56.65 -> 56.43.  With capacity 2 (ps|ss), (ps|ps) and
+// (ds|ps) are slower (10.2 -> 11.2, 6.4 -> 7.5 and 4.1 -> 6.1 ms: the extra accumulators
+// cost registers, the coefficient loads and products every primitive quartet, and few of
+// their bras are families), so they, like every other class, take one member per list
+// entry (capacity 1).
 __host__ __device__ constexpr int fam_cap_l(int la, int lb, int lc, int ld) {
   return (la == 0 && lb == 0 && lc == 0 && ld == 0) ? 4 : (la == 2 && lb == 0 && lc == 0 && ld == 0) ? 2 : 1;
 }
@@ -35,7 +36,6 @@ __host__ __device__ constexpr int fam_cap_l(int la, int lb, int lc, int ld) {
 struct JKArgs {
   const int2* quartets;
   long long n;
-  const PairRec* pairs;
   const PrimPair* prim_full;
   const PrimPair* prim_skip;
   const double* P;              // Cartesian density (per-molecule blocks)

@@ -9,9 +9,10 @@
 // Per build:
 //   k_density_to_cart  P (Tonto basis) -> P in the Cartesian basis
 //   k_pmax             max |P| per shell pair, global max (molecule.fock.foo:3601)
-//   k_count / k_write  Schwarz-screened quartet lists per class pair, bra-major,
+//   k_quartets         Schwarz-screened quartet lists per class pair, bra-major,
 //                      deterministic order (Schwarz_inequality_test :3454-3495)
-//   k_jk<LA,LB,LC,LD>  one thread per quartet: Rys ERIs + digestion into J, K
+//   k_jk, k_jk_rows    ERIs + digestion into J, K: a thread per quartet or a few lanes
+//                      (tf_thread.cuh), or a lane group (tf_rows.cuh)
 //   k_finalize         J = 2(J + J^T), K = K + K^T (weight_diagonal_blocks,
 //                      blockwise_symmetric_fold, symmetric_reflect :4181-4263),
 //                      back to the Tonto basis
@@ -115,7 +116,8 @@ __global__ void k_pair_prep(int n_pairs, PairRec* __restrict__ pairs, const doub
 
 // Schwarz bounds, one warp per pair: the lanes share the pair's n^2 primitive quartets
 // (up to 4,096 for two eight-primitive shells: on one thread (H2O)9 cc-pVDZ's (ss|ss) took
-// 1.17 ms; tf_set_geometry of that cluster, with its host lists, 3.9 -> 1.7 ms), sum the (e0|f0) block by shuffles and then all hold the integrals.
+// 1.17 ms; tf_set_geometry of that cluster, with its host lists, 2.7 -> 0.94 ms), sum the
+// (e0|f0) block by shuffles and then all hold the integrals.
 constexpr int SCHWARZ_WARPS = 4;
 template <int LA, int LB>
 __global__ void __launch_bounds__(32 * SCHWARZ_WARPS) k_schwarz(const int* __restrict__ ids, int n,
@@ -649,9 +651,10 @@ __global__ void k_fock(long long n, const double* __restrict__ H, const double* 
 }
 
 // ---------------------------------------------------------------------------
-// kernel: one-electron integrals S, T, V (Cartesian blocks), one thread per
-// shell pair a >= b.  Overlap and kinetic by the Obara-Saika 1D recurrences,
-// nuclear attraction by Rys quadrature (molecule.ints.foo:34-420 in meaning).
+// kernels: one-electron integrals S, T, V (Cartesian blocks) of the shell pairs
+// a >= b: a warp per pair (k_one_electron), or a thread per pair where nothing may be
+// allocated (k_one_electron_single).  Overlap and kinetic by the Obara-Saika 1D
+// recurrences, nuclear attraction by Rys quadrature (molecule.ints.foo:34-420 in meaning).
 // ---------------------------------------------------------------------------
 template <int N>
 __device__ __forceinline__ void rys_eval_n(double x, double* u, double* w) {
@@ -667,8 +670,9 @@ __device__ __forceinline__ void rys_eval_n(double x, double* u, double* w) {
 // atom) for V, each with its own na x nb sums in registers, added up by shuffles at the end.
 // (One thread a pair, with run-time angular momenta and its tables in local memory, left
 // a 64-primitive pair of a 27-atom cluster as a serial chain of 1,728 Rys evaluations:
-// (H2O)9 cc-pVDZ 4.97 ms, where the whole call, copies back included, now takes 0.46.)  Primitive pairs as k_pair_prep left them: cc = c_a c_b / zeta
-// times the Gaussian product's factor.
+// (H2O)9 cc-pVDZ 5.1 ms for the call, copies back included; a warp a pair 0.23.)
+// Primitive pairs as k_pair_prep left them: cc = c_a c_b / zeta times the Gaussian
+// product's factor.
 constexpr int ONE_EL_WARPS = 4;
 template <int N>
 struct OneElRoots : std::conditional_t<N == 1, RysSmem<1>, RysPoly<N>> {};
@@ -1224,7 +1228,6 @@ struct tf_ctx {
   tf::DBuf<double> d_cimax;
   tf::DBuf<int4> d_fam_mem;                                // family members of every pair
   tf::DBuf<unsigned char> d_qmask;                         // per list entry: the bra members it holds
-  tf::DBuf<unsigned long long> d_qcount;                   // member quartets per class, FP64 then FP32
   tf::DBuf<int> d_shell_atom, d_shell_nprim, d_shell_poff, d_shell_l, d_shell_first_bf, d_shell_nbf, d_shell_cart;
   tf::DBuf<int> d_cart_shell, d_cart_local, d_bf_shell, d_bf_local, d_sorted, d_schwarz_ids;
   tf::DBuf<tf::PairRec> d_pairs;
@@ -2083,11 +2086,13 @@ double class_flops(int la, int lb, int lc, int ld, double nq, double npq) {
 // fixed-point words per element (fock_add), the lo words after all the hi words,
 // and the kernels are their deterministic instantiations (variant bit 4, fock_add)
 // with the K contributions of neighbouring lanes that hit the same element always
-// summed in FP64 first (bit 2, whatever the autotuner chose): which lanes are
-// summed, and in which order, follows from an entry's position in its class pair's
-// list (lane = position mod 32), which neither the launch shape, the graph nor the
-// list chunking changes, so every path adds the same values.  (Each contribution
-// costs two integer atomics here, so the merged ones pay twice.)
+// summed in FP64 first (bit 2, whatever the autotuner chose).  Which lanes are summed, in
+// which order, and how many lanes share a quartet, follow from the class pair's list
+// alone: an entry's position in its cost bucket, the buckets' counts (LaunchPlan) and the
+// list's length (k_jk_rows).  Neither the launch shape, the graph nor the list chunking
+// changes these, so every path adds the same values; another shard plan, or other
+// molecules in the batch, make other lists.  (Each contribution costs two integer atomics
+// here, so the merged ones pay twice.)
 static long long fx_offset(const tf_ctx* c) { return c->opt.deterministic ? c->cmat_off[c->n_mol] : 0; }
 static long long acc_elems(const tf_ctx* c) { return (c->opt.deterministic ? 2 : 1) * c->cmat_off[c->n_mol]; }
 static int jk_variant(const tf_ctx* c, int g) {
@@ -2096,9 +2101,9 @@ static int jk_variant(const tf_ctx* c, int g) {
 
 // The list pass MODE over tasks [t0, t1): the plain tasks, then the family tasks
 // among them (their own instantiation, over the family task list).  The two passes
-// touch disjoint tasks (their counts, records and list positions), so when the
-// context has a branch stream (tf_autotune creates them) the family pass runs on it,
-// beside the plain pass, and the context stream waits for both.
+// touch disjoint tasks (their counts, records and list positions), so the family pass
+// runs on the first branch stream, beside the plain pass, and the context stream waits
+// for both.
 template <int MODE>
 static int launch_list(tf_ctx* c, ListArgs a, long long t0, long long t1, long long* counts,
                        const long long* offsets, int2* out, cudaStream_t s, int& kernels) {
@@ -2284,7 +2289,7 @@ static int enqueue_graph_body(tf_ctx* c, const BuildIO& io, bool mixed, int want
     class_l(c->group_cls[g].x, l1h, l1l);
     class_l(c->group_cls[g].y, l2h, l2l);
     cudaStream_t sg = branch_of(c, g, ns);
-    JKArgs a{c->d_quartets.p, 0, c->d_pairs.p, c->d_prim_full.p, c->d_prim_skip.p, c->d_Pc.p, c->d_Jc.p,
+    JKArgs a{c->d_quartets.p, 0, c->d_prim_full.p, c->d_prim_skip.p, c->d_Pc.p, c->d_Jc.p,
              c->d_Kc.p, c->d_mols.p, c->d_prim_count.p, c->d_plans.p + 2 * g, c->d_group_offsets.p + 3 * g, 0,
              c->graph_cap, 0, c->d_jkrec.p, c->d_xyz4.p, dPb ? c->d_PcB.p : nullptr, dPb ? c->d_JcB.p : nullptr,
              dPb ? c->d_KcB.p : nullptr, want};
@@ -2537,7 +2542,6 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
                           s));
   TF_CUDA(cudaStreamSynchronize(s));
   TF_CUDA(cudaEventRecord(c->ev1, s));
-  const long long nq_total = ng > 0 ? goff[3 * (ng - 1) + 2] : 0;
   // The lists are written and consumed in chunks of whole class pairs, each at
   // most list_budget quartets (a single larger class pair is one chunk), so a
   // large batch needs one chunk-sized list buffer rather than the whole list.
@@ -2608,7 +2612,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
       class_l(c->group_cls[g].y, l2h, l2l);
       const cudaStream_t sg = branch_of(c, g, ns);
       TF_CUDA(cudaEventRecord(c->cls_ev[2 * g], sg));
-      JKArgs a{c->d_quartets.p, goff[3 * g + 1] - goff[3 * g], c->d_pairs.p,
+      JKArgs a{c->d_quartets.p, goff[3 * g + 1] - goff[3 * g],
                c->d_prim_full.p, c->d_prim_skip.p, c->d_Pc.p, c->d_Jc.p, c->d_Kc.p, c->d_mols.p,
                c->d_prim_count.p, c->d_plans.p + 2 * g, nullptr, base, LLONG_MAX, goff[3 * g], c->d_jkrec.p,
                c->d_xyz4.p,
@@ -2640,7 +2644,6 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
     }
     TF_CUDA(branches.join());
   }
-  (void)nq_total;
   rc = enqueue_finalize(c, dJ, dK, dJb, dKb, kernels);
   if (rc) return rc;
   TF_CUDA(cudaEventRecord(c->ev2, s));
