@@ -2428,6 +2428,16 @@ static void resolve_times(tf_ctx* c) {
   c->stats.eri_ms = sum + (hi - lo);
 }
 
+// Device time of group g in the last direct build (0: it had no entries, so no events).
+static int class_time(const tf_ctx* c, int g, double& out) {
+  out = 0.0;
+  if (c->pin->goff[3 * g + 2] == c->pin->goff[3 * g]) return TF_OK;
+  float ms = 0.f;
+  TF_CUDA(cudaEventElapsedTime(&ms, c->cls_ev[2 * g], c->cls_ev[2 * g + 1]));
+  out = ms;
+  return TF_OK;
+}
+
 // One J/K build for every molecule of the context: dP, dJ, dK are the
 // concatenated per-molecule n_bf x n_bf (column-major) device blocks.
 static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, int flags,
@@ -2607,6 +2617,7 @@ static int build_jk_device(tf_ctx* c, const double* dP, double* dJ, double* dK, 
     Fork branches(c, ns);
     TF_CUDA(branches.fork());
     for (int g = g0; g < g1; ++g) {
+      if (goff[3 * g + 2] == goff[3 * g]) continue;      // no entries
       int l1h, l1l, l2h, l2l;
       class_l(c->group_cls[g].x, l1h, l1l);
       class_l(c->group_cls[g].y, l2h, l2l);
@@ -2985,11 +2996,7 @@ int tf_autotune(tf_ctx* c, const double* dP, double* dJ, double* dK, int flags, 
       rc = build_jk_device(c, dP, dJ, dK, flags);
       if (rc) return rc;
     }
-    for (int g = 0; g < ng; ++g) {
-      float ms = 0.f;
-      TF_CUDA(cudaEventElapsedTime(&ms, c->cls_ev[2 * g], c->cls_ev[2 * g + 1]));
-      tv[v][g] = ms;
-    }
+    for (int g = 0; g < ng; ++g) TF_TRY_RC(class_time(c, g, tv[v][g]));
   }
   for (int g = 0; g < ng; ++g) {
     int l1h, l1l, l2h, l2l;
@@ -3007,11 +3014,7 @@ int tf_autotune(tf_ctx* c, const double* dP, double* dJ, double* dK, int flags, 
   if (rc) return rc;
   res.direct_ms = c->stats.build_ms;
   std::vector<double> t(ng, 0.0);
-  for (int g = 0; g < ng; ++g) {
-    float ms = 0.f;
-    TF_CUDA(cudaEventElapsedTime(&ms, c->cls_ev[2 * g], c->cls_ev[2 * g + 1]));
-    t[g] = ms;
-  }
+  for (int g = 0; g < ng; ++g) TF_TRY_RC(class_time(c, g, t[g]));
   std::vector<int> order(ng);
   for (int g = 0; g < ng; ++g) order[g] = g;
   std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return t[x] > t[y]; });
