@@ -193,9 +193,11 @@ int tf_set_screen_record_budget(tf_ctx* ctx, long long bytes);
 /* CUDA-graph builds (default on).  After a first build has sized the quartet
  * list, each build is one captured graph (density transform, screening, list,
  * every class launch with its quartet range read on the device, Fock
- * accumulation) with no host round trip inside; it is re-captured when the
- * density/J/K arrays, the precision flag or the cutoff change, and a build whose
- * list outgrows the buffer is redone on the direct path.  on = 0: every build
+ * accumulation) with no host round trip inside, whatever density, J and K arrays
+ * it is given; restricted and unrestricted builds have a graph each.  It is
+ * re-captured when the precision flag, the J/K selection or the cutoff change or
+ * the lists have become much longer, and a build whose list outgrows the buffer
+ * is redone on the direct path.  on = 0: every build
  * launches class by class after reading the list sizes back.  No reference
  * counterpart. */
 int tf_set_graph(tf_ctx* ctx, int on);
