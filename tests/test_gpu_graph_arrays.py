@@ -17,7 +17,8 @@ def _captures(builds):
         builds()
         torch.cuda.synchronize()
     names = [e.name() for e in prof.profiler.kineto_results.events()]
-    assert any("cudaGraphLaunch" in n for n in names)         # the profiler sees the runtime's calls
+    if not any("cudaGraphLaunch" in n for n in names):
+        pytest.skip("the profiler does not see the runtime's calls here")
     return sum("GraphInstantiate" in n for n in names)
 
 
@@ -60,6 +61,6 @@ def test_one_graph_serves_any_arrays(cuda_ok, oracle_mod, basis, spherical, dete
         fb.make_u_JK(dens[0], dens[1])
 
     builds(False)                                             # sizes the list, captures both graphs
-    assert _captures(lambda: builds(False)) == 0
     builds(True)
+    assert _captures(lambda: builds(False)) == 0
     fb.close()
